@@ -113,6 +113,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// the same without try_wait's suspension: a look at the barrier
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait for the phase of `parity` to complete.  false = gave up (abort raised).
 __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity,
                                             volatile int* abort_flag,
@@ -472,7 +484,7 @@ __host__ __device__ inline SmemPlan smem_plan(int kb, int brows, int stages, int
   p.sel_off = p.b_off + size_t(stages) * brows * 128;
   p.pub_off = p.sel_off + size_t(nh) * SelectorOf<KH>::type::smem_bytes();
   p.bar_off = p.pub_off + (nh > 1 ? size_t(2) * BM * sizeof(float) : 0);
-  p.total = p.bar_off + 512 + 1024;          // barriers + slack for 1024-byte alignment
+  p.total = p.bar_off + 512;                 // barriers; the buffer itself is 1024-byte aligned
   return p;
 }
 
@@ -480,10 +492,15 @@ __host__ __device__ inline SmemPlan smem_plan(int kb, int brows, int stages, int
 // quarter, each filtering half of the columns into its own list; the two lists of a row share
 // their thresholds while filtering and are merged when the query tile is done).
 // PAIR: two-CTA clusters, 256-row work items (see the file comment).
-// DUAL: two CTAs per SM.  Each CTA holds 256 TMEM columns: every 256-key tile is computed as two
-// N=128 halves into two 128-column accumulators, so the MMA of the next half runs while the
-// epilogue filters the current one; the two CTAs' epilogue warps share each scheduler.  Needs
-// one K atom per row (the halves read the same key stage) and the tagged walk.
+// DUAL: two CTAs per SM.  Each CTA holds 256 TMEM columns: every 256-key tile is loaded and
+// computed as two halves of 128 keys into two 128-column accumulators, so the loads and the MMAs
+// of the next halves run while the epilogue filters the current one; the two CTAs' epilogue warps
+// share each scheduler.  Needs one K atom per row and the tagged walk (tags 2·tile + half).
+// Half-tile stages: with one 256-key stage per CTA the next tile's load could only start when the
+// last MMA of the current one was done, and a tile that no row took a key of cost 3,570 cycles
+// of load and MMA latency (850 for its epilogue).  Half-tile stages and the look-ahead at the next
+// accumulator: main scan at 1.3M x 50 36.1 -> 34.5 ms, MMA waiting for keys 12.4 -> 2.5 M cycles
+// per CTA.
 template <int KH, int NEPI, bool PAIR, bool DUAL>
 __global__ void __launch_bounds__((DUAL ? 64 : 128) + 32 * NEPI, DUAL ? 2 : 1)
 knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -499,10 +516,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   constexpr int EPI0 = DUAL ? 2 : EPI_WARP0;            // first epilogue warp
   constexpr int TMEM_WARP = DUAL ? 0 : 2;
   using Sel = typename SelectorOf<KH>::type;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  const int brows = PAIR ? P.bn / 2 : P.bn;            // key rows this CTA stages per tile
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int brows = (PAIR || DUAL) ? P.bn / 2 : P.bn;  // key rows this CTA stages at a time
   const SmemPlan sp = smem_plan<KH>(P.kb, brows, P.stages, P.na, NH);
   unsigned char* Asm = smem + sp.a_off;
   unsigned char* Bsm = smem + sp.b_off;
@@ -705,16 +720,33 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             return int(uint32_t(e));
           };
           for (int kt = next_tile(); kt >= 0 && ok; kt = next_tile()) {
-            for (int kb = 0; kb < P.kb; ++kb) {           // one pipeline stage per K atom
-              const long long tw = P.prof ? clock64() : 0;
-              ok = mbar_wait(&b_empty[stage], sphase ^ 1, abort_flag);
-              if (P.prof) c_wait += clock64() - tw;
-              if (!ok) break;
-              if (meta && kb == 0) *reinterpret_cast<volatile int*>(&stage_meta[stage]) = kt;
-              mbar_expect_tx(&b_full[stage], uint32_t(b_bytes));
-              tma_load_2d(Bsm + stage * b_bytes, &tmB, &b_full[stage], kb * 64,
-                          w.key0 + kt * P.bn + int(rank) * brows);
-              if (++stage == P.stages) { stage = 0; sphase ^= 1; }
+            if constexpr (DUAL) {
+              // one pipeline stage per half tile (tagged 2·kt + half); a half without keys is
+              // left out
+              const int halves = (kt * 2 + 1) * brows < w.nkeys ? 2 : 1;
+              for (int hf = 0; hf < halves; ++hf) {
+                const long long tw = P.prof ? clock64() : 0;
+                ok = mbar_wait(&b_empty[stage], sphase ^ 1, abort_flag);
+                if (P.prof) c_wait += clock64() - tw;
+                if (!ok) break;
+                *reinterpret_cast<volatile int*>(&stage_meta[stage]) = 2 * kt + hf;
+                mbar_expect_tx(&b_full[stage], uint32_t(b_bytes));
+                tma_load_2d(Bsm + stage * b_bytes, &tmB, &b_full[stage], 0,
+                            w.key0 + kt * P.bn + hf * brows);
+                if (++stage == P.stages) { stage = 0; sphase ^= 1; }
+              }
+            } else {
+              for (int kb = 0; kb < P.kb; ++kb) {         // one pipeline stage per K atom
+                const long long tw = P.prof ? clock64() : 0;
+                ok = mbar_wait(&b_empty[stage], sphase ^ 1, abort_flag);
+                if (P.prof) c_wait += clock64() - tw;
+                if (!ok) break;
+                if (meta && kb == 0) *reinterpret_cast<volatile int*>(&stage_meta[stage]) = kt;
+                mbar_expect_tx(&b_full[stage], uint32_t(b_bytes));
+                tma_load_2d(Bsm + stage * b_bytes, &tmB, &b_full[stage], kb * 64,
+                            w.key0 + kt * P.bn + int(rank) * brows);
+                if (++stage == P.stages) { stage = 0; sphase ^= 1; }
+              }
             }
           }
           if (ok && meta) {
@@ -804,32 +836,6 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               }
               kt_meta = kt;
             }
-            if constexpr (DUAL) {
-              // the tile's two N=128 halves, each into the next free accumulator (tagged 2·kt+half);
-              // the key stage is released once both halves have read it
-              const uint32_t b_base = smem_u32(Bsm + stage * b_bytes);
-              for (int hf = 0; hf < 2; ++hf) {
-                const long long t2 = P.prof ? clock64() : 0;
-                ok = mbar_wait(&acc_empty[acc], accphase ^ 1, abort_flag);
-                if (P.prof) c_acc += clock64() - t2;
-                if (!ok) break;
-                *reinterpret_cast<volatile int*>(&acc_meta[acc]) = 2 * kt_meta + hf;
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + uint32_t(acc * acc_cols);
-                const uint32_t bh = b_base + uint32_t(hf * acc_cols * 128);
-                for (int ks = 0; ks < P.ksteps; ++ks)
-                  umma_f16_g<false>(d_tmem, sdesc(a_base + uint32_t((ks & 3) * 32)),
-                                    sdesc(bh + uint32_t((ks & 3) * 32)), P.idesc, ks > 0 ? 1u : 0u);
-                umma_commit_g<false>(&acc_full[acc]);
-                mbar_arrive(&acc_full[acc]);              // releases acc_meta to the epilogue
-                if (++acc == NACC) { acc = 0; accphase ^= 1; }
-              }
-              if (!ok) break;
-              umma_commit_g<false>(&b_empty[stage]);
-              if (++stage == P.stages) { stage = 0; sphase ^= 1; }
-              issued = true;
-              continue;
-            }
             const long long t2 = P.prof ? clock64() : 0;
             ok = PAIR ? mbar_wait_cl(&acc_empty[acc], accphase ^ 1, abort_flag)
                       : mbar_wait(&acc_empty[acc], accphase ^ 1, abort_flag);
@@ -838,7 +844,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             // the epilogue read this accumulator's previous tile before it released it
             if (meta) *reinterpret_cast<volatile int*>(&acc_meta[acc]) = kt_meta;
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + uint32_t(acc * P.bn);
+            const uint32_t d_tmem = tmem_base + uint32_t(acc * acc_cols);
             for (int kb = 0; kb < P.kb; ++kb) {
               if (!(meta && kb == 0)) {                    // tagged: the first stage is waited for
                 const long long t1 = P.prof ? clock64() : 0;
@@ -943,19 +949,26 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       if (!meta) walk_init(walk, w, it);
       // ordered: R = threshold + roff of this row, published per warp after every tile
       const double roff_row = (ordered && row < nq) ? P.roff[qrow + row] : 0.0;
+      // two register buffers: the next chunk's TMEM load is in flight while the current chunk
+      // is filtered; the accumulator is released right after its last load completes
+      uint32_t ra[32], rb[32];
+      bool ahead = false;                  // the tile's first chunk is already being loaded
+      int kt_next = 0;
       for (;;) {
         int kt = 0;
         if (!meta) {
           kt = walk.next();
           if (kt < 0) break;
         }
-        const long long te = P.prof ? clock64() : 0;
-        ok = __all_sync(FULL, mbar_wait(&acc_full[acc], accphase, abort_flag));
-        if (P.prof) c_ew += clock64() - te;
-        if (!ok) break;
+        if (!ahead) {
+          const long long te = P.prof ? clock64() : 0;
+          ok = __all_sync(FULL, mbar_wait(&acc_full[acc], accphase, abort_flag));
+          if (P.prof) c_ew += clock64() - te;
+          if (!ok) break;
+        }
         int half = 0;                      // DUAL: which N=128 half of key tile kt
         if (meta) {
-          kt = *reinterpret_cast<volatile int*>(&acc_meta[acc]);
+          kt = ahead ? kt_next : *reinterpret_cast<volatile int*>(&acc_meta[acc]);
           if (kt < 0) {                    // the item's walk ended: hand the turn back
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -964,14 +977,11 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           }
           if constexpr (DUAL) { half = kt & 1; kt >>= 1; }
         }
-        tc_fence_after();
+        if (!ahead) tc_fence_after();
         sel.refresh();
         const uint32_t t0 =
             tmem_base + uint32_t(acc * acc_cols + h * gcols) + (uint32_t(q * 32) << 16);
         const int col_base = w.key0 + kt * P.bn + half * acc_cols + h * gcols;
-        // two register buffers: the next chunk's TMEM load is in flight while the current chunk
-        // is filtered; the accumulator is released right after its last load completes
-        uint32_t ra[32], rb[32];
         auto release = [&]() {
           tc_fence_before();
           __syncwarp();
@@ -1017,6 +1027,35 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             if (!cycle(c + 2, rc, ra, rb)) break;
             if (!cycle(c + 4, rb, rc, ra)) break;
           }
+        } else if constexpr (DUAL) {
+          // four chunks of 32 columns.  Before the last one is filtered, the next accumulator is
+          // looked at: if it is full (the usual case, the MMAs run ahead), its tile tag is read
+          // and its first load goes out, so that the wait, the tag and the load latency are hidden
+          // behind the last chunk instead of being paid once per 128 columns.
+          auto push = [&](int c, uint32_t(&x)[32]) {
+            sel.push32(reinterpret_cast<const float(&)[32]>(x), col_base + c * 32, self, limit);
+          };
+          if (!ahead) tmem_ld32_async(t0, ra);
+          tmem_wait(ra);
+          tmem_ld32_async(t0 + 32u, rb);
+          push(0, ra);
+          tmem_wait(rb);
+          tmem_ld32_async(t0 + 64u, ra);
+          push(1, rb);
+          tmem_wait(ra);
+          tmem_ld32_async(t0 + 96u, rb);
+          push(2, ra);
+          const int na = acc ^ 1;
+          ahead = __all_sync(FULL, mbar_poll(&acc_full[na], accphase ^ uint32_t(acc)));
+          if (ahead) {
+            kt_next = *reinterpret_cast<volatile int*>(&acc_meta[na]);
+            tc_fence_after();
+          }
+          tmem_wait(rb);
+          release();
+          if (ahead && kt_next >= 0)
+            tmem_ld32_async(tmem_base + uint32_t(na * acc_cols) + (uint32_t(q * 32) << 16), ra);
+          push(3, rb);
         } else {
           tmem_ld32_async(t0, ra);
           tmem_wait(ra);
@@ -1185,11 +1224,20 @@ int make_map(CUtensorMap* m, const void* base, int64_t rows, int kp, int box_row
 
 size_t config_smem(const TcConfig& c, int kb, int na) {
   const int nh = c.epi / 4;
-  const int brows = c.pair ? c.bn / 2 : c.bn;
-  if (c.kpl == 32) return smem_plan<32>(kb, brows, c.stages, na, nh).total;
-  if (c.kpl == 48) return smem_plan<48>(kb, brows, c.stages, na, nh).total;
-  if (c.kpl == 64) return smem_plan<64>(kb, brows, c.stages, na, nh).total;
+  const int brows = (c.pair || c.ctas == 2) ? c.bn / 2 : c.bn;
+  const int stages = c.ctas == 2 ? 2 * c.stages : c.stages;      // two CTAs per SM: half tiles
+  if (c.kpl == 32) return smem_plan<32>(kb, brows, stages, na, nh).total;
+  if (c.kpl == 48) return smem_plan<48>(kb, brows, stages, na, nh).total;
+  if (c.kpl == 64) return smem_plan<64>(kb, brows, stages, na, nh).total;
   return SIZE_MAX;
+}
+
+// half-tile stages of two CTAs per SM: as many as the list leaves room for (two to four)
+int half_stages(const TcConfig& c, int kb) {
+  const size_t used = config_smem(c, kb, 1);
+  const size_t stage = size_t(c.bn / 2) * 128;
+  const size_t room = SMEM_PER_SM / 2 - SMEM_BLOCK_RESERVE - used;
+  return std::min(8, 2 * c.stages + int(room / stage));
 }
 
 int pick_na(const TcConfig& c, int kb) {
@@ -1201,7 +1249,7 @@ template <int KH, int NEPI, bool PAIR, bool DUAL>
 int launch_tc_t(const TcParams& P, const CUtensorMap& ma, const CUtensorMap& mb,
                 const WorkItem* items, Ctl* ctl, int32_t* cand_idx, float* cand_thr,
                 cudaStream_t st) {
-  const int brows = PAIR ? P.bn / 2 : P.bn;
+  const int brows = (PAIR || DUAL) ? P.bn / 2 : P.bn;
   const size_t smem = smem_plan<KH>(P.kb, brows, P.stages, P.na, NEPI / 4).total;
   auto kern = knn_tc_kernel<KH, NEPI, PAIR, DUAL>;
   MSC_CUDA_TRY(raise_smem_cap(kern, smem));
@@ -1282,8 +1330,8 @@ bool tc_config_ok(const TcConfig& c, int kp, int kprime) {
   if (c.bn != 32 && c.bn != 64 && c.bn != 128 && c.bn != 256) return false;
   if (c.ctas != 1 && c.ctas != 2) return false;
   if (c.ctas == 2) {
-    // two CTAs per SM: single CTAs, four epilogue warps, 256-key tiles computed in two halves,
-    // one K atom per row; both CTAs' shared memory (and the per-block reserve) within the SM's
+    // two CTAs per SM: single CTAs, four epilogue warps, 256-key tiles in two halves (a stage
+    // counts two half tiles here), one K atom per row; both CTAs' shared memory (and the per-block reserve) within the SM's
     if (c.pair || c.epi != 4 || c.bn != 256 || kp != 64 || c.stages < 1 || c.stages > 8)
       return false;
     if (c.kpl < kprime || (c.kpl != 32 && c.kpl != 48 && c.kpl != 64)) return false;
@@ -1350,12 +1398,13 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
   const bool bf16 = prec != PREC_FP16;
   CUtensorMap ma, mb;
   MSC_TRY(make_map(&ma, Aop, a_rows, kp, BM, bf16));
-  MSC_TRY(make_map(&mb, Bop, b_rows, kp, cfg.pair ? cfg.bn / 2 : cfg.bn, bf16));
+  MSC_TRY(make_map(&mb, Bop, b_rows, kp, cfg.pair || cfg.ctas == 2 ? cfg.bn / 2 : cfg.bn,
+                   bf16));
   TcParams P;
   P.ksteps = kmma / 16;
   P.kb = (P.ksteps + 3) / 4;                           // K atoms the MMAs read
   P.bn = cfg.bn;
-  P.stages = cfg.stages;
+  P.stages = cfg.ctas == 2 ? half_stages(cfg, P.kb) : cfg.stages;
   P.na = pick_na(cfg, P.kb);
   P.kprime = kprime;
   P.cand_stride = cand_stride;
