@@ -14,6 +14,7 @@
 #include <tuple>
 #include <vector>
 #include <algorithm>
+#include <cmath>
 #include <unordered_map>
 
 #include <cstdlib>
@@ -163,6 +164,13 @@ struct Problem {
   // key-tile pruning of the tensor-core scan (prune.cu): workspace carved, mask words per item
   bool prune = false;
   int prune_words = 0;
+  // full scan of a small sample: no locality order, no pruning plan; every query tile's keys split
+  // into `split` ranges with a list of kper candidates each (kprime = split·kper in all)
+  bool dense = false;
+  int split = 1;
+  int kper = 0;
+  int64_t stride = 1;     // the cells' order in packed space (launch_plain_order)
+  int kref = 0;           // candidates per row of the refine pass
 };
 
 struct KnnWs {
@@ -227,6 +235,49 @@ int check_common(int64_t n, int d, int k, int metric, int prec, int kprime,
   return MSC_OK;
 }
 
+// Small samples are scanned in full, in no particular order: the order's ~14 launches per level,
+// the near pass and the plan cost a fixed time that the scan they save does not repay.
+// Graph times of the ordered and pruned path against the full scan (k = 15 at 50
+// dimensions / k = 10 at 100, cosine): 2.30 / 2.59 against 0.76 / 0.75 ms at 10,000 cells, 3.16 /
+// 4.08 against 1.66 / 1.81 at 31,007, 4.34 / 5.56 against 3.21 / 3.27 at 57,000, 4.82 / 6.44
+// against 4.89 / 5.12 at 80,000: the line lies where the full scan still wins at every width.
+constexpr int64_t DENSE_MAX_CELLS = 224 * 256;
+// work items of the full scan aimed at per resident CTA, ranges at most, list slots at most
+constexpr int DENSE_ITEMS_PER_CTA = 3, DENSE_MAX_SPLIT = 8, DENSE_SLOTS = 64;
+
+// The full scan's key ranges and list lengths.  A range's list must hold the row's k-1 nearest
+// keys of that range and a few more, for the certificate to have room: with the cells spread
+// evenly over S ranges the number of a row's m = k-1+8 nearest in one range is binomial, and the
+// list takes its mean plus four standard deviations (a row that still overflows one fails the
+// certificate and goes to the refine pass).  All lists of a row together stay within the
+// re-rank's 64 slots.  More ranges fill more CTAs when there are few query tiles, but each list
+// inserts anew, so no more are taken than the CTAs need.
+void plan_dense(Problem& P, int prec, int d, int64_t n, int k, int kprime) {
+  const int base = kprime ? kprime : default_kprime(prec, k);
+  const int nkt = int(ceil_div(n, 256));
+  P.split = 1;
+  P.kper = std::max(base, k - 1);
+  for (int S = 2; S <= std::min(DENSE_MAX_SPLIT, nkt); S *= 2) {
+    const TcConfig c = tc_default_config(prec, d, P.kper);
+    if (c.pair || P.ntiles * P.split >= int64_t(DENSE_ITEMS_PER_CTA) * c.ctas * num_sms()) break;
+    const double m = double(k - 1 + 8) / S;
+    int kper = int(std::ceil(m + 4.0 * std::sqrt(m * (1.0 - 1.0 / S)))) + 1;
+    kper = std::max(kper, int(ceil_div(std::max(kprime, k - 1), S)));
+    if (kper * S > DENSE_SLOTS) break;
+    P.split = S;
+    P.kper = kper;
+  }
+  P.kprime = P.split * P.kper;
+  // a stride near n / golden ratio, coprime to n, spreads cells stored by cluster over the ranges
+  P.stride = 1;
+  if (P.split > 1) {
+    int64_t s = std::max<int64_t>(1, int64_t(0.6180339887 * double(n)));
+    auto gcd = [](int64_t a, int64_t b) { while (b) { const int64_t t = a % b; a = b; b = t; } return a; };
+    while (gcd(s, n) != 1) ++s;
+    P.stride = s;
+  }
+}
+
 // key-tile pruning: samples from this size on, key tiles of this many rows, mask size cap
 constexpr int64_t PRUNE_MIN_CELLS = 4096;
 constexpr int PRUNE_BN = 256;
@@ -272,9 +323,20 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
       P.L = op_layout(PREC_FP32, d);
     }
   }
+  P.kref = P.kprime;
+  if (!offsets && P.candidates && k > 1 && P.prec != PREC_FP32) {
+    // MSC_B200_DENSE=<cells>: the full scan up to that many cells (tuning, tests; 0: never)
+    const char* env = std::getenv("MSC_B200_DENSE");
+    const int64_t most = env && *env ? std::atoll(env) : DENSE_MAX_CELLS;
+    if (n <= most) {
+      P.dense = true;
+      plan_dense(P, P.prec, d, n, k, kprime);
+      P.kref = std::min(P.kprime, std::max(k - 1, default_kprime(PREC_BF16X3, k)));
+    }
+  }
   if (P.candidates && k > 1 && (P.prec == PREC_FP16 || P.prec == PREC_BF16)) {
     P.L3 = op_layout(PREC_BF16X3, d);
-    P.refine = tc_config_ok(tc_default_config(PREC_BF16X3, d, P.kprime), P.L3.kp, P.kprime);
+    P.refine = tc_config_ok(tc_default_config(PREC_BF16X3, d, P.kref), P.L3.kp, P.kref);
   }
   // Pruning pays once a sample spans many key tiles beyond the near ones; its mask (one bit per
   // 256-key tile per 128-row query tile) is capped at 2 GB.  MSC_B200_PRUNE=0 turns it off.  The
@@ -282,7 +344,7 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
   // the forms at equal pruning).
   const char* env32 = std::getenv("MSC_B200_PRUNE_FP32");
   const bool prune32 = env32 && *env32 == '1';
-  if (P.candidates && k > 1 && (P.prec != PREC_FP32 || prune32) &&
+  if (P.candidates && !P.dense && k > 1 && (P.prec != PREC_FP32 || prune32) &&
       P.max_seg >= PRUNE_MIN_CELLS) {
     const char* env = std::getenv("MSC_B200_PRUNE");
     const int words = prune_mask_words(P.max_seg, PRUNE_BN);
@@ -294,6 +356,8 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
   return MSC_OK;
 }
 
+// refine items of the full scan that are split over key ranges (with more, they fill the CTAs)
+constexpr int DENSE_REFINE_ITEMS = 32;
 // leaves of the locality tree (order.cu) hold at most this many rows
 constexpr int ORDER_LEAF = 256;
 // first tree level on the projected rows: the levels above split the sample between clusters, and
@@ -320,13 +384,15 @@ KnnWs carve_knn(Carver& c, const Problem& P) {
   }
   w.qs = c.take<QStat>(P.npacked);
   w.cand_idx = c.take<int32_t>(size_t(P.n) * P.kprime);
-  w.cand_thr = c.take<float>(P.n);
+  w.cand_thr = c.take<float>(size_t(P.n) * P.split);
   w.fail_rows = c.take<int32_t>(P.n);
   w.perm = c.take<int32_t>(P.npacked);
   // the order's rows: projected when d > ORDER_PROJ_D
-  w.Xo = P.d > ORDER_PROJ_D ? c.take<float>(size_t(P.n) * ORDER_PROJ_D) : nullptr;
-  w.order_ws_bytes = order_workspace_bytes(P.npacked, std::max(P.d, ORDER_PROJ_D), ORDER_LEAF);
-  w.order_ws = c.take<unsigned char>(w.order_ws_bytes);
+  if (!P.dense) {
+    w.Xo = P.d > ORDER_PROJ_D ? c.take<float>(size_t(P.n) * ORDER_PROJ_D) : nullptr;
+    w.order_ws_bytes = order_workspace_bytes(P.npacked, std::max(P.d, ORDER_PROJ_D), ORDER_LEAF);
+    w.order_ws = c.take<unsigned char>(w.order_ws_bytes);
+  }
   if (P.refine) {
     w.flags = c.take<int32_t>(P.npacked);
     w.S = c.take<int64_t>(P.npacked + 1);
@@ -338,6 +404,8 @@ KnnWs carve_knn(Carver& c, const Problem& P) {
     w.qs3 = c.take<QStat>(P.npacked);
     w.km3 = c.take<KeyMax>(1);
   }
+  if (P.dense && P.refine)
+    carve_refine_parts(c, w.pr, int(std::min<int64_t>(DENSE_REFINE_ITEMS, P.ntiles)), P.kref);
   if (P.prune)
     w.pr = carve_prune(c, P.npacked, P.nseg, P.d, P.ntiles, P.prune_words, P.n, P.kprime);
   return w;
@@ -360,7 +428,7 @@ int order_levels(const Problem& P, bool tc) {
 }
 
 int decode_tile_config(int32_t code, const Problem& P, TcConfig& cfg) {
-  cfg = tc_default_config(P.prec, P.d, P.kprime);
+  cfg = tc_default_config(P.prec, P.d, P.dense ? P.kper : P.kprime);
   if (code == 0) {
     // tuning override for the automatic choice (same encoding as tile_config)
     const char* env = std::getenv("MSC_B200_TILE_CONFIG");
@@ -396,6 +464,9 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
   const bool tc = P.candidates && P.k > 1 && P.prec != PREC_FP32;
   TcConfig cfg{};
   if (tc) MSC_TRY(decode_tile_config(tile_code, P, cfg));
+  // (a CTA-pair configuration from the environment runs the full scan unsplit)
+  const int split = P.dense && !cfg.pair ? P.split : 1;
+  const int kscan = split > 1 ? P.kper : P.kprime;
   const bool pair_items = tc && cfg.pair;
   const int64_t n_items = pair_items ? P.nptiles : P.ntiles;
   MSC_TRY(launch_build_items(w.seg, P.nseg, n_items, pair_items ? 2 * QTILE : QTILE, w.items, w.ctl,
@@ -410,7 +481,10 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
   if (const char* pe = std::getenv("MSC_B200_ORDER_PROJ")) proj_from = std::atoi(pe);
   const bool proj = w.Xo && levels > proj_from && proj_from >= 0;
   if (proj) MSC_TRY(launch_project(Xu, P.n, P.d, w.Xo, st));
-  MSC_TRY(launch_order(Xu, P.d, w.seg, P.nseg, P.npacked, levels,
+  if (P.dense)
+    MSC_TRY(launch_plain_order(w.seg, P.nseg, P.npacked, P.stride, w.perm, st));
+  else
+    MSC_TRY(launch_order(Xu, P.d, w.seg, P.nseg, P.npacked, levels,
                        ORDER_LEAF, w.perm, (prune || prune32) ? w.pr.leaf : nullptr, w.order_ws,
                        w.order_ws_bytes, st, P.max_seg, proj ? w.Xo : nullptr, ORDER_PROJ_D,
                        proj_from));
@@ -495,10 +569,10 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
       const VisitOrder order{w.pr.vlist, w.pr.voff, w.pr.roff, &w.ctl->ordered_ok};
       MSC_TRY(launch_knn_tc(P.prec, cfg, w.Aop, w.Bop, P.npacked, P.npacked, P.L.kp, P.L.kmma,
                             w.items, n_items, w.perm, nullptr, nullptr, &w.ctl->tc_counter[0],
-                            w.ctl, P.kprime, w.cand_idx, w.cand_thr, P.kprime, st, mask, words,
+                            w.ctl, kscan, w.cand_idx, w.cand_thr, P.kprime, st, mask, words,
                             false, prune && P.nseg == 1, prune ? w.pr.seed : nullptr,
                             prune ? &init : nullptr, nullptr,
-                            ordered ? &order : nullptr, claim));
+                            ordered ? &order : nullptr, claim, split, P.n));
     }
   }
   stage_mark(st, 4);
@@ -506,21 +580,21 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
   MSC_TRY(launch_rerank(Xu, P.d, w.perm, w.seg, P.nseg, P.npacked, w.cand_idx, w.cand_thr,
                         P.kprime, P.kprime, w.qs, w.km, P.prec, P.L.kmma, P.k, cosine, knn_idx,
                         knn_dist, w.fail_rows, w.ctl, nullptr, nullptr, 0,
-                        P.refine ? w.flags : nullptr, st));
+                        P.refine ? w.flags : nullptr, st, split, P.n));
   if (P.refine) {
     // the rows the one-term candidates could not certify, again with the three-term split
     // with pruning, a small refine set is split over key ranges (prune.cu)
-    const bool split = prune;
+    const bool parts = w.pr.part != nullptr && (prune || P.dense);
     MSC_TRY(launch_refine_plan(w.flags, P.npacked, w.seg, P.nseg, w.qmap, w.items3, w.S,
-                               w.scan_scratch, w.ctl, split ? REFINE_SPLIT : 1,
-                               split ? w.pr.max_split_items : 0, st));
+                               w.scan_scratch, w.ctl, parts ? REFINE_SPLIT : 1,
+                               parts ? w.pr.max_split_items : 0, st));
     MSC_CUDA_TRY(cudaMemsetAsync(w.km3, 0, sizeof(KeyMax), st));
     MSC_TRY(launch_pack_tc(PREC_BF16X3, Xu, w.perm, w.seg, P.nseg, w.mean, P.d, P.npacked,
                            nullptr, nullptr, 0, nullptr, w.B3, w.qs3, w.km3, w.ctl, st));
     MSC_TRY(launch_pack_tc(PREC_BF16X3, Xu, w.perm, w.seg, P.nseg, w.mean, P.d, P.npacked,
                            w.qmap, &w.ctl->n_refine, P.n, w.A3, nullptr, nullptr, nullptr, w.ctl,
                            st));
-    const TcConfig cfg3 = tc_default_config(PREC_BF16X3, P.d, P.kprime);
+    const TcConfig cfg3 = tc_default_config(PREC_BF16X3, P.d, P.kref);
     const uint32_t* mask3 = nullptr;
     int words3 = 0;
     if (prune && !cfg3.pair && cfg3.bn == PRUNE_BN) {
@@ -530,21 +604,21 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
                                  P.prec, P.L.kmma, P.L3.kmma, P.d, w.pr, st));
       mask3 = w.pr.mask3;
     }
-    const RefineSplit rs{&w.ctl->refine_split, split ? w.pr.part : nullptr,
-                         split ? w.pr.part_thr : nullptr};
-    const int64_t max_work = split ? std::max<int64_t>(P.ntiles,
+    const RefineSplit rs{&w.ctl->refine_split, parts ? w.pr.part : nullptr,
+                         parts ? w.pr.part_thr : nullptr};
+    const int64_t max_work = parts ? std::max<int64_t>(P.ntiles,
                                                        int64_t(w.pr.max_split_items) * REFINE_SPLIT)
                                    : P.ntiles;
     MSC_TRY(launch_knn_tc(PREC_BF16X3, cfg3, w.A3, w.B3, P.n, P.npacked, P.L3.kp, P.L3.kmma,
                           w.items3, max_work, w.perm, w.qmap, &w.ctl->n_items_refine_eff,
-                          &w.ctl->tc_counter[1], w.ctl, P.kprime, w.cand_idx, w.cand_thr,
-                          P.kprime, st, mask3, words3, false, false, nullptr, nullptr,
-                          split ? &rs : nullptr));
-    if (split)
+                          &w.ctl->tc_counter[1], w.ctl, P.kref, w.cand_idx, w.cand_thr,
+                          P.kref, st, mask3, words3, false, false, nullptr, nullptr,
+                          parts ? &rs : nullptr));
+    if (parts)
       MSC_TRY(launch_refine_merge(w.items3, &w.ctl->n_items_refine, w.ctl, w.qmap, w.perm, P.n,
-                                  w.pr, P.kprime, w.cand_idx, w.cand_thr, st));
+                                  w.pr, P.kref, w.cand_idx, w.cand_thr, st));
     MSC_TRY(launch_rerank(Xu, P.d, w.perm, w.seg, P.nseg, P.npacked, w.cand_idx, w.cand_thr,
-                          P.kprime, P.kprime, w.qs3, w.km3, PREC_BF16X3, P.L3.kmma, P.k, cosine,
+                          P.kref, P.kref, w.qs3, w.km3, PREC_BF16X3, P.L3.kmma, P.k, cosine,
                           knn_idx, knn_dist, w.fail_rows, w.ctl, w.qmap, &w.ctl->n_refine, P.n,
                           nullptr, st));
   }

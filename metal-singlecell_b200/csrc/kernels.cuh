@@ -115,6 +115,10 @@ int launch_order(const float* X, int d, const SegDesc* seg, int nseg, int64_t np
                  int leaf, int32_t* perm, int32_t* leaf_out, void* ws, size_t ws_bytes,
                  cudaStream_t st, int64_t max_seg, const float* Xp = nullptr, int dp = 0,
                  int proj_from = 0);
+// the order of the full scan: cell (j·stride) mod n of a sample at its j-th position (stride
+// coprime to every sample's size, 1: plain order)
+int launch_plain_order(const SegDesc* seg, int nseg, int64_t npacked, int64_t stride,
+                       int32_t* perm, cudaStream_t st);
 size_t scan_i32_scratch_elems(int64_t n);
 int scan_excl_i32(const int32_t* in, int64_t n, int64_t* out, int64_t* scratch, cudaStream_t st);
 int launch_single_segment(SegDesc* seg, int64_t n, cudaStream_t st);
@@ -161,6 +165,8 @@ struct PruneWs {
 int prune_mask_words(int64_t max_seg, int bn);
 PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items, int words,
                     int64_t n, int kprime);
+// the split refine pass's partial lists alone (a scan without a pruning plan)
+void carve_refine_parts(Carver& c, PruneWs& w, int max_items, int kprime);
 // after the near pass (key tiles of bn rows): R per row, outliers to the end of each sample
 // (perm is rewritten), the inverse permutation and every row's near-pass key ranges
 int launch_prune_partition(const float* X, int d, const SegDesc* seg, int nseg, int64_t npacked,
@@ -272,7 +278,8 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
                   const uint32_t* mask = nullptr, int mask_words = 0, bool near_only = false,
                   bool reverse = false, const float* seed = nullptr,
                   const NearInit* init = nullptr, const RefineSplit* split = nullptr,
-                  const VisitOrder* order = nullptr, const int32_t* claim = nullptr);
+                  const VisitOrder* order = nullptr, const int32_t* claim = nullptr,
+                  int split_host = 1, int64_t thr_stride = 0);
 
 // ---- rerank.cu ----
 int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg, int nseg,
@@ -281,7 +288,7 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
                   const QStat* qs, const KeyMax* km, int prec, int kmma, int k, int cosine,
                   int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,
                   const int32_t* rows, const int32_t* nrows, int64_t max_rows,
-                  int32_t* fail_flags, cudaStream_t st);
+                  int32_t* fail_flags, cudaStream_t st, int n_thr = 1, int64_t thr_stride = 0);
 // refine plan: compact the flagged packed rows (sorted) into qmap, count them (ctl->n_refine)
 // and cut them into per-sample query tiles (items, ctl->n_items_refine); S: npacked+1 int64
 // split > 1: when there are at most max_split_items refine items, each becomes `split` work

@@ -361,6 +361,10 @@ struct TcParams {
   const int32_t* split_dev;
   int2* part;
   float* part_thr;
+  // full scan split over key ranges by the host (1: no split): range r of a row writes its k'
+  // candidates at column r·k' of the row and its threshold to cand_thr[r·thr_stride + row]
+  int split_host;
+  int64_t thr_stride;
   float* cand_val;              // near pass: also write the values of the kept candidates
   // main pass after a near pass: load every row's list from the near pass's candidates (values,
   // original rows -> packed positions through iperm) and never offer its keys again (excl)
@@ -495,7 +499,8 @@ __host__ __device__ inline SmemPlan smem_plan(int kb, int brows, int stages, int
 // DUAL: two CTAs per SM.  Each CTA holds 256 TMEM columns: every 256-key tile is loaded and
 // computed as two halves of 128 keys into two 128-column accumulators, so the loads and the MMAs
 // of the next halves run while the epilogue filters the current one; the two CTAs' epilogue warps
-// share each scheduler.  Needs one K atom per row and the tagged walk (tags 2·tile + half).
+// share each scheduler.  A pipeline stage is one K atom of a half tile; needs the tagged walk
+// (tags 2·tile + half).
 // Half-tile stages: with one 256-key stage per CTA the next tile's load could only start when the
 // last MMA of the current one was done, and a tile that no row took a key of cost 3,570 cycles
 // of load and MMA latency (850 for its epilogue).  Half-tile stages and the look-ahead at the next
@@ -629,15 +634,15 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     it = v;
     return true;
   };
-  // Refine items split over key ranges: work item it = (refine item it / S, range it % S).
-  const int S = P.split_dev ? max(1, *P.split_dev) : 1;
+  // Items split over key ranges: work item it = (query tile it / S, range it % S).
+  const int S = P.split_dev ? max(1, *P.split_dev) : P.split_host;
   auto item_of = [&](int it) { return S > 1 ? it / S : it; };
   auto walk_init = [&](KeyTileWalk& walk, const WorkItem& w, int it) {
     const int r = item_of(it);
     walk.init(w, P.qmap ? P.qmap[w.qrow0] : w.qrow0, P.bn,
               P.mask ? P.mask + int64_t(r) * P.mask_words : nullptr, P.mask_words,
               P.near_only != 0);
-    if (P.qmap) {
+    if (P.qmap || S > 1) {
       const int sidx = S > 1 ? it % S : 0;
       const int chunk = (walk.nkt + S - 1) / S;
       walk.set_range(sidx * chunk, min(walk.nkt, (sidx + 1) * chunk));
@@ -721,17 +726,18 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           };
           for (int kt = next_tile(); kt >= 0 && ok; kt = next_tile()) {
             if constexpr (DUAL) {
-              // one pipeline stage per half tile (tagged 2·kt + half); a half without keys is
-              // left out
+              // one pipeline stage per K atom of a half tile (the first tagged 2·kt + half); a
+              // half without keys is left out
               const int halves = (kt * 2 + 1) * brows < w.nkeys ? 2 : 1;
-              for (int hf = 0; hf < halves; ++hf) {
+              for (int x = 0; x < halves * P.kb; ++x) {
+                const int hf = x >= P.kb ? 1 : 0, kb = x - hf * P.kb;
                 const long long tw = P.prof ? clock64() : 0;
                 ok = mbar_wait(&b_empty[stage], sphase ^ 1, abort_flag);
                 if (P.prof) c_wait += clock64() - tw;
                 if (!ok) break;
-                *reinterpret_cast<volatile int*>(&stage_meta[stage]) = 2 * kt + hf;
+                if (kb == 0) *reinterpret_cast<volatile int*>(&stage_meta[stage]) = 2 * kt + hf;
                 mbar_expect_tx(&b_full[stage], uint32_t(b_bytes));
-                tma_load_2d(Bsm + stage * b_bytes, &tmB, &b_full[stage], 0,
+                tma_load_2d(Bsm + stage * b_bytes, &tmB, &b_full[stage], kb * 64,
                             w.key0 + kt * P.bn + hf * brows);
                 if (++stage == P.stages) { stage = 0; sphase ^= 1; }
               }
@@ -1094,11 +1100,12 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int wrow0 = q * 32;
       const int nvalid = min(32, nq - wrow0);
       auto write_out = [&]() {
-        if (S > 1)
+        const int sidx = S > 1 ? it % S : 0;
+        if (S > 1 && P.part)
           sel.finish_partial(P.part, P.part_thr, int64_t(it) * BM + wrow0, P.perm, nvalid,
                              P.kprime);
         else
-          sel.finish(cand_idx, cand_thr, P.cand_stride, P.perm, P.qmap, int64_t(qrow) + wrow0,
+          sel.finish(cand_idx + sidx * P.kprime, cand_thr + sidx * P.thr_stride, P.cand_stride, P.perm, P.qmap, int64_t(qrow) + wrow0,
                      nvalid, P.kprime, P.cand_val);
       };
       if (NH == 1) {
@@ -1232,7 +1239,7 @@ size_t config_smem(const TcConfig& c, int kb, int na) {
   return SIZE_MAX;
 }
 
-// half-tile stages of two CTAs per SM: as many as the list leaves room for (two to four)
+// stages (K atoms of a half tile) of two CTAs per SM: as many as the list leaves room for
 int half_stages(const TcConfig& c, int kb) {
   const size_t used = config_smem(c, kb, 1);
   const size_t stage = size_t(c.bn / 2) * 128;
@@ -1331,9 +1338,9 @@ bool tc_config_ok(const TcConfig& c, int kp, int kprime) {
   if (c.ctas != 1 && c.ctas != 2) return false;
   if (c.ctas == 2) {
     // two CTAs per SM: single CTAs, four epilogue warps, 256-key tiles in two halves (a stage
-    // counts two half tiles here), one K atom per row; both CTAs' shared memory (and the per-block reserve) within the SM's
-    if (c.pair || c.epi != 4 || c.bn != 256 || kp != 64 || c.stages < 1 || c.stages > 8)
-      return false;
+    // counts two K atoms of a half tile here); both CTAs' shared memory (and the per-block
+    // reserve) within the SM's
+    if (c.pair || c.epi != 4 || c.bn != 256 || c.stages < 1 || c.stages > 8) return false;
     if (c.kpl < kprime || (c.kpl != 32 && c.kpl != 48 && c.kpl != 64)) return false;
     if (c.cb != 16 && c.cb != 32) return false;
     return 2 * (config_smem(c, kp / 64, 1) + SMEM_BLOCK_RESERVE) <= SMEM_PER_SM;
@@ -1362,8 +1369,8 @@ TcConfig tc_default_config(int prec, int d, int kprime) {
   // eight warps whose two column halves each keep a list), else eight; then the deepest K-atom
   // pipeline that fits
   {
-    // two CTAs per SM where they fit (one K atom per row): every scheduler runs two epilogue
-    // warps of different rows.  MSC_B200_DUAL=0 turns this off.
+    // two CTAs per SM where they fit (one K atom per row, or two with lists of at most 48, three
+    // with lists of 32): every scheduler runs two epilogue warps of different rows.  MSC_B200_DUAL=0 turns this off.
     const char* env = std::getenv("MSC_B200_DUAL");
     if (!(env && *env == '0'))
       for (int stages = 8; stages >= 1; --stages) {
@@ -1388,7 +1395,8 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
                   int32_t* cand_idx, float* cand_thr, int cand_stride, cudaStream_t st,
                   const uint32_t* mask, int mask_words, bool near_only, bool reverse,
                   const float* seed, const NearInit* init, const RefineSplit* split,
-                  const VisitOrder* order, const int32_t* claim) {
+                  const VisitOrder* order, const int32_t* claim, int split_host,
+                  int64_t thr_stride) {
   const int prof_slot = near_only ? 0 : (qmap ? 2 : 1);
   if (!tc_config_ok(cfg, kp, kprime)) {
     set_error("tensor-core tile config (bn=%d stages=%d kpl=%d cb=%d epi=%d pair=%d) does not fit",
@@ -1409,7 +1417,9 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
   P.kprime = kprime;
   P.cand_stride = cand_stride;
   P.bf16 = bf16;
-  P.n_items = int(n_items);
+  P.split_host = std::max(1, split_host);
+  P.thr_stride = thr_stride;
+  P.n_items = int(n_items * P.split_host);
   P.idesc = idesc_f16(bf16, cfg.pair ? 2 * BM : BM, cfg.ctas == 2 ? cfg.bn / 2 : cfg.bn);
   P.prof = profiling_enabled() ? 1 : 0;
   P.perm = perm;
@@ -1443,8 +1453,8 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
     const char* env = std::getenv("MSC_B200_META_WALK");
     P.meta_walk = (env && *env == '0') ? 0 : 1;
   }
-  if (cfg.pair && (mask || near_only)) {
-    set_error("pruned scans run on single CTAs only");
+  if (cfg.pair && (mask || near_only || P.split_host > 1)) {
+    set_error("pruned and split scans run on single CTAs only");
     return MSC_ERR_INVALID_ARG;
   }
   if (cfg.pair) {

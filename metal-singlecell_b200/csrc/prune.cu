@@ -900,10 +900,7 @@ PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items
   w.cand_val = c.take<float>(size_t(n) * kprime);
   w.iperm = c.take<int32_t>(n);
   w.excl = c.take<int4>(npacked);
-  w.max_split_items = int(std::min<int64_t>(256, n_items));
-  const int64_t prow = int64_t(w.max_split_items) * REFINE_SPLIT * QTILE;
-  w.part = c.take<int2>(size_t(prow) * kprime);
-  w.part_thr = c.take<float>(prow);
+  carve_refine_parts(c, w, int(std::min<int64_t>(256, n_items)), kprime);
   w.seed = c.take<float>(npacked);
   w.roff = c.take<double>(npacked);
   w.vcnt = c.take<int32_t>(n_items);
@@ -917,6 +914,13 @@ PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items
   w.vcap = std::min<int64_t>(all, std::max<int64_t>(int64_t(16) << 20, all / 4));
   w.vlist = c.take<unsigned long long>(w.vcap);
   return w;
+}
+
+void carve_refine_parts(Carver& c, PruneWs& w, int max_items, int kprime) {
+  w.max_split_items = max_items;
+  const int64_t prow = int64_t(max_items) * REFINE_SPLIT * QTILE;
+  w.part = c.take<int2>(size_t(prow) * kprime);
+  w.part_thr = c.take<float>(prow);
 }
 
 int launch_prune_partition(const float* X, int d, const SegDesc* seg, int nseg, int64_t npacked,

@@ -83,7 +83,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
               int prec, int kmma, int k, int cosine, int32_t* __restrict__ knn_idx,
               float* __restrict__ knn_dist, int32_t* __restrict__ fail_rows,
               const int32_t* __restrict__ rows, const int32_t* __restrict__ nrows,
-              int32_t* __restrict__ fail_flags) {
+              int32_t* __restrict__ fail_flags, int n_thr, int64_t thr_stride) {
   __shared__ __align__(16) float xs_all[RR_WARPS][MSC_MAX_D];
   __shared__ int wsc_all[RR_WARPS][32];                 // a row's window, compacted
   const int lane = lane_id(), wib = warp_id();
@@ -187,12 +187,16 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
     // 4. certificate
     bool cert;
     const int nvalid = int(min64(ns - 1, kprime));
-    if (ns - 1 <= kprime) {
+    if (n_thr == 1 && ns - 1 <= kprime) {
       cert = true;                                      // every key is a candidate
     } else {
       const QStat q = qs[p];
       const double eps = cert_eps(q, kmv, prec, kmma, d);
-      const double T = double(cand_thr[i]);
+      // a scan split over key ranges: a key left out of its range's list is at or above that
+      // range's threshold (+inf: no key of the range was left out)
+      float t = cand_thr[i];
+      for (int r = 1; r < n_thr; ++r) t = fminf(t, cand_thr[r * thr_stride + i]);
+      const double T = double(t);
       cert = f2 * Dk < q.sq + T - eps;
     }
     (void)nvalid;
@@ -353,7 +357,7 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
                   const QStat* qs, const KeyMax* km, int prec, int kmma, int k, int cosine,
                   int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,
                   const int32_t* rows, const int32_t* nrows, int64_t max_rows,
-                  int32_t* fail_flags, cudaStream_t st) {
+                  int32_t* fail_flags, cudaStream_t st, int n_thr, int64_t thr_stride) {
   if (kprime > 64 || k - 1 > 64) {
     set_error("rerank: kprime=%d / k=%d beyond 64", kprime, k);
     return MSC_ERR_UNSUPPORTED;
@@ -362,7 +366,8 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
   int blocks = int(std::min<int64_t>(ceil_div(n_work, RR_WARPS), int64_t(num_sms()) * 8));
   rerank_kernel<<<std::max(blocks, 1), RR_WARPS * 32, 0, st>>>(
       X, d, perm, seg, nseg, npacked, cand_idx, cand_thr, cand_stride, kprime, qs, km, ctl, prec,
-      kmma, k, cosine, knn_idx, knn_dist, fail_rows, rows, nrows, fail_flags);
+      kmma, k, cosine, knn_idx, knn_dist, fail_rows, rows, nrows, fail_flags, n_thr,
+      thr_stride);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
