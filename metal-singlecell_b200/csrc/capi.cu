@@ -636,8 +636,6 @@ int copy_stats(const KnnWs& w, int64_t* stats_dev, cudaStream_t st) {
 }
 
 struct GraphWs {
-  float* sigma;
-  float* rho;
   float* w;
   double* gsum;
   double* sig2;
@@ -648,8 +646,6 @@ struct GraphWs {
 GraphWs carve_graph(Carver& c, int64_t n, int k, int method) {
   GraphWs g{};
   if (method == MSC_METHOD_UMAP) {
-    g.sigma = c.take<float>(n);
-    g.rho = c.take<float>(n);
     g.w = c.take<float>(size_t(n) * k);
     g.gsum = c.take<double>(1 + 1024);
   } else {
@@ -827,11 +823,13 @@ int msc_neighbors_ex(const float* X_dev, int64_t n, int32_t d, int32_t k, int32_
   if (distances_ready_event)
     MSC_CUDA_TRY(cudaEventRecord(static_cast<cudaEvent_t>(distances_ready_event), st));
   if (method == MSC_METHOD_UMAP) {
-    MSC_TRY(launch_smooth_knn(knn_dist_dev, n, k, 1.0f, g.sigma, g.rho, g.gsum, st));
-    MSC_TRY(launch_membership(knn_idx_dev, knn_dist_dev, g.sigma, g.rho, n, k, g.w, st));
+    int32_t* indeg = nullptr;
+    MSC_TRY(union_begin(n, k, g.uws, &indeg, st));
+    MSC_TRY(launch_smooth_membership(knn_idx_dev, knn_dist_dev, n, k, 1.0f, g.w, indeg, g.gsum,
+                                     st));
     stage_mark(st, 6);
     MSC_TRY(launch_union(0, knn_idx_dev, g.w, nullptr, n, k, conn_indptr_dev, conn_indices_dev,
-                         conn_data_dev, nullptr, g.uws, g.uws_bytes, st));
+                         conn_data_dev, nullptr, g.uws, g.uws_bytes, st, true));
   } else {
     MSC_TRY(launch_gauss_sigma(knn_dist_dev, n, k, g.sig2, st));
     stage_mark(st, 6);

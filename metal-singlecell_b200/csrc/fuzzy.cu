@@ -15,8 +15,8 @@
 //      (slot from an atomic cursor — order within the segment is arbitrary);
 //   4. per row: its own list (read straight from the kNN arrays) and its reverse records sorted by
 //      key = (column << 1 | reverse) — a warp bitonic network in registers up to 128 entries
-//      (inline with the row's neighbours), up to 512 in a second warp-per-row pass, a block
-//      network beyond — then the pairs merged (a column present in both directions) and
+//      (inline with the row's neighbours), a small block's network up to 512, a large block's
+//      beyond — then the pairs merged (a column present in both directions) and
 //      the unique entries written left-justified into the segment;
 //   5. exclusive scan of the unique counts → indptr; 6. copy into indices / data.
 #include "kernels.cuh"
@@ -72,11 +72,29 @@ __global__ void scan_reduce_kernel(const T* __restrict__ in, int64_t n, int64_t*
   if (threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
+// Every block finds its own offset: the sum of the block sums before it (bsum), or of the input
+// before it where that is short (bsum null: no reduce launch), or it is given (boff).  A scan of
+// up to SCAN_DIRECT blocks is one launch, of up to SCAN_FLAT two (each was three: 2 us of kernel and
+// 2 us of gap apiece on inputs of some ten thousand entries).
+constexpr int64_t SCAN_DIRECT = 8, SCAN_FLAT = 4096;
 template <class T>
 __global__ void scan_apply_kernel(const T* __restrict__ in, int64_t n,
+                                  const int64_t* __restrict__ bsum,
                                   const int64_t* __restrict__ boff, int64_t* __restrict__ out) {
   __shared__ int64_t sh[32];
   const int64_t b0 = int64_t(blockIdx.x) * SCAN_B;
+  int64_t before = 0;
+  if (boff) {
+    before = boff[blockIdx.x];
+  } else if (blockIdx.x > 0) {
+    int64_t a = 0;
+    if (bsum)
+      for (int64_t i = threadIdx.x; i < blockIdx.x; i += SCAN_T) a += bsum[i];
+    else
+#pragma unroll 4
+      for (int64_t i = threadIdx.x; i < b0; i += SCAN_T) a += int64_t(in[i]);
+    block_excl_scan(a, sh, before);
+  }
   int64_t v[SCAN_E];
   int64_t s = 0;
   const int64_t base_i = b0 + int64_t(threadIdx.x) * SCAN_E;     // contiguous per thread
@@ -86,7 +104,7 @@ __global__ void scan_apply_kernel(const T* __restrict__ in, int64_t n,
     s += v[e];
   }
   int64_t total;
-  int64_t pre = block_excl_scan(s, sh, total) + (boff ? boff[blockIdx.x] : 0);
+  int64_t pre = block_excl_scan(s, sh, total) + before;
   for (int e = 0; e < SCAN_E; ++e) {
     int64_t i = base_i + e;
     if (i < n) out[i] = pre;
@@ -109,8 +127,8 @@ size_t scan_scratch_elems(int64_t n) {
 template <class T>
 int scan_excl(const T* in, int64_t n, int64_t* out, int64_t* scratch, cudaStream_t st) {
   const int64_t nb = ceil_div(std::max<int64_t>(n, 1), SCAN_B);
-  if (nb == 1) {
-    scan_apply_kernel<T><<<1, SCAN_T, 0, st>>>(in, n, nullptr, out);
+  if (nb <= SCAN_DIRECT) {
+    scan_apply_kernel<T><<<unsigned(nb), SCAN_T, 0, st>>>(in, n, nullptr, nullptr, out);
     MSC_LAUNCH_CHECK();
     return MSC_OK;
   }
@@ -118,8 +136,13 @@ int scan_excl(const T* in, int64_t n, int64_t* out, int64_t* scratch, cudaStream
   int64_t* boff = scratch + nb + 1;
   scan_reduce_kernel<T><<<unsigned(nb), SCAN_T, 0, st>>>(in, n, bsum);
   MSC_LAUNCH_CHECK();
+  if (nb <= SCAN_FLAT) {
+    scan_apply_kernel<T><<<unsigned(nb), SCAN_T, 0, st>>>(in, n, bsum, nullptr, out);
+    MSC_LAUNCH_CHECK();
+    return MSC_OK;
+  }
   MSC_TRY(scan_excl<int64_t>(bsum, nb, boff, scratch + 2 * (nb + 1), st));
-  scan_apply_kernel<T><<<unsigned(nb), SCAN_T, 0, st>>>(in, n, boff, out);
+  scan_apply_kernel<T><<<unsigned(nb), SCAN_T, 0, st>>>(in, n, nullptr, boff, out);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
@@ -132,9 +155,20 @@ __device__ __forceinline__ bool kept(int mode, int t, float v) {
   return mode == 0 ? (v > 0.f) : (t > 0);
 }
 
-// The lanes of a warp walk the k·32 list entries of 32 consecutive rows in memory order (coalesced
-// loads).  Entry x of the group is row x / k, position x % k; the division is a multiply-shift,
-// exact for x < 32·k and k <= 129 (x·ceil(2^22 / k) >> 22 = floor(x / k), checked exhaustively).
+// The lanes of a warp walk the list entries of `rpw` <= 32 consecutive rows in memory order
+// (coalesced loads).  Entry x of the group is row x / k, position x % k; the division is a
+// multiply-shift, exact for x < 32·k and k <= 129 (x·ceil(2^22 / k) >> 22 = floor(x / k), checked
+// exhaustively).
+//
+// Rows per warp: 32 once that still makes WARPS_WANTED warps, fewer below, down to one entry per
+// lane.  With 32 rows per warp at every size, 500 cells were 16 warps of 15 dependent atomics each
+// (rev_fill 13 us, and 121 us for the merge below, whose warps took 32 rows one after another).
+constexpr int64_t WARPS_WANTED_PER_SM = 128;
+int rows_per_warp(int64_t n, int sms) {
+  int r = 32;
+  while (r > 1 && ceil_div(n, r) < WARPS_WANTED_PER_SM * sms) r >>= 1;
+  return r;
+}
 __host__ __device__ __forceinline__ uint32_t div_magic(int k) {
   return uint32_t(((uint64_t(1) << 22) + uint64_t(k) - 1) / uint64_t(k));
 }
@@ -142,13 +176,13 @@ __host__ __device__ __forceinline__ uint32_t div_magic(int k) {
 template <class F>
 __device__ __forceinline__ void for_each_kept_edge(int mode, const int32_t* __restrict__ idx,
                                                    const float* __restrict__ vals, int64_t n, int k,
-                                                   uint32_t magic, F&& f) {
+                                                   uint32_t magic, int rpw, F&& f) {
   const int lane = lane_id();
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; g * 32 < n;
+  for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; g * rpw < n;
        g += nwarps) {
-    const int64_t r0 = g * 32;
-    const int ne = int(min64(32, n - r0)) * k;
+    const int64_t r0 = g * rpw;
+    const int ne = int(min64(rpw, n - r0)) * k;
     const int64_t e0 = r0 * k;
     for (int x = lane; x < ne; x += 32) {
       const int r = int((uint32_t(x) * magic) >> 22);
@@ -163,8 +197,8 @@ __device__ __forceinline__ void for_each_kept_edge(int mode, const int32_t* __re
 
 __global__ void __launch_bounds__(256)
 rev_count_kernel(int mode, const int32_t* __restrict__ idx, const float* __restrict__ vals,
-                 int64_t n, int k, uint32_t magic, int32_t* __restrict__ indeg) {
-  for_each_kept_edge(mode, idx, vals, n, k, magic,
+                 int64_t n, int k, uint32_t magic, int rpw, int32_t* __restrict__ indeg) {
+  for_each_kept_edge(mode, idx, vals, n, k, magic, rpw,
                      [&](int64_t, int32_t j, float) { atomicAdd(&indeg[j], 1); });
 }
 
@@ -172,9 +206,9 @@ rev_count_kernel(int mode, const int32_t* __restrict__ idx, const float* __restr
 // in-degrees): k slots for its own list, then its reverse records (i' → i, in any order).
 __global__ void __launch_bounds__(256)
 rev_fill_kernel(int mode, const int32_t* __restrict__ idx, const float* __restrict__ vals,
-                int64_t n, int k, uint32_t magic, const int64_t* __restrict__ rptr,
+                int64_t n, int k, uint32_t magic, int rpw, const int64_t* __restrict__ rptr,
                 int32_t* __restrict__ cursor, int2* __restrict__ rec) {
-  for_each_kept_edge(mode, idx, vals, n, k, magic, [&](int64_t i, int32_t j, float v) {
+  for_each_kept_edge(mode, idx, vals, n, k, magic, rpw, [&](int64_t i, int32_t j, float v) {
     const int64_t slot = int64_t(j) * k + rptr[j] + k + atomicAdd(&cursor[j], 1);
     rec[slot] = make_int2(int((uint32_t(i) << 1) | 1u), __float_as_int(v));
   });
@@ -306,7 +340,7 @@ __device__ __forceinline__ int merge_row_regs(int mode, int64_t i, int k, int L,
 }
 
 constexpr int WARP_MAX = 128;    // longest row the warp tier sorts (4 keys per lane)
-constexpr int MID_MAX = 512;     // longest row the mid tier sorts (16 keys per lane)
+constexpr int MID_MAX = 512;     // longest row the mid tier sorts
 
 // rows of 65..128 entries are rare: their sort stays out of line, so that the common paths (one or
 // two keys per lane) keep a small instruction footprint
@@ -317,20 +351,20 @@ __device__ __noinline__ int merge_row_regs4(int mode, int64_t i, int k, int L, i
   return merge_row_regs<4>(mode, i, k, L, n, idx, vals, seg, sig2);
 }
 
-// A warp takes 32 consecutive rows at a time: their segment offsets come in one coalesced load,
-// then the rows are merged one after another.
+// A warp takes `rpw` consecutive rows at a time (rows_per_warp): their segment offsets come in one
+// coalesced load, then the rows are merged one after another.
 __global__ void __launch_bounds__(UW * 32)
 merge_warp_kernel(int mode, int64_t n, int k, const int32_t* __restrict__ idx,
                   const float* __restrict__ vals, const int64_t* __restrict__ rptr,
                   int2* __restrict__ rec, const double* __restrict__ sig2,
                   int32_t* __restrict__ uniq, int32_t* __restrict__ big_rows,
-                  int32_t* __restrict__ n_big) {
+                  int32_t* __restrict__ n_big, int rpw) {
   const int lane = lane_id();
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; g * 32 < n;
+  for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; g * rpw < n;
        g += nwarps) {
-    const int64_t r0 = g * 32;
-    const int nr = int(min64(32, n - r0));
+    const int64_t r0 = g * rpw;
+    const int nr = int(min64(rpw, n - r0));
     const int64_t my_p0 = lane < nr ? rptr[r0 + lane] : 0;
     const int64_t my_p1 = lane < nr ? rptr[r0 + lane + 1] : 0;
     int my_u = 0;
@@ -366,36 +400,89 @@ merge_warp_kernel(int mode, int64_t n, int k, const int32_t* __restrict__ idx,
   }
 }
 
-// mid tier: a warp per listed long row of up to MID_MAX entries, sorted in registers (8 or 16
-// keys per lane); longer rows are listed again for the block tier.  (Rows of 129..512 entries in
-// the block tier -- a 1024-thread block with a barrier per network stage for a few hundred keys --
-// took 1.7 ms at 1.3M cells.)
-constexpr int MID_W = 8;         // warps per block
-__global__ void __launch_bounds__(MID_W * 32)
+// mid tier: a small block per listed long row of up to MID_MAX entries, sorted in shared memory;
+// longer rows are listed again for the block tier.  (In the block tier -- 1024 threads and a
+// barrier per network stage for a few hundred keys -- these rows took 1.7 ms at 1.3M cells, and
+// as a warp each, 16 keys a lane, 0.42 ms and 28 us for the first row: the unrolled network of
+// 7,000 instructions does not stay in the instruction cache.  Now 0.18 ms and 7 us.)
+constexpr int MID_T = 128;       // threads per block: up to four entries each
+__global__ void __launch_bounds__(MID_T)
 merge_mid_kernel(int mode, int64_t n, int k, const int32_t* __restrict__ idx,
                  const float* __restrict__ vals, const int64_t* __restrict__ rptr,
                  int2* __restrict__ rec, const double* __restrict__ sig2,
                  int32_t* __restrict__ uniq, const int32_t* __restrict__ big_rows,
                  const int32_t* __restrict__ n_big, int32_t* __restrict__ huge_rows,
                  int32_t* __restrict__ n_huge) {
-  const int lane = lane_id();
+  __shared__ int2 S[MID_MAX];
+  __shared__ int wsum[MID_T / 32];
+  const int tid = threadIdx.x, lane = lane_id(), wib = warp_id();
   const int nb = *n_big;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; r < nb; r += nwarps) {
+  for (int r = blockIdx.x; r < nb; r += gridDim.x) {
     const int64_t i = big_rows[r];
     const int64_t p0 = rptr[i];
     const int L = k + int(rptr[i + 1] - p0);
-    int2* seg = rec + i * k + p0;
-    int u;
-    if (L <= 256) {
-      u = merge_row_regs<8>(mode, i, k, L, n, idx, vals, seg, sig2);
-    } else if (L <= MID_MAX) {
-      u = merge_row_regs<16>(mode, i, k, L, n, idx, vals, seg, sig2);
-    } else {
-      if (lane == 0) huge_rows[atomicAdd(n_huge, 1)] = int32_t(i);
+    if (L > MID_MAX) {                           // block-uniform
+      if (tid == 0) huge_rows[atomicAdd(n_huge, 1)] = int32_t(i);
       continue;
     }
-    if (lane == 0) uniq[i] = u;
+    int2* seg = rec + i * k + p0;
+    const int P = L <= 256 ? 256 : MID_MAX;
+    for (int e = tid; e < P; e += MID_T) {       // its own list is in the segment (first tier)
+      int2 x = make_int2(int(SENT), 0);
+      if (e < L) x = seg[e];
+      S[e] = x;
+    }
+    __syncthreads();
+    for (int size = 2; size <= P; size <<= 1)
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int q = tid; q < P / 2; q += MID_T) {
+          const int lo = ((q & ~(stride - 1)) << 1) | (q & (stride - 1)), hi = lo | stride;
+          const int2 a = S[lo], b = S[hi];
+          if ((uint32_t(a.x) > uint32_t(b.x)) == ((lo & size) == 0)) { S[lo] = b; S[hi] = a; }
+        }
+        __syncthreads();
+      }
+    // the unique columns left-justified: each thread its run of entries, offsets by a block scan
+    const int per = P / MID_T, e0 = tid * per;
+    int mine = 0;
+    float out[MID_MAX / MID_T];
+    uint32_t col[MID_MAX / MID_T];
+#pragma unroll
+    for (int x = 0; x < MID_MAX / MID_T; ++x) {
+      col[x] = SENT;
+      const int e = e0 + x;
+      if (x >= per) continue;
+      const uint32_t kk = uint32_t(S[e].x);
+      const uint32_t c = kk >> 1;
+      if (kk == SENT || (e > 0 && (uint32_t(S[e - 1].x) >> 1) == c)) continue;
+      const float v = __int_as_float(S[e].y);
+      const uint32_t nk = e + 1 < P ? uint32_t(S[e + 1].x) : SENT;
+      if (nk != SENT && (nk >> 1) == c) {
+        out[x] = pair_value(mode, i, c, true, v, true, __int_as_float(S[e + 1].y), sig2);
+      } else {
+        const bool rev = kk & 1u;
+        out[x] = pair_value(mode, i, c, !rev, v, rev, v, sig2);
+      }
+      col[x] = c;
+      ++mine;
+    }
+    int inc = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) wsum[wib] = inc;
+    __syncthreads();
+    int at = inc - mine, total = 0;
+    for (int w = 0; w < MID_T / 32; ++w) {
+      if (w < wib) at += wsum[w];
+      total += wsum[w];
+    }
+#pragma unroll
+    for (int x = 0; x < MID_MAX / MID_T; ++x)
+      if (col[x] != SENT) seg[at++] = make_int2(int(col[x]), __float_as_int(out[x]));
+    if (tid == 0) uniq[i] = total;
+    __syncthreads();                             // S and wsum are read before the next row
   }
 }
 
@@ -524,9 +611,25 @@ size_t union_workspace_bytes(int64_t n, int k) {
   return c.bytes();
 }
 
+namespace {
+// in-degrees, cursors and the long-row counters are contiguous at the start: one memset
+int clear_counts(const UnionWs& w, cudaStream_t st) {
+  MSC_CUDA_TRY(cudaMemsetAsync(w.indeg, 0, reinterpret_cast<char*>(w.uniq) -
+                                               reinterpret_cast<char*>(w.indeg), st));
+  return MSC_OK;
+}
+}  // namespace
+
+int union_begin(int64_t n, int k, void* ws, int32_t** indeg, cudaStream_t st) {
+  Carver c(ws);
+  UnionWs w = carve_union(c, n, k);
+  *indeg = w.indeg;
+  return clear_counts(w, st);
+}
+
 int launch_union(int mode, const int32_t* idx, const float* vals, const double* sig2, int64_t n,
                  int k, int64_t* indptr, int32_t* indices, float* data, int64_t* nnz_dev,
-                 void* ws, size_t ws_bytes, cudaStream_t st) {
+                 void* ws, size_t ws_bytes, cudaStream_t st, bool counted) {
   if (ws_bytes < union_workspace_bytes(n, k)) {
     set_error("fuzzy union: workspace %zu < %zu bytes", ws_bytes, union_workspace_bytes(n, k));
     return MSC_ERR_WORKSPACE;
@@ -535,23 +638,28 @@ int launch_union(int mode, const int32_t* idx, const float* vals, const double* 
   if (k < 1 || k > MSC_MAX_K) { set_error("fuzzy union: k=%d out of range", k); return MSC_ERR_INVALID_ARG; }
   Carver c(ws);
   UnionWs w = carve_union(c, n, k);
-  // in-degrees, cursors and the long-row counter are contiguous at the start: one memset
-  MSC_CUDA_TRY(cudaMemsetAsync(w.indeg, 0, reinterpret_cast<char*>(w.uniq) - reinterpret_cast<char*>(w.indeg), st));
   const int sms = num_sms();
   const uint32_t magic = div_magic(k);
-  const int g1 = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), int64_t(sms) * 8)));
-  rev_count_kernel<<<g1, 256, 0, st>>>(mode, idx, vals, n, k, magic, w.indeg);
-  MSC_LAUNCH_CHECK();
+  const int rpw = rows_per_warp(n, sms);
+  // the list passes keep at least a warp's worth of entries per group
+  const int lpw = std::max(rpw, std::min(32, int(ceil_div(32, k))));
+  const int g1 = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ceil_div(n, lpw), 8),
+                                                            int64_t(sms) * 16)));
+  if (!counted) {
+    MSC_TRY(clear_counts(w, st));
+    rev_count_kernel<<<g1, 256, 0, st>>>(mode, idx, vals, n, k, magic, lpw, w.indeg);
+    MSC_LAUNCH_CHECK();
+  }
   MSC_TRY(scan_excl<int32_t>(w.indeg, n, w.rptr, w.scan, st));
-  rev_fill_kernel<<<g1, 256, 0, st>>>(mode, idx, vals, n, k, magic, w.rptr, w.cursor, w.rec);
+  rev_fill_kernel<<<g1, 256, 0, st>>>(mode, idx, vals, n, k, magic, lpw, w.rptr, w.cursor, w.rec);
   MSC_LAUNCH_CHECK();
   const int g2 = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, UW), int64_t(sms) * 16)));
   merge_warp_kernel<<<g2, UW * 32, 0, st>>>(mode, n, k, idx, vals, w.rptr, w.rec, sig2, w.uniq,
-                                             w.big, w.nbig);
+                                             w.big, w.nbig, rpw);
   MSC_LAUNCH_CHECK();
-  // rows longer than WARP_MAX: a warp each up to MID_MAX (nbig[0] listed), then the longest
-  // (nbig[1] listed) a block each
-  merge_mid_kernel<<<sms * 4, MID_W * 32, 0, st>>>(mode, n, k, idx, vals, w.rptr, w.rec, sig2,
+  // rows longer than WARP_MAX: a small block each up to MID_MAX (nbig[0] listed), then the longest
+  // (nbig[1] listed) a large block each
+  merge_mid_kernel<<<sms * 12, MID_T, 0, st>>>(mode, n, k, idx, vals, w.rptr, w.rec, sig2,
                                                    w.uniq, w.big, w.nbig, w.huge, w.nbig + 1);
   MSC_LAUNCH_CHECK();
   const size_t bsm = size_t(BLK_SMEM_MAX) * sizeof(int2);

@@ -305,6 +305,10 @@ int launch_fp64_scan(const float* X, int d, const int32_t* perm, const SegDesc* 
 // ---- umap.cu ----
 int launch_smooth_knn(const float* dist, int64_t n, int k, float local_connectivity,
                       float* sigma, float* rho, double* gsum, cudaStream_t st);
+// ρ/σ, the memberships w (n × k) and the in-degrees of the kept edges in one pass over the lists
+int launch_smooth_membership(const int32_t* idx, const float* dist, int64_t n, int k,
+                             float local_connectivity, float* w, int32_t* indeg, double* gsum,
+                             cudaStream_t st);
 int launch_membership(const int32_t* idx, const float* dist, const float* sigma,
                       const float* rho, int64_t n, int k, float* w, cudaStream_t st);
 int launch_distances_csr(const int32_t* idx, const float* dist, int64_t n, int k,
@@ -321,7 +325,11 @@ size_t union_workspace_bytes(int64_t n, int k);
 // mode 0: umap fuzzy union of memberships w; mode 1: gauss kernel from distances + sig2
 int launch_union(int mode, const int32_t* idx, const float* vals, const double* sig2,
                  int64_t n, int k, int64_t* indptr, int32_t* indices, float* data,
-                 int64_t* nnz_dev, void* ws, size_t ws_bytes, cudaStream_t st);
+                 int64_t* nnz_dev, void* ws, size_t ws_bytes, cudaStream_t st,
+                 bool counted = false);
+// the union's in-degree counters, cleared, for a caller that counts the kept edges itself (kept =
+// value > 0, another cell) and then passes counted = true
+int union_begin(int64_t n, int k, void* ws, int32_t** indeg, cudaStream_t st);
 
 
 // ---- bbknn.cu ----

@@ -19,6 +19,11 @@
 
 namespace msc {
 
+__device__ __forceinline__ double warp_sum_d(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+  return v;
+}
+
 // ------------------------------------------------------------------------------------------------
 // cosine: x̂ = float32(x · 1/sqrt(Σ x_t²)), the sum in FP64 in dimension order (thread per row)
 // ------------------------------------------------------------------------------------------------
@@ -81,15 +86,18 @@ __global__ void colsum_partial_kernel(const float* __restrict__ X, const SegDesc
   if (bad) atomicAdd(reinterpret_cast<unsigned long long*>(nonfinite), 1ull);
 }
 
+// one warp per (sample, column), a fixed order: lane l adds blocks l, l + 32, ..., then the lanes
+// as a tree (one thread adding 256 partials one after another took 15 us at any size)
 __global__ void colmean_finalize_kernel(const double* __restrict__ partial,
                                         const SegDesc* __restrict__ seg, int nseg, int d, int nb,
                                         double* __restrict__ mean) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nseg * d) return;
-  int s = i / d, t = i % d;
+  const int64_t i = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  if (i >= int64_t(nseg) * d) return;
+  const int s = int(i / d), t = int(i % d);
   double a = 0.0;
-  for (int b = 0; b < nb; ++b) a += partial[(int64_t(s) * nb + b) * d + t];
-  mean[i] = seg[s].n > 0 ? a / double(seg[s].n) : 0.0;
+  for (int b = lane_id(); b < nb; b += 32) a += partial[(int64_t(s) * nb + b) * d + t];
+  a = warp_sum_d(a);
+  if (lane_id() == 0) mean[i] = seg[s].n > 0 ? a / double(seg[s].n) : 0.0;
 }
 
 size_t colmean_partial_elems(int nseg, int d, int nb) { return size_t(nseg) * nb * d; }
@@ -101,7 +109,7 @@ int launch_colmean(const float* X, const SegDesc* seg, int nseg, int64_t max_seg
   dim3 grid(nb, nseg);
   colsum_partial_kernel<<<grid, 256, 0, st>>>(X, seg, d, nb, partial, nonfinite);
   MSC_LAUNCH_CHECK();
-  colmean_finalize_kernel<<<unsigned(ceil_div(int64_t(nseg) * d, 256)), 256, 0, st>>>(
+  colmean_finalize_kernel<<<unsigned(ceil_div(int64_t(nseg) * d, 8)), 256, 0, st>>>(
       partial, seg, nseg, d, nb, mean);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
@@ -150,12 +158,6 @@ template <> __device__ __forceinline__ __nv_bfloat16 to_op<__nv_bfloat16>(double
 }
 __device__ __forceinline__ double op_val(__half v) { return double(__half2float(v)); }
 __device__ __forceinline__ double op_val(__nv_bfloat16 v) { return double(__bfloat162float(v)); }
-
-__device__ __forceinline__ double warp_sum_d(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  return v;
-}
-
 
 // block-level max of 5 non-negative fields, then one atomicMax per field per block
 __device__ __forceinline__ void block_keymax(float (&m)[5], KeyMax* km) {

@@ -33,27 +33,25 @@ __global__ void dist_sum_partial_kernel(const float* __restrict__ dist, int64_t 
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
+// one warp, a fixed order: lane l adds partials l, l + 32, ..., then the lanes as a tree (one
+// thread adding 1,024 partials one after another took 28 us)
 __global__ void dist_sum_final_kernel(const double* __restrict__ partial, int nb,
                                       double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double a = 0.0;
-    for (int b = 0; b < nb; ++b) a += partial[b];
-    *out = a;
-  }
+  double a = 0.0;
+  for (int b = threadIdx.x; b < nb; b += 32) a += partial[b];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(FULL, a, o);
+  if (threadIdx.x == 0) *out = a;
 }
 
-__global__ void __launch_bounds__(SK_THREADS)
-smooth_knn_kernel(const float* __restrict__ dist, int64_t n, int k, float local_connectivity,
-                  const double* __restrict__ gsum, float* __restrict__ sigma,
-                  float* __restrict__ rho_out) {
-  extern __shared__ float sd[];                    // [SK_THREADS][k]
-  const int64_t row0 = int64_t(blockIdx.x) * SK_THREADS;
-  const int nrows = int(min64(SK_THREADS, n - row0));
-  for (int e = threadIdx.x; e < nrows * k; e += SK_THREADS) sd[e] = dist[row0 * k + e];
-  __syncthreads();
-  if (threadIdx.x >= nrows) return;
-  const int64_t i = row0 + threadIdx.x;
-  const float* D = sd + threadIdx.x * k;
+// rho and sigma of one row D[0..k) by a group of L lanes (all of them return both; T[0..k) is the
+// group's scratch, unused for L = 1)
+template <int L>
+__device__ __forceinline__ void smooth_row(const float* D, float* T, int k, int64_t n,
+                                           float local_connectivity, const double* gsum,
+                                           float& sigma, float& rho_out) {
+  const int sub = lane_id() & (L - 1);
+  static_assert(L == 1 || L == 2 || L == 4 || L == 8 || L == 16, "part of a warp");
+  const unsigned group = ((1u << L) - 1u) << (lane_id() & ~(L - 1));
   const double target = log2(double(k));
   // rho
   int nz = 0;
@@ -82,18 +80,22 @@ smooth_knn_kernel(const float* __restrict__ dist, int64_t n, int k, float local_
     for (int j = 0; j < k; ++j) if (D[j] > 0.f) m = fmaxf(m, D[j]);
     rho = m;
   }
-  // bisection for sigma (float32 state, column order)
+  // Bisection for sigma (float32 state, column order).  A step's sum decides two things: whether
+  // it is within the tolerance of the target, and on which side it lies.  Most steps are far from
+  // the target, and there a float32 estimate decides both: __expf is within 2 + 1.173|x| ulp, so a
+  // term e^-x is within 3e-7 of the exact one, its argument's rounding adds 1e-7 and the exact
+  // term's own rounding 6e-8 (1e-6 is taken), and each of the k-2 additions of either sum errs by
+  // at most 2^-24 of the sum.  Within that margin of the tolerance (or NaN) the step's sum is
+  // evaluated as defined: exp in FP64, rounded once per term, added in column order.  Of about 18
+  // steps 2 or 3 need it.  The estimated steps run in a loop of their own, so that the rows of a
+  // warp meet at the FP64 steps instead of each taking them at its own step number.  The FP64
+  // exponentials bound this kernel at large n: with the memberships and the in-degrees in the same
+  // pass 1.09 -> 0.54 ms at 1.3M cells, k = 15.  At small n it is one row's chain of steps: L = 8
+  // lanes a row, 53 -> 19 us at 500 cells.
   float lo = 0.f, hi = __int_as_float(0x7f800000), mid = 1.f;
-  for (int it = 0; it < 64; ++it) {
-    float psum = 0.f;
-    for (int j = 1; j < k; ++j) {
-      const float dd = __fsub_rn(D[j], rho);
-      if (dd > 0.f) psum = __fadd_rn(psum, exp_f32(-__fdiv_rn(dd, mid)));
-      else psum = __fadd_rn(psum, 1.f);
-    }
-    const double p64 = double(psum);
-    if (fabs(p64 - target) < double(SMOOTH_K_TOLERANCE)) break;
-    if (p64 > target) {
+  const float targetf = float(target);
+  auto move = [&](bool above) {
+    if (above) {
       hi = mid;
       mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
     } else {
@@ -101,6 +103,42 @@ smooth_knn_kernel(const float* __restrict__ dist, int64_t n, int k, float local_
       if (isinf(hi)) mid = __fmul_rn(mid, 2.f);
       else mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
     }
+  };
+  for (int it = 0; it < 64; ++it) {
+    bool close = false;
+    for (; it < 64; ++it) {
+      const float inv = __frcp_rn(mid);
+      float est = 0.f;
+#pragma unroll 4
+      for (int j = 1 + sub; j < k; j += L) {
+        const float dd = __fsub_rn(D[j], rho);
+        est += dd > 0.f ? __expf(-dd * inv) : 1.f;
+      }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) est += __shfl_xor_sync(group, est, o);
+      const float margin = 1.2e-5f + float(k - 1) * (1e-6f + 1.3e-7f * est) + 1e-6f * targetf;
+      if (!(fabsf(est - targetf) > margin)) { close = true; break; }
+      move(est > targetf);
+    }
+    if (!close) break;                       // 64 steps
+    auto term = [&](int j) {
+      const float dd = __fsub_rn(D[j], rho);
+      return dd > 0.f ? exp_f32(-__fdiv_rn(dd, mid)) : 1.f;
+    };
+    float psum = 0.f;
+    if (L == 1) {
+#pragma unroll 2
+      for (int j = 1; j < k; ++j) psum = __fadd_rn(psum, term(j));
+    } else {
+      for (int j = 1 + sub; j < k; j += L) T[j] = term(j);
+      __syncwarp(group);
+#pragma unroll 4
+      for (int j = 1; j < k; ++j) psum = __fadd_rn(psum, T[j]);
+      __syncwarp(group);
+    }
+    const double p64 = double(psum);
+    if (fabs(p64 - target) < double(SMOOTH_K_TOLERANCE)) break;
+    move(p64 > target);
   }
   float result = mid;
   if (rho > 0.f) {
@@ -112,8 +150,53 @@ smooth_knn_kernel(const float* __restrict__ dist, int64_t n, int k, float local_
     const double fl = MIN_K_DIST_SCALE * (*gsum / (double(n) * double(k)));
     if (double(result) < fl) result = __double2float_rn(fl);
   }
-  sigma[i] = result;
-  rho_out[i] = rho;
+  sigma = result;
+  rho_out = rho;
+}
+
+// FUSED: the memberships and the in-degrees of the kept edges as well (the rows are staged
+// already): w replaces the staged distances row by row and leaves in memory order.  L lanes a row.
+template <bool FUSED, int L>
+__global__ void __launch_bounds__(SK_THREADS)
+smooth_knn_kernel(const float* __restrict__ dist, int64_t n, int k, float local_connectivity,
+                  const double* __restrict__ gsum, float* __restrict__ sigma,
+                  float* __restrict__ rho_out, const int32_t* __restrict__ idx,
+                  float* __restrict__ w, int32_t* __restrict__ indeg) {
+  extern __shared__ float sd[];                    // [ROWS][k], and a scratch row each for L > 1
+  constexpr int ROWS = SK_THREADS / L;
+  const int64_t row0 = int64_t(blockIdx.x) * ROWS;
+  const int nrows = int(min64(ROWS, n - row0));
+  for (int e = threadIdx.x; e < nrows * k; e += SK_THREADS) sd[e] = dist[row0 * k + e];
+  __syncthreads();
+  const int r = threadIdx.x / L, sub = threadIdx.x & (L - 1);
+  if (r < nrows) {
+    float* D = sd + r * k;
+    float sg, rho;
+    smooth_row<L>(D, sd + (ROWS + r) * k, k, n, local_connectivity, gsum, sg, rho);
+    if (!FUSED) {
+      if (sub == 0) {
+        sigma[row0 + r] = sg;
+        rho_out[row0 + r] = rho;
+      }
+    } else {
+      if (L > 1)                                   // the group has read D
+        __syncwarp(((1u << L) - 1u) << (lane_id() & ~(L - 1)));
+      for (int j = sub; j < k; j += L) {
+        const float dd = __fsub_rn(D[j], rho);
+        D[j] = (dd <= 0.f || sg == 0.f) ? 1.f : exp_f32(-__fdiv_rn(dd, sg));
+      }
+    }
+  }
+  if (FUSED) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < nrows * k; e += SK_THREADS) {
+      const int64_t i = row0 + e / k;
+      const int32_t j = idx[row0 * k + e];
+      const float v = j == i ? 0.f : sd[e];
+      w[row0 * k + e] = v;
+      if (j != i && j >= 0 && j < n && v > 0.f) atomicAdd(&indeg[j], 1);
+    }
+  }
 }
 
 __global__ void membership_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dist,
@@ -197,21 +280,56 @@ gauss_sigma_kernel(const float* __restrict__ dist, int64_t n, int k, double* __r
 
 }  // namespace
 
-int launch_smooth_knn(const float* dist, int64_t n, int k, float local_connectivity,
-                      float* sigma, float* rho, double* gsum, cudaStream_t st) {
-  // gsum: workspace of >= 1 + 1024 doubles (total at [0], partials after)
+namespace {
+// gsum: workspace of >= 1 + 1024 doubles (total at [0], partials after)
+int launch_dist_sum(const float* dist, int64_t n, int k, double* gsum, cudaStream_t st) {
   const int nb = int(std::min<int64_t>(1024, std::max<int64_t>(1, ceil_div(n * k, 4096))));
   dist_sum_partial_kernel<<<nb, 256, 0, st>>>(dist, n * k, gsum + 1);
   MSC_LAUNCH_CHECK();
   dist_sum_final_kernel<<<1, 32, 0, st>>>(gsum + 1, nb, gsum);
   MSC_LAUNCH_CHECK();
-  const size_t smem = size_t(SK_THREADS) * k * sizeof(float);
-  if (smem > 48 * 1024)
-    MSC_CUDA_TRY(raise_smem_cap(smooth_knn_kernel, smem));
-  smooth_knn_kernel<<<unsigned(ceil_div(n, SK_THREADS)), SK_THREADS, smem, st>>>(
-      dist, n, k, local_connectivity, gsum, sigma, rho);
+  return MSC_OK;
+}
+
+template <bool FUSED, int L>
+int launch_smooth_l(const float* dist, int64_t n, int k, float lc, const double* gsum,
+                    float* sigma, float* rho, const int32_t* idx, float* w, int32_t* indeg,
+                    cudaStream_t st) {
+  constexpr int ROWS = SK_THREADS / L;
+  const size_t smem = size_t(ROWS) * (L > 1 ? 2 : 1) * k * sizeof(float);
+  if (smem > 48 * 1024) MSC_CUDA_TRY(raise_smem_cap(smooth_knn_kernel<FUSED, L>, smem));
+  smooth_knn_kernel<FUSED, L><<<unsigned(ceil_div(n, ROWS)), SK_THREADS, smem, st>>>(
+      dist, n, k, lc, gsum, sigma, rho, idx, w, indeg);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
+}
+
+// Eight lanes a row while that is at most SK_WIDE_WARPS warps per SM: below it the rows do not
+// fill the SMs and a row's chain of steps is the time; above it the lanes' ordered sums are extra
+// work.
+constexpr int64_t SK_WIDE_WARPS = 64;
+template <bool FUSED>
+int launch_smooth(const float* dist, int64_t n, int k, float lc, const double* gsum, float* sigma,
+                  float* rho, const int32_t* idx, float* w, int32_t* indeg, cudaStream_t st) {
+  if (n <= SK_WIDE_WARPS * 4 * num_sms())
+    return launch_smooth_l<FUSED, 8>(dist, n, k, lc, gsum, sigma, rho, idx, w, indeg, st);
+  return launch_smooth_l<FUSED, 1>(dist, n, k, lc, gsum, sigma, rho, idx, w, indeg, st);
+}
+}  // namespace
+
+int launch_smooth_knn(const float* dist, int64_t n, int k, float local_connectivity,
+                      float* sigma, float* rho, double* gsum, cudaStream_t st) {
+  MSC_TRY(launch_dist_sum(dist, n, k, gsum, st));
+  return launch_smooth<false>(dist, n, k, local_connectivity, gsum, sigma, rho, nullptr, nullptr,
+                              nullptr, st);
+}
+
+int launch_smooth_membership(const int32_t* idx, const float* dist, int64_t n, int k,
+                             float local_connectivity, float* w, int32_t* indeg, double* gsum,
+                             cudaStream_t st) {
+  MSC_TRY(launch_dist_sum(dist, n, k, gsum, st));
+  return launch_smooth<true>(dist, n, k, local_connectivity, gsum, nullptr, nullptr, idx, w, indeg,
+                             st);
 }
 
 int launch_membership(const int32_t* idx, const float* dist, const float* sigma,
