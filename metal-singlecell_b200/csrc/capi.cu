@@ -394,9 +394,11 @@ KnnWs carve_knn(Carver& c, const Problem& P) {
     w.order_ws = c.take<unsigned char>(w.order_ws_bytes);
   }
   if (P.refine) {
-    w.flags = c.take<int32_t>(P.npacked);
-    w.S = c.take<int64_t>(P.npacked + 1);
-    w.scan_scratch = c.take<int64_t>(scan_i32_scratch_elems(P.npacked));
+    if (!P.dense) {
+      w.flags = c.take<int32_t>(P.npacked);
+      w.S = c.take<int64_t>(P.npacked + 1);
+      w.scan_scratch = c.take<int64_t>(scan_i32_scratch_elems(P.npacked));
+    }
     w.qmap = c.take<int32_t>(P.n);
     w.items3 = c.take<WorkItem>(P.ntiles);
     w.A3 = c.take<uint16_t>(size_t(P.n) * P.L3.kp);
@@ -449,18 +451,12 @@ int decode_tile_config(int32_t code, const Problem& P, TcConfig& cfg) {
 int launch_set_stat(Ctl* ctl, int idx, int64_t v, cudaStream_t st);
 
 // The kNN pipeline after the sample table (w.seg) is in place.
+// single: one sample, whose table the pipeline writes itself.
 int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, float* knn_dist,
-            int32_t tile_code, cudaStream_t st) {
+            int32_t tile_code, cudaStream_t st, bool single) {
   stage_mark(st, 0);
-  MSC_CUDA_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), st));
-  MSC_CUDA_TRY(cudaMemsetAsync(w.km, 0, sizeof(KeyMax), st));
-  MSC_TRY(launch_set_stat(w.ctl, MSC_STAT_PRECISION, P.candidates ? P.prec : -1, st));
   const bool cosine = P.metric == MSC_METRIC_COSINE;
   const float* Xu = X;
-  if (cosine) {
-    MSC_TRY(launch_normalize(X, w.Xn, P.n, P.d, &w.ctl->stats[MSC_STAT_NONFINITE], st));
-    Xu = w.Xn;
-  }
   const bool tc = P.candidates && P.k > 1 && P.prec != PREC_FP32;
   TcConfig cfg{};
   if (tc) MSC_TRY(decode_tile_config(tile_code, P, cfg));
@@ -469,8 +465,27 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
   const int kscan = split > 1 ? P.kper : P.kprime;
   const bool pair_items = tc && cfg.pair;
   const int64_t n_items = pair_items ? P.nptiles : P.ntiles;
-  MSC_TRY(launch_build_items(w.seg, P.nseg, n_items, pair_items ? 2 * QTILE : QTILE, w.items, w.ctl,
-                             st));
+  const int item_rows = pair_items ? 2 * QTILE : QTILE;
+  // the uncertified rows go to the refine pass as flags (packed order: neighbouring rows share
+  // most of their mask) or, without masks, as a list
+  int32_t* flags = P.refine && !P.dense ? w.flags : nullptr;
+  int32_t* fail_list = P.refine && P.dense ? w.qmap : nullptr;
+  if (single) {
+    MSC_TRY(launch_begin_single(P.n, P.npacked, n_items, item_rows, P.candidates ? P.prec : -1,
+                                P.stride, w.ctl, w.km, w.km3, w.seg, w.items,
+                                P.dense ? w.perm : nullptr, flags, st));
+  } else {
+    MSC_CUDA_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), st));
+    MSC_CUDA_TRY(cudaMemsetAsync(w.km, 0, sizeof(KeyMax), st));
+    if (flags) MSC_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int32_t) * P.npacked, st));
+    if (w.km3) MSC_CUDA_TRY(cudaMemsetAsync(w.km3, 0, sizeof(KeyMax), st));
+    MSC_TRY(launch_set_stat(w.ctl, MSC_STAT_PRECISION, P.candidates ? P.prec : -1, st));
+    MSC_TRY(launch_build_items(w.seg, P.nseg, n_items, item_rows, w.items, w.ctl, st));
+  }
+  if (cosine) {
+    MSC_TRY(launch_normalize(X, w.Xn, P.n, P.d, &w.ctl->stats[MSC_STAT_NONFINITE], st));
+    Xu = w.Xn;
+  }
   // pruning needs single-CTA work items over 256-key tiles (or the FP32 SIMT kernel)
   const bool prune = P.prune && tc && !cfg.pair && cfg.bn == PRUNE_BN;
   const bool prune32 = P.prune && P.candidates && P.k > 1 && P.prec == PREC_FP32;
@@ -481,9 +496,7 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
   if (const char* pe = std::getenv("MSC_B200_ORDER_PROJ")) proj_from = std::atoi(pe);
   const bool proj = w.Xo && levels > proj_from && proj_from >= 0;
   if (proj) MSC_TRY(launch_project(Xu, P.n, P.d, w.Xo, st));
-  if (P.dense)
-    MSC_TRY(launch_plain_order(w.seg, P.nseg, P.npacked, P.stride, w.perm, st));
-  else
+  if (!P.dense)
     MSC_TRY(launch_order(Xu, P.d, w.seg, P.nseg, P.npacked, levels,
                        ORDER_LEAF, w.perm, (prune || prune32) ? w.pr.leaf : nullptr, w.order_ws,
                        w.order_ws_bytes, st, P.max_seg, proj ? w.Xo : nullptr, ORDER_PROJ_D,
@@ -576,21 +589,24 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
     }
   }
   stage_mark(st, 4);
-  if (P.refine) MSC_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int32_t) * P.npacked, st));
   MSC_TRY(launch_rerank(Xu, P.d, w.perm, w.seg, P.nseg, P.npacked, w.cand_idx, w.cand_thr,
                         P.kprime, P.kprime, w.qs, w.km, P.prec, P.L.kmma, P.k, cosine, knn_idx,
                         knn_dist, w.fail_rows, w.ctl, nullptr, nullptr, 0,
-                        P.refine ? w.flags : nullptr, st, split, P.n));
+                        flags, st, split, P.n, fail_list));
   if (P.refine) {
     // the rows the one-term candidates could not certify, again with the three-term split
     // with pruning, a small refine set is split over key ranges (prune.cu)
     const bool parts = w.pr.part != nullptr && (prune || P.dense);
-    MSC_TRY(launch_refine_plan(w.flags, P.npacked, w.seg, P.nseg, w.qmap, w.items3, w.S,
+    if (P.dense)
+      MSC_TRY(launch_refine_list_plan(P.n, w.items3, w.ctl, REFINE_SPLIT, w.pr.max_split_items,
+                                      st));
+    else
+      MSC_TRY(launch_refine_plan(w.flags, P.npacked, w.seg, P.nseg, w.qmap, w.items3, w.S,
                                w.scan_scratch, w.ctl, parts ? REFINE_SPLIT : 1,
                                parts ? w.pr.max_split_items : 0, st));
-    MSC_CUDA_TRY(cudaMemsetAsync(w.km3, 0, sizeof(KeyMax), st));
     MSC_TRY(launch_pack_tc(PREC_BF16X3, Xu, w.perm, w.seg, P.nseg, w.mean, P.d, P.npacked,
-                           nullptr, nullptr, 0, nullptr, w.B3, w.qs3, w.km3, w.ctl, st));
+                           nullptr, nullptr, 0, nullptr, w.B3, w.qs3, w.km3, w.ctl, st,
+                           &w.ctl->n_refine));
     MSC_TRY(launch_pack_tc(PREC_BF16X3, Xu, w.perm, w.seg, P.nseg, w.mean, P.d, P.npacked,
                            w.qmap, &w.ctl->n_refine, P.n, w.A3, nullptr, nullptr, nullptr, w.ctl,
                            st));
@@ -665,8 +681,11 @@ int launch_set_stat(Ctl* ctl, int idx, int64_t v, cudaStream_t st) {
   return MSC_OK;
 }
 
-__global__ void store_nnz_kernel(const int64_t* __restrict__ indptr, int64_t n, Ctl* ctl) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) ctl->stats[MSC_STAT_CONN_NNZ] = indptr[n];
+// the graph's entry count into the stats block, and the block to the caller
+__global__ void finish_stats_kernel(const int64_t* __restrict__ indptr, int64_t n,
+                                    const Ctl* __restrict__ ctl, int64_t* __restrict__ stats) {
+  const int t = threadIdx.x;
+  if (t < MSC_STATS_LEN) stats[t] = t == MSC_STAT_CONN_NNZ ? indptr[n] : ctl->stats[t];
 }
 
 cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
@@ -759,8 +778,7 @@ int msc_knn(const float* X_dev, int64_t n, int32_t d, int32_t k, int32_t metric,
     return MSC_ERR_WORKSPACE;
   }
   cudaStream_t st = as_stream(stream);
-  MSC_TRY(launch_single_segment(w.seg, n, st));
-  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, 0, st));
+  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, 0, st, true));
   return copy_stats(w, stats_dev, st);
 }
 
@@ -814,8 +832,7 @@ int msc_neighbors_ex(const float* X_dev, int64_t n, int32_t d, int32_t k, int32_
     return MSC_ERR_WORKSPACE;
   }
   cudaStream_t st = as_stream(stream);
-  MSC_TRY(launch_single_segment(w.seg, n, st));
-  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, 0, st));
+  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, 0, st, true));
   MSC_TRY(launch_distances_csr(knn_idx_dev, knn_dist_dev, n, k, dist_indptr_dev, dist_indices_dev,
                                dist_data_dev, st));
   // the distances CSR (and the kNN lists) are final here: a caller can copy them out on another
@@ -836,10 +853,12 @@ int msc_neighbors_ex(const float* X_dev, int64_t n, int32_t d, int32_t k, int32_
     MSC_TRY(launch_union(1, knn_idx_dev, knn_dist_dev, g.sig2, n, k, conn_indptr_dev,
                          conn_indices_dev, conn_data_dev, nullptr, g.uws, g.uws_bytes, st));
   }
-  store_nnz_kernel<<<1, 32, 0, st>>>(conn_indptr_dev, n, w.ctl);
-  MSC_LAUNCH_CHECK();
+  if (stats_dev) {
+    finish_stats_kernel<<<1, 32, 0, st>>>(conn_indptr_dev, n, w.ctl, stats_dev);
+    MSC_LAUNCH_CHECK();
+  }
   stage_mark(st, 7);
-  return copy_stats(w, stats_dev, st);
+  return MSC_OK;
 }
 
 size_t msc_batched_workspace_bytes(const int64_t* offsets_host, int32_t n_samples, int32_t d,
@@ -918,7 +937,7 @@ int msc_batched_knn(const float* X_dev, const int64_t* offsets_host, int32_t n_s
     return MSC_ERR_WORKSPACE;
   }
   cudaStream_t st = as_stream(stream);
-  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, tile_config, st));
+  MSC_TRY(run_knn(P, w, X_dev, knn_idx_dev, knn_dist_dev, tile_config, st, false));
   return copy_stats(w, stats_dev, st);
 }
 

@@ -93,12 +93,13 @@ size_t colmean_partial_elems(int nseg, int d, int nb);
 int launch_maxnorm(const float* X, const SegDesc* seg, int nseg, const double* mean, int d,
                    int64_t npacked, Ctl* ctl, cudaStream_t st);
 // packed row p holds original row perm[p] (-1: padding) of the sample seg[find_seg(p)]
+// gate (optional, device): nothing is packed when it is 0
 // rows/nrows: pack only the listed packed rows (device count, at most max_rows) into output rows
 // 0..; null: every packed row.  Aop or Bop may be null; qs/km (key statistics) may be null.
 int launch_pack_tc(int prec, const float* X, const int32_t* perm, const SegDesc* seg, int nseg,
                    const double* mean, int d, int64_t npacked, const int32_t* rows,
                    const int32_t* nrows, int64_t max_rows, void* Aop, void* Bop, QStat* qs,
-                   KeyMax* km, const Ctl* ctl, cudaStream_t st);
+                   KeyMax* km, const Ctl* ctl, cudaStream_t st, const int32_t* gate = nullptr);
 int launch_pack_fp32(const float* X, const int32_t* perm, const SegDesc* seg, int nseg,
                      const double* mean, int d, int dpad, int64_t npacked, float* A32, float* sq32,
                      QStat* qs, KeyMax* km, cudaStream_t st);
@@ -115,13 +116,16 @@ int launch_order(const float* X, int d, const SegDesc* seg, int nseg, int64_t np
                  int leaf, int32_t* perm, int32_t* leaf_out, void* ws, size_t ws_bytes,
                  cudaStream_t st, int64_t max_seg, const float* Xp = nullptr, int dp = 0,
                  int proj_from = 0);
-// the order of the full scan: cell (j·stride) mod n of a sample at its j-th position (stride
-// coprime to every sample's size, 1: plain order)
-int launch_plain_order(const SegDesc* seg, int nseg, int64_t npacked, int64_t stride,
-                       int32_t* perm, cudaStream_t st);
 size_t scan_i32_scratch_elems(int64_t n);
 int scan_excl_i32(const int32_t* in, int64_t n, int64_t* out, int64_t* scratch, cudaStream_t st);
 int launch_single_segment(SegDesc* seg, int64_t n, cudaStream_t st);
+// the start of a single-sample pipeline: ctl, km, km3, flags cleared (km3, flags may be null),
+// sample table and work items of `rows` query rows written; perm (optional): the full scan's
+// order, cell (j·stride) mod n at position j (stride coprime to n, 1: plain order)
+int launch_begin_single(int64_t n, int64_t npacked, int64_t n_items, int rows,
+                        int64_t stat_precision, int64_t stride, Ctl* ctl, KeyMax* km, KeyMax* km3,
+                        SegDesc* seg, WorkItem* items, int32_t* perm, int32_t* flags,
+                        cudaStream_t st);
 // one work item per `rows` (128 or 256) query rows of every sample
 int launch_build_items(const SegDesc* seg, int nseg, int64_t n_items, int rows, WorkItem* items,
                        Ctl* ctl, cudaStream_t st);
@@ -288,7 +292,12 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
                   const QStat* qs, const KeyMax* km, int prec, int kmma, int k, int cosine,
                   int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,
                   const int32_t* rows, const int32_t* nrows, int64_t max_rows,
-                  int32_t* fail_flags, cudaStream_t st, int n_thr = 1, int64_t thr_stride = 0);
+                  int32_t* fail_flags, cudaStream_t st, int n_thr = 1, int64_t thr_stride = 0,
+                  int32_t* fail_list = nullptr);
+// the refine plan of a single sample whose uncertified rows the re-rank listed itself (qmap, any
+// order; ctl->n_refine of them): no flags to scan
+int launch_refine_list_plan(int64_t n, WorkItem* items, Ctl* ctl, int split, int max_split_items,
+                            cudaStream_t st);
 // refine plan: compact the flagged packed rows (sorted) into qmap, count them (ctl->n_refine)
 // and cut them into per-sample query tiles (items, ctl->n_items_refine); S: npacked+1 int64
 // split > 1: when there are at most max_split_items refine items, each becomes `split` work

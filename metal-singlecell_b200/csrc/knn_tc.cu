@@ -560,6 +560,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   const int acc_cols = DUAL ? P.bn / 2 : P.bn;          // TMEM columns of one accumulator
   const uint32_t tmem_cols = uint32_t(NACC * acc_cols);
   const int n_items = P.n_items_dev ? *P.n_items_dev : P.n_items;
+  if (n_items <= 0) return;                             // a refine pass without rows
   // the producer drives the walk from the sorted list and ends it early (single CTAs only)
   const bool ordered = !PAIR && !P.near_only && P.qmap == nullptr && P.vlist != nullptr &&
                        *P.vok != 0;

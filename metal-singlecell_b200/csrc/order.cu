@@ -162,17 +162,6 @@ __global__ void order_init_kernel(const SegDesc* __restrict__ seg, int nseg, int
   }
 }
 
-// positions of a sample filled with its cells stride apart (see launch_plain_order)
-__global__ void plain_order_kernel(const SegDesc* __restrict__ seg, int nseg, int64_t npacked,
-                                   int64_t stride, int32_t* __restrict__ perm) {
-  for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < npacked;
-       p += int64_t(gridDim.x) * blockDim.x) {
-    const int s = find_seg(seg, nseg, p);
-    const int64_t j = p - seg[s].poff;
-    perm[p] = j < seg[s].n ? int32_t(seg[s].off + (j * stride) % seg[s].n) : -1;
-  }
-}
-
 // atomicMax of key into best[s]; the lanes of a warp that share node s combine first (positions
 // are contiguous, so a warp almost always lies inside one node and issues a single atomic)
 __device__ __forceinline__ void warp_far_max(unsigned long long* best, int s, bool active,
@@ -835,15 +824,6 @@ size_t order_workspace_bytes(int64_t npacked, int d, int leaf) {
   c.take<double>(size_t(max_split_nodes(npacked, leaf)) * (2 * d + 2));   // side sums, counts
   c.take<int32_t>(size_t(max_split_nodes(npacked, leaf)));            // split-node starts by id
   return c.bytes();
-}
-
-int launch_plain_order(const SegDesc* seg, int nseg, int64_t npacked, int64_t stride,
-                       int32_t* perm, cudaStream_t st) {
-  const int grid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(npacked, OR_T),
-                                                              int64_t(num_sms()) * 8)));
-  plain_order_kernel<<<grid, OR_T, 0, st>>>(seg, nseg, npacked, stride, perm);
-  MSC_LAUNCH_CHECK();
-  return MSC_OK;
 }
 
 int launch_order(const float* X, int d, const SegDesc* seg, int nseg, int64_t npacked, int levels,

@@ -190,7 +190,8 @@ __global__ void pack_tc_kernel(const float* __restrict__ X, const int32_t* __res
                                const int32_t* __restrict__ nrows, T* __restrict__ Aop,
                                T* __restrict__ Bop, QStat* __restrict__ qs,
                                KeyMax* __restrict__ km, const Ctl* __restrict__ ctl,
-                               double pad_term) {
+                               double pad_term, const int32_t* __restrict__ gate) {
+  if (gate && *gate == 0) return;               // nothing to refine: no operands either
   const int lane = lane_id();
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const double f = op_scale(prec, ctl);
@@ -274,7 +275,7 @@ __global__ void pack_tc_kernel(const float* __restrict__ X, const int32_t* __res
 int launch_pack_tc(int prec, const float* X, const int32_t* perm, const SegDesc* seg, int nseg,
                    const double* mean, int d, int64_t npacked, const int32_t* rows,
                    const int32_t* nrows, int64_t max_rows, void* Aop, void* Bop, QStat* qs,
-                   KeyMax* km, const Ctl* ctl, cudaStream_t st) {
+                   KeyMax* km, const Ctl* ctl, cudaStream_t st, const int32_t* gate) {
   const OpLayout L = op_layout(prec, d);
   const int64_t n_out = rows ? max_rows : npacked;
   int blocks = int(std::min<int64_t>(ceil_div(n_out, 8), int64_t(num_sms()) * 16));
@@ -284,18 +285,19 @@ int launch_pack_tc(int prec, const float* X, const int32_t* perm, const SegDesc*
       pack_tc_kernel<__nv_bfloat16, 3><<<blocks, 256, 0, st>>>(
           X, perm, seg, nseg, mean, d, L.kp, prec, npacked, rows, nrows,
           static_cast<__nv_bfloat16*>(Aop), static_cast<__nv_bfloat16*>(Bop), qs, km, ctl,
-          PAD_NORM_TERM_BF16);
+          PAD_NORM_TERM_BF16, gate);
       break;
     case PREC_BF16:
       pack_tc_kernel<__nv_bfloat16, 1><<<blocks, 256, 0, st>>>(
           X, perm, seg, nseg, mean, d, L.kp, prec, npacked, rows, nrows,
           static_cast<__nv_bfloat16*>(Aop), static_cast<__nv_bfloat16*>(Bop), qs, km, ctl,
-          PAD_NORM_TERM_BF16);
+          PAD_NORM_TERM_BF16, gate);
       break;
     case PREC_FP16:
       pack_tc_kernel<__half, 1><<<blocks, 256, 0, st>>>(
           X, perm, seg, nseg, mean, d, L.kp, prec, npacked, rows, nrows,
-          static_cast<__half*>(Aop), static_cast<__half*>(Bop), qs, km, ctl, PAD_NORM_TERM_FP16);
+          static_cast<__half*>(Aop), static_cast<__half*>(Bop), qs, km, ctl, PAD_NORM_TERM_FP16,
+          gate);
       break;
     default:
       set_error("pack_tc: bad precision %d", prec);
@@ -380,6 +382,69 @@ __global__ void single_segment_kernel(SegDesc* seg, int64_t n) {
 
 int launch_single_segment(SegDesc* seg, int64_t n, cudaStream_t st) {
   single_segment_kernel<<<1, 1, 0, st>>>(seg, n);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+// The start of a single-sample pipeline in one launch: control block, key maxima, refine flags and
+// counters cleared, sample table, work items and (perm set) the full scan's order written.  They
+// were up to eight launches of about 2 us of kernel and gap and 4 us of host time each.
+__global__ void begin_single_kernel(int64_t n, int64_t npacked, int64_t n_items, int rows,
+                                    int64_t stat_precision, int64_t stride, Ctl* ctl, KeyMax* km,
+                                    KeyMax* km3, SegDesc* seg, WorkItem* items, int32_t* perm,
+                                    int32_t* flags) {
+  const int64_t t0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int64_t nt = int64_t(gridDim.x) * blockDim.x;
+  if (blockIdx.x == 0) {
+    for (int i = threadIdx.x; i < int(sizeof(Ctl) / 4); i += blockDim.x)
+      reinterpret_cast<int32_t*>(ctl)[i] = 0;
+    if (threadIdx.x < int(sizeof(KeyMax) / 4)) {
+      reinterpret_cast<int32_t*>(km)[threadIdx.x] = 0;
+      if (km3) reinterpret_cast<int32_t*>(km3)[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ctl->stats[MSC_STAT_PRECISION] = stat_precision;
+      ctl->n_items = int32_t(n_items);
+      SegDesc s;
+      s.off = 0;
+      s.n = n;
+      s.poff = 0;
+      s.padlen = npacked;
+      s.tile0 = 0;
+      s.ntiles = (n + QTILE - 1) / QTILE;
+      s.ptile0 = 0;
+      s.pad1 = 0;
+      *seg = s;
+    }
+  }
+  for (int64_t t = t0; t < n_items; t += nt) {
+    WorkItem w;
+    w.qrow0 = int32_t(t * rows);
+    w.nq = int32_t(min64(rows, n - t * rows));
+    w.key0 = 0;
+    w.nkeys = int32_t(n);
+    w.orig_off = 0;
+    w.qorig0 = int32_t(t * rows);
+    w.pad0 = w.pad1 = 0;
+    items[t] = w;
+  }
+  if (perm)
+    for (int64_t p = t0; p < npacked; p += nt)
+      perm[p] = p < n ? int32_t((p * stride) % n) : -1;
+  if (flags)
+    for (int64_t p = t0; p < npacked; p += nt) flags[p] = 0;
+}
+
+int launch_begin_single(int64_t n, int64_t npacked, int64_t n_items, int rows,
+                        int64_t stat_precision, int64_t stride, Ctl* ctl, KeyMax* km, KeyMax* km3,
+                        SegDesc* seg, WorkItem* items, int32_t* perm, int32_t* flags,
+                        cudaStream_t st) {
+  const int64_t most = perm || flags ? npacked : n_items;
+  const int blocks = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(most, 256),
+                                                               int64_t(num_sms()) * 8)));
+  begin_single_kernel<<<blocks, 256, 0, st>>>(n, npacked, n_items, rows, stat_precision, stride,
+                                              ctl, km, km3, seg, items, perm, flags);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }

@@ -83,7 +83,8 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
               int prec, int kmma, int k, int cosine, int32_t* __restrict__ knn_idx,
               float* __restrict__ knn_dist, int32_t* __restrict__ fail_rows,
               const int32_t* __restrict__ rows, const int32_t* __restrict__ nrows,
-              int32_t* __restrict__ fail_flags, int n_thr, int64_t thr_stride) {
+              int32_t* __restrict__ fail_flags, int n_thr, int64_t thr_stride,
+              int32_t* __restrict__ fail_list) {
   __shared__ __align__(16) float xs_all[RR_WARPS][MSC_MAX_D];
   __shared__ int wsc_all[RR_WARPS][32];                 // a row's window, compacted
   const int lane = lane_id(), wib = warp_id();
@@ -220,7 +221,9 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
       if (cert) {
         ++n_cert;
       } else if (fail_flags) {
-        fail_flags[p] = 1;                              // to the refine pass
+        fail_flags[p] = 1;                              // to the refine pass, in packed order
+      } else if (fail_list) {
+        fail_list[atomicAdd(&ctl->n_refine, 1)] = int32_t(p);   // to the refine pass
       } else {
         int slot = atomicAdd(&ctl->n_fail, 1);
         fail_rows[slot] = int32_t(p);                   // packed row, to the FP64 scan
@@ -341,7 +344,38 @@ __global__ void refine_items_kernel(const SegDesc* __restrict__ seg, int nseg,
   ctl->n_items_refine_eff = n * sp;
 }
 
+__global__ void refine_list_plan_kernel(int64_t n, WorkItem* __restrict__ items,
+                                        Ctl* __restrict__ ctl, int split, int max_split_items) {
+  const int64_t rows = ctl->n_refine;
+  const int m = int((rows + QTILE - 1) / QTILE);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
+    WorkItem w;
+    w.qrow0 = t * QTILE;
+    w.nq = int32_t(min64(QTILE, rows - int64_t(t) * QTILE));
+    w.key0 = 0;
+    w.nkeys = int32_t(n);
+    w.orig_off = 0;
+    w.qorig0 = 0;
+    w.pad0 = w.pad1 = 0;
+    items[t] = w;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int sp = (split > 1 && m <= max_split_items) ? split : 1;
+    ctl->stats[MSC_STAT_REFINED] = rows;
+    ctl->n_items_refine = m;
+    ctl->refine_split = sp;
+    ctl->n_items_refine_eff = m * sp;
+  }
+}
+
 }  // namespace
+
+int launch_refine_list_plan(int64_t n, WorkItem* items, Ctl* ctl, int split, int max_split_items,
+                            cudaStream_t st) {
+  refine_list_plan_kernel<<<1, 256, 0, st>>>(n, items, ctl, split, max_split_items);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
 
 int launch_all_rows_fail(const int32_t* perm, int64_t npacked, int32_t* fail_rows, Ctl* ctl,
                          cudaStream_t st) {
@@ -357,7 +391,8 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
                   const QStat* qs, const KeyMax* km, int prec, int kmma, int k, int cosine,
                   int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,
                   const int32_t* rows, const int32_t* nrows, int64_t max_rows,
-                  int32_t* fail_flags, cudaStream_t st, int n_thr, int64_t thr_stride) {
+                  int32_t* fail_flags, cudaStream_t st, int n_thr, int64_t thr_stride,
+                  int32_t* fail_list) {
   if (kprime > 64 || k - 1 > 64) {
     set_error("rerank: kprime=%d / k=%d beyond 64", kprime, k);
     return MSC_ERR_UNSUPPORTED;
@@ -367,7 +402,7 @@ int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg
   rerank_kernel<<<std::max(blocks, 1), RR_WARPS * 32, 0, st>>>(
       X, d, perm, seg, nseg, npacked, cand_idx, cand_thr, cand_stride, kprime, qs, km, ctl, prec,
       kmma, k, cosine, knn_idx, knn_dist, fail_rows, rows, nrows, fail_flags, n_thr,
-      thr_stride);
+      thr_stride, fail_list);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
