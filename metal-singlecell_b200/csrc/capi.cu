@@ -171,6 +171,7 @@ struct Problem {
   int kper = 0;
   int64_t stride = 1;     // the cells' order in packed space (launch_plain_order)
   int kref = 0;           // candidates per row of the refine pass
+  bool wide = false;      // !candidates: FP32 differences with FP64 around the k-th place (wide.cu)
 };
 
 struct KnnWs {
@@ -189,6 +190,7 @@ struct KnnWs {
   int32_t* cand_idx;
   float* cand_thr;
   int32_t* fail_rows;
+  WideWs wide;
   int32_t* perm;          // packed row -> original row (-1: padding)
   float* Xo;              // the rows projected for the locality order (d > ORDER_PROJ_D)
   void* order_ws;
@@ -324,6 +326,7 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
     }
   }
   P.kref = P.kprime;
+  P.wide = !P.candidates && wide_scan_ok(P.max_seg, d, k);
   if (!offsets && P.candidates && k > 1 && P.prec != PREC_FP32) {
     // MSC_B200_DENSE=<cells>: the full scan up to that many cells (tuning, tests; 0: never)
     const char* env = std::getenv("MSC_B200_DENSE");
@@ -387,6 +390,7 @@ KnnWs carve_knn(Carver& c, const Problem& P) {
   w.cand_thr = c.take<float>(size_t(P.n) * P.split);
   w.fail_rows = c.take<int32_t>(P.n);
   w.perm = c.take<int32_t>(P.npacked);
+  if (P.wide) w.wide = carve_wide(c, P.npacked, P.k);
   // the order's rows: projected when d > ORDER_PROJ_D
   if (!P.dense) {
     w.Xo = P.d > ORDER_PROJ_D ? c.take<float>(size_t(P.n) * ORDER_PROJ_D) : nullptr;
@@ -502,7 +506,13 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
                        w.order_ws_bytes, st, P.max_seg, proj ? w.Xo : nullptr, ORDER_PROJ_D,
                        proj_from));
   if (!P.candidates) {
-    MSC_TRY(launch_all_rows_fail(w.perm, P.npacked, w.fail_rows, w.ctl, st));
+    // wide lists: FP32 differences and FP64 around the k-th place (wide.cu), the FP64 scan for what
+    // it leaves open, or for every row where the list is too short a part of the cells to sample
+    if (P.wide)
+      MSC_TRY(launch_wide_scan(Xu, P.d, w.perm, w.seg, P.nseg, P.npacked, P.max_seg, P.k, cosine,
+                               w.wide, knn_idx, knn_dist, w.fail_rows, w.ctl, st));
+    else
+      MSC_TRY(launch_all_rows_fail(w.perm, P.npacked, w.fail_rows, w.ctl, st));
     MSC_TRY(launch_fp64_scan(Xu, P.d, w.perm, w.seg, P.nseg, w.fail_rows, P.n, P.k, cosine,
                              knn_idx, knn_dist, w.ctl, st));
     return MSC_OK;

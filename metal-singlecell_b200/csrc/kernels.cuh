@@ -311,6 +311,21 @@ int launch_fp64_scan(const float* X, int d, const int32_t* perm, const SegDesc* 
                      const int32_t* fail_rows, int64_t max_rows, int k, int cosine,
                      int32_t* knn_idx, float* knn_dist, Ctl* ctl, cudaStream_t st);
 
+// ---- wide.cu ----
+// exact kNN of every row for wide lists (k - 1 <= 512); the rows it leaves open go to fail_rows
+// (ctl->n_fail) for the FP64 scan
+bool wide_scan_ok(int64_t max_seg, int d, int k);
+struct WideWs {
+  float* thr;         // per packed row: collect keys with an FP32 value at or below
+  int32_t* cnt;       // keys collected
+  int2* buf;          // (value, key) of the rows in flight
+};
+WideWs carve_wide(Carver& c, int64_t npacked, int k);
+int launch_wide_scan(const float* X, int d, const int32_t* perm, const SegDesc* seg, int nseg,
+                     int64_t npacked, int64_t max_seg, int k, int cosine, const WideWs& ws,
+                     int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,
+                     cudaStream_t st);
+
 // ---- umap.cu ----
 int launch_smooth_knn(const float* dist, int64_t n, int k, float local_connectivity,
                       float* sigma, float* rho, double* gsum, cudaStream_t st);
