@@ -149,7 +149,7 @@ int launch_maxnorm(const float* X, const SegDesc* seg, int nseg, const double* m
 }
 
 // ------------------------------------------------------------------------------------------------
-// operand packing: one warp per packed row (grid-stride), lanes over dimensions
+// operand packing
 // ------------------------------------------------------------------------------------------------
 template <class T> __device__ __forceinline__ T to_op(double v);
 template <> __device__ __forceinline__ __half to_op<__half>(double v) { return __double2half(v); }
@@ -192,8 +192,13 @@ __global__ void pack_tc_kernel(const float* __restrict__ X, const int32_t* __res
                                KeyMax* __restrict__ km, const Ctl* __restrict__ ctl,
                                double pad_term, const int32_t* __restrict__ gate) {
   if (gate && *gate == 0) return;               // nothing to refine: no operands either
-  const int lane = lane_id();
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  // Eight lanes a row, four rows a warp: the four FP64 sums of a row take 3 shuffle steps of 8
+  // lanes for four rows at once (a warp a row took 40 shuffles, four cycles each, for every row, and
+  // bound the kernel), and a lane writes eight consecutive columns as one 16-byte store.  Two passes
+  // over the row, the second from L1: the norm terms are known only after the sums.
+  constexpr int PL = 8;
+  const int lane = lane_id(), sub = lane & (PL - 1);
+  const int64_t ngroups = (int64_t(gridDim.x) * blockDim.x) / PL;
   const double f = op_scale(prec, ctl);
   const T zero = to_op<T>(0.0);
   const T one = to_op<T>(1.0);
@@ -201,39 +206,38 @@ __global__ void pack_tc_kernel(const float* __restrict__ X, const int32_t* __res
   const int kd = SPLIT * d;                     // first column after the data terms
   const int64_t count = rows ? int64_t(*nrows) : npacked;
   float mx[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int64_t q = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; q < count;
-       q += nwarps) {
-    const int64_t p = rows ? int64_t(rows[q]) : q;
+  // the groups of a warp stay together (the shuffles take all lanes); q < count decides the writes
+  for (int64_t q0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / 32 * (32 / PL); q0 < count;
+       q0 += ngroups) {
+    const int64_t q = q0 + lane / PL;
+    const bool here = q < count;
+    const int64_t p = here ? (rows ? int64_t(rows[q]) : q) : 0;
     const int s = find_seg(seg, nseg, p);
-    const int64_t orow = perm[p];
+    const int64_t orow = here ? int64_t(perm[p]) : -1;
     const bool valid = orow >= 0;
     const double* c = mean + int64_t(s) * d;
-    T* arow = Aop ? Aop + q * kp : nullptr;
-    T* brow = Bop ? Bop + q * kp : nullptr;
+    const float* x = X + (valid ? orow : 0) * d;
     double sq = 0.0, nh = 0.0, nl = 0.0, nr = 0.0;
-    for (int t = lane; t < d; t += 32) {
-      double z = valid ? (double(X[orow * d + t]) - c[t]) * f : 0.0;
-      T hi = to_op<T>(z);
-      double hv = op_val(hi);
-      T lo = to_op<T>(SPLIT == 3 ? z - hv : 0.0);
-      double lv = SPLIT == 3 ? op_val(lo) : 0.0;
-      double r = z - hv - lv;
-      sq += z * z;
-      nh += hv * hv;
-      nl += lv * lv;
-      nr += r * r;
-      if (SPLIT == 3) {
-        if (arow) { arow[t] = hi; arow[d + t] = hi; arow[2 * d + t] = lo; }
-        if (brow) {
-          brow[t] = to_op<T>(-2.0 * hv); brow[d + t] = to_op<T>(-2.0 * lv);
-          brow[2 * d + t] = to_op<T>(-2.0 * hv);
-        }
-      } else {
-        if (arow) arow[t] = hi;
-        if (brow) brow[t] = to_op<T>(-2.0 * hv);
+    if (valid) {
+#pragma unroll 4
+      for (int t = sub; t < d; t += PL) {
+        const double z = (double(x[t]) - c[t]) * f;
+        const double hv = op_val(to_op<T>(z));
+        const double lv = SPLIT == 3 ? op_val(to_op<T>(z - hv)) : 0.0;
+        const double r = z - hv - lv;
+        sq += z * z;
+        nh += hv * hv;
+        if (SPLIT == 3) nl += lv * lv;
+        nr += r * r;
       }
     }
-    sq = warp_sum_d(sq); nh = warp_sum_d(nh); nl = warp_sum_d(nl); nr = warp_sum_d(nr);
+#pragma unroll
+    for (int o = PL / 2; o > 0; o >>= 1) {
+      sq += __shfl_xor_sync(FULL, sq, o);
+      nh += __shfl_xor_sync(FULL, nh, o);
+      if (SPLIT == 3) nl += __shfl_xor_sync(FULL, nl, o);
+      nr += __shfl_xor_sync(FULL, nr, o);
+    }
     const T t1 = to_op<T>(sq);
     const double s1 = op_val(t1);
     const T t2 = to_op<T>(sq - s1);
@@ -241,18 +245,45 @@ __global__ void pack_tc_kernel(const float* __restrict__ X, const int32_t* __res
     const T t3 = to_op<T>(sq - s1 - s2);
     const double s3 = op_val(t3);
     const double nerr = fabs(sq - s1 - s2 - s3);
-    for (int col = kd + lane; col < kp; col += 32) {
-      const int jj = col - kd;
-      if (arow) arow[col] = (jj < 3 && valid) ? one : zero;
-      if (brow) {
-        T v = zero;
-        if (jj == 0) v = valid ? t1 : padt;
-        if (jj == 1) v = valid ? t2 : padt;
-        if (jj == 2) v = valid ? t3 : padt;
-        brow[col] = v;
+    if (here) {
+      int seg3 = 0, t = sub * 8;                // column -> (term, dimension)
+      while (t >= d && seg3 < SPLIT) { t -= d; ++seg3; }
+      for (int col = sub * 8; col < kp; col += PL * 8) {
+        __align__(16) T av[8];
+        __align__(16) T bv[8];
+        int sg = seg3, tt = t;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          T a = zero, b = zero;
+          if (sg < SPLIT) {
+            const double z = valid ? (double(x[tt]) - c[tt]) * f : 0.0;
+            const T hi = to_op<T>(z);
+            if (SPLIT == 3) {
+              const double hv = op_val(hi);
+              const T lo = to_op<T>(z - hv);
+              a = sg == 2 ? lo : hi;
+              b = to_op<T>(-2.0 * (sg == 1 ? op_val(lo) : hv));
+            } else {
+              a = hi;
+              b = to_op<T>(-2.0 * op_val(hi));
+            }
+            if (++tt == d) { tt = 0; ++sg; }
+          } else {
+            const int jj = col + e - kd;
+            a = (jj < 3 && valid) ? one : zero;
+            b = jj == 0 ? (valid ? t1 : padt) : (jj == 1 ? (valid ? t2 : padt)
+                                                         : (jj == 2 ? (valid ? t3 : padt) : zero));
+          }
+          av[e] = a;
+          bv[e] = b;
+        }
+        if (Aop) *reinterpret_cast<uint4*>(Aop + q * kp + col) = *reinterpret_cast<uint4*>(av);
+        if (Bop) *reinterpret_cast<uint4*>(Bop + q * kp + col) = *reinterpret_cast<uint4*>(bv);
+        t += PL * 8;
+        while (t >= d && seg3 < SPLIT) { t -= d; ++seg3; }
       }
     }
-    if (lane == 0 && qs) {
+    if (here && sub == 0 && qs) {
       QStat qq;
       qq.sq = sq;
       qq.hi = __double2float_ru(sqrt(nh));
@@ -278,7 +309,7 @@ int launch_pack_tc(int prec, const float* X, const int32_t* perm, const SegDesc*
                    KeyMax* km, const Ctl* ctl, cudaStream_t st, const int32_t* gate) {
   const OpLayout L = op_layout(prec, d);
   const int64_t n_out = rows ? max_rows : npacked;
-  int blocks = int(std::min<int64_t>(ceil_div(n_out, 8), int64_t(num_sms()) * 16));
+  int blocks = int(std::min<int64_t>(ceil_div(n_out, 32), int64_t(num_sms()) * 16));
   blocks = std::max(blocks, 1);
   switch (prec) {
     case PREC_BF16X3:
