@@ -180,62 +180,112 @@ __global__ void partition_kernel(const int32_t* __restrict__ perm, const int32_t
   }
 }
 
+// Centres that lanes read for consecutive balls (key tiles, sub-balls) lie interleaved: balls in
+// groups of 32, float4 t of ball g at [g / 32][t][g % 32], so that a warp's 32 reads of one float4 are
+// 512 consecutive bytes.  (Row after row, 208 bytes apart at 50 dimensions, each read touched 32
+// lines: the plan at 1.3M cells took 7.03 ms, 6.63 interleaved.)
+__device__ __forceinline__ int64_t inter_at(int64_t g, int n4) {
+  return (g >> 5) * (32 * n4) + (g & 31);
+}
+constexpr int INTER = 32;        // float4s from one to the next of an interleaved ball
+__device__ __forceinline__ void store_centre(float* centre, int64_t g, int dp, int t, float v,
+                                             bool interleaved) {
+  if (interleaved)
+    centre[(inter_at(g, dp / 4) + int64_t(t >> 2) * INTER) * 4 + (t & 3)] = v;
+  else
+    centre[g * dp + t] = v;
+}
+
+// Squared distance of a row to a centre (shared memory, float) by 8 lanes, FP64: every lane of the
+// group returns it.  Four rows of a warp go at once, so a row's sum takes 3 shuffle steps for four
+// rows where a warp a row takes 5 for one.
+__device__ __forceinline__ double row_d2_8(const float* __restrict__ x, const float* c, int d,
+                                           int sub) {
+  double a = 0.0;
+  for (int t = sub; t < d; t += 8) {
+    const double u = double(x[t]) - double(c[t]);
+    a += u * u;
+  }
+  a += __shfl_xor_sync(FULL, a, 4);
+  a += __shfl_xor_sync(FULL, a, 2);
+  a += __shfl_xor_sync(FULL, a, 1);
+  return a;
+}
+
 // One ball per group of G packed rows (G = 128 or 256): centre = float(mean of the rows), radius =
-// max distance to that centre, rounded up.  One warp per group; lane t sums dimensions t, t+32, ...
-template <int G>
-__global__ void group_ball_kernel(const float* __restrict__ X, int d, int dp,
-                                  const int32_t* __restrict__ perm, int64_t ngroups,
-                                  float* __restrict__ centre, float* __restrict__ radius) {
-  const int lane = lane_id();
-  const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t g = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; g < ngroups;
-       g += warps) {
+// max distance to that centre, rounded up.  A block of eight warps per group, G / 8 rows each (one
+// warp per group read 256 rows one after another, 157 us at any n up to 100,000).
+template <int G, bool INTERLEAVED>
+__global__ void __launch_bounds__(PR_T)
+group_ball_kernel(const float* __restrict__ X, int d, int dp, const int32_t* __restrict__ perm,
+                  int64_t ngroups, float* __restrict__ centre, float* __restrict__ radius) {
+  constexpr int W = PR_T / 32, R = G / W;
+  __shared__ double part[W][MSC_MAX_D];
+  __shared__ float c[MSC_MAX_D];
+  __shared__ double mxs[W];
+  __shared__ int cnts[W];
+  const int lane = lane_id(), wib = warp_id();
+  for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t p0 = g * G + wib * R;
+    const int32_t my_i = lane < R ? perm[p0 + lane] : -1;
     double s[4] = {0, 0, 0, 0};
-    int cnt = 0;
-    for (int r = 0; r < G; ++r) {
-      const int32_t i = perm[g * G + r];
+#pragma unroll 4
+    for (int r = 0; r < R; ++r) {
+      const int32_t i = __shfl_sync(FULL, my_i, r);
       if (i < 0) continue;
-      ++cnt;
+#pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int t = lane + 32 * j;
         if (t < d) s[j] += X[int64_t(i) * d + t];
       }
     }
-    float c[4];
-    for (int j = 0; j < 4; ++j) {
-      const int t = lane + 32 * j;
-      c[j] = (cnt && t < d) ? float(s[j] / cnt) : 0.f;
-      if (t < dp) centre[g * dp + t] = c[j];
-    }
-    double mx = 0.0;
-    for (int r = 0; r < G; ++r) {
-      const int32_t i = perm[g * G + r];
-      if (i < 0) continue;
+    __syncthreads();                           // the previous group's values are read
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (lane + 32 * j < d) part[wib][lane + 32 * j] = s[j];
+    const unsigned have = __ballot_sync(FULL, my_i >= 0);
+    if (lane == 0) cnts[wib] = __popc(have);
+    __syncthreads();
+    int cnt = 0;
+    for (int w = 0; w < W; ++w) cnt += cnts[w];
+    for (int t = threadIdx.x; t < dp; t += PR_T) {
       double a = 0.0;
-      for (int j = 0; j < 4; ++j) {
-        const int t = lane + 32 * j;
-        if (t < d) {
-          const double u = double(X[int64_t(i) * d + t]) - double(c[j]);
-          a += u * u;
-        }
-      }
-      mx = fmax(mx, warp_sum_d(a));
+      if (t < d)
+        for (int w = 0; w < W; ++w) a += part[w][t];
+      const float v = (cnt && t < d) ? float(a / cnt) : 0.f;
+      c[t] = v;
+      store_centre(centre, g, dp, t, v, INTERLEAVED);
     }
-    if (lane == 0)
+    __syncthreads();
+    double mx = 0.0;
+    for (int r = 0; r < R; r += 4) {
+      const int32_t i = __shfl_sync(FULL, my_i, r + (lane >> 3));
+      const double a = row_d2_8(X + int64_t(i < 0 ? 0 : i) * d, c, d, lane & 7);
+      if (i >= 0) mx = fmax(mx, a);
+    }
+    mx = warp_max_d(mx);
+    if (lane == 0) mxs[wib] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < W; ++w) mx = fmax(mx, mxs[w]);
       radius[g] = cnt ? __double2float_ru(sqrt(mx) * (1.0 + 0x1p-40)) : NO_BALL;
+    }
   }
 }
 
 // Two balls per 32-row block, split at the first row whose leaf differs from the block's first
 // row (rows of one leaf are close, rows of two leaves may lie in two clusters), and the block's
 // max R.  Ball 2b covers rows [0, m), ball 2b+1 rows [m, 32).
-__global__ void sub_ball_kernel(const float* __restrict__ X, int d, int dp,
+__global__ void __launch_bounds__(PR_T)
+sub_ball_kernel(const float* __restrict__ X, int d, int dp,
                                 const int32_t* __restrict__ perm,
                                 const int32_t* __restrict__ leaf,
                                 const double* __restrict__ rpos, int64_t nsub,
                                 float* __restrict__ centre, float* __restrict__ radius,
                                 double* __restrict__ rsub) {
+  __shared__ float c_all[PR_T / 32][MSC_MAX_D];
   const int lane = lane_id();
+  float* c = c_all[warp_id()];
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t b = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; b < nsub; b += warps) {
     const int64_t p0 = b * SUB;
@@ -256,67 +306,77 @@ __global__ void sub_ball_kernel(const float* __restrict__ X, int d, int dp,
       const int r0 = h ? m : 0, r1 = h ? SUB : m;
       double s[4] = {0, 0, 0, 0};
       int cnt = 0;
+#pragma unroll 4
       for (int r = r0; r < r1; ++r) {
         const int32_t i = __shfl_sync(FULL, my_i, r);
         if (i < 0) continue;
         ++cnt;
+#pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int t = lane + 32 * j;
           if (t < d) s[j] += X[int64_t(i) * d + t];
         }
       }
-      float c[4];
-      float* cdst = centre + (2 * b + h) * dp;
+      __syncwarp();                              // the previous ball's centre is read
+#pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int t = lane + 32 * j;
-        c[j] = (cnt && t < d) ? float(s[j] / cnt) : 0.f;
-        if (t < dp) cdst[t] = c[j];
-      }
-      double mx = 0.0;
-      for (int r = r0; r < r1; ++r) {
-        const int32_t i = __shfl_sync(FULL, my_i, r);
-        if (i < 0) continue;
-        double a = 0.0;
-        for (int j = 0; j < 4; ++j) {
-          const int t = lane + 32 * j;
-          if (t < d) {
-            const double u = double(X[int64_t(i) * d + t]) - double(c[j]);
-            a += u * u;
-          }
+        const float v = (cnt && t < d) ? float(s[j] / cnt) : 0.f;
+        if (t < dp) {
+          c[t] = v;
+          store_centre(centre, 2 * b + h, dp, t, v, true);
         }
-        mx = fmax(mx, warp_sum_d(a));
       }
+      __syncwarp();
+      double mx = 0.0;
+      for (int r = r0; r < r1; r += 4) {
+        const int rr = r + (lane >> 3);
+        const int32_t i = __shfl_sync(FULL, my_i, rr & 31);
+        const bool in = rr < r1 && i >= 0;
+        const double a = row_d2_8(X + int64_t(in ? i : 0) * d, c, d, lane & 7);
+        if (in) mx = fmax(mx, a);
+      }
+      mx = warp_max_d(mx);
       if (lane == 0)
         radius[2 * b + h] = cnt ? __double2float_ru(sqrt(mx) * (1.0 + 0x1p-40)) : NO_BALL;
     }
   }
 }
 
-// Are the balls (cu, ru) and (cw, rw) so far apart that no row of u can take a key of w?  R = max
-// R over u's rows (z-space), f2 = square of the operand scale.  An empty ball is separated from
-// everything; an unknown R (inf / NaN) from nothing.  Centres are n4 float4 (zero padded); the
-// FP32 distance is lowered by its rounding bound (d+8 units of 2^-23 relative) before the test.
-__device__ __forceinline__ bool separated(const float* __restrict__ cu, float ru, double R,
-                                          const float* __restrict__ cw, float rw, int n4, int d,
-                                          double f2) {
-  if (ru < 0.f || rw < 0.f) return true;
-  if (!(R < 1e300)) return false;
-  const float4* a = reinterpret_cast<const float4*>(cu);
-  const float4* b = reinterpret_cast<const float4*>(cw);
+// Are the balls (cu, ru) and (cw, rw) so far apart that no row of u can take a key of w?  That is
+// L = |cu - cw| - ru - rw > 0 and f²·L² > R·(1 + 1e-9) (R = max R over u's rows, z-space, f = the
+// operand scale), which is |cu - cw| > ru + rw + reach with reach = sqrt(R·(1 + 1e-9)) / f: the root is
+// taken once per ball u (ball_reach) and a test compares squares (its 1e-12 covers the FP64
+// roundings).  An empty ball is separated from everything; an unknown R (reach +inf) from nothing.
+// Centres are n4 float4 (zero padded), SA and SB float4s apart; the FP32 distance is lowered by its
+// rounding bound (d+8 units of 2^-23 relative) before the test.
+__device__ __forceinline__ double ball_reach(double R, double f) {
+  return R < 1e300 ? sqrt(R * (1.0 + 1e-9)) / f : __longlong_as_double(0x7ff0000000000000ll);
+}
+template <int SA, int SB>
+__device__ __forceinline__ float ball_d2(const float4* a, const float4* b, int n4) {
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll 4
   for (int t = 0; t < n4; ++t) {
-    const float4 x = a[t], y = b[t];
+    const float4 x = a[t * SA], y = b[t * SB];
     const float e0 = x.x - y.x, e1 = x.y - y.y, e2 = x.z - y.z, e3 = x.w - y.w;
     s0 = fmaf(e0, e0, s0);
     s1 = fmaf(e1, e1, s1);
     s2 = fmaf(e2, e2, s2);
     s3 = fmaf(e3, e3, s3);
   }
-  const float s = (s0 + s1) + (s2 + s3);
-  const double lo = double(s) * (1.0 - double(d + 8) * 0x1p-23);
-  const double L = sqrt(lo) - double(ru) - double(rw);
-  return L > 0.0 && f2 * L * L > R * (1.0 + 1e-9);
+  return (s0 + s1) + (s2 + s3);
+}
+__device__ __forceinline__ bool apart(float d2, float ru, float rw, double reach, int d) {
+  if (ru < 0.f || rw < 0.f) return true;
+  const double lo = double(d2) * (1.0 - double(d + 8) * 0x1p-23);
+  const double far = (double(ru) + double(rw) + reach) * (1.0 + 1e-12);
+  return lo > far * far;
+}
+template <int SA, int SB>
+__device__ __forceinline__ bool separated(const float4* a, float ru, double reach, const float4* b,
+                                          float rw, int n4, int d) {
+  return apart(ball_d2<SA, SB>(a, b, n4), ru, rw, reach, d);
 }
 
 // One warp per query tile (work item).  Level 1, lane = key tile: the query tile's ball against
@@ -326,7 +386,12 @@ __device__ __forceinline__ bool separated(const float* __restrict__ cu, float ru
 // the other side — with the (key tile, sub-ball) tests spread over the lanes; then, per key tile
 // left, the remaining sub-ball pairs, one pair per lane.
 constexpr int PLAN_WARPS = 4;
-constexpr int PLAN_WORDS = 8;     // mask words (256 key tiles) per warp task
+// mask words (32 key tiles each) per warp task: at most 4, fewer while the tasks do not give every
+// resident warp PLAN_TASKS of them.  The work of a task varies from one test a tile to some fifty, and
+// at 100,000 cells the launch waited for the few warps with the most (0.73 ms with 8 words, 0.85 ms
+// with the n-th set bits found by __fns, 0.12 ms now; 1.3M cells 6.63 -> 5.90 without __fns, 5.27
+// with squared tests and 4-word tasks, 4.36 with the visits of level 1).
+constexpr int PLAN_WORDS_MAX = 4, PLAN_TASKS = 16;
 constexpr int PLAN_MAX_PAIRS = 32;  // sub-ball pairs tested per key tile (one per lane);
                                     // MSC_B200_PLAN_PAIRS overrides (tuning)
 __global__ void __launch_bounds__(PLAN_WARPS * 32, 6)
@@ -335,22 +400,33 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
             const float* __restrict__ kc, const float* __restrict__ kr,
             const float* __restrict__ sc, const float* __restrict__ sr,
             const double* __restrict__ rsub, int words, uint32_t* __restrict__ mask, int prof,
-            int max_pairs) {
+            int max_pairs, int task_words) {
   extern __shared__ float4 sm4[];
   __shared__ unsigned ubits_all[PLAN_WARPS][32], wbits_all[PLAN_WARPS][32];
+  // positions of set bits, written by the lanes that hold them: the failing tiles of a chunk, the
+  // ones (a) left open, and the open sub-balls of a pair of tiles (finding the n-th set bit of a
+  // mask with __fns, a software loop, for every test took most of this kernel's time)
+  __shared__ uint8_t fail_all[PLAN_WARPS][32], open_all[PLAN_WARPS][32];
+  __shared__ uint8_t ulist_all[PLAN_WARPS][8], wlist_all[PLAN_WARPS][32];
+  __shared__ double reach_all[PLAN_WARPS][4];
   const int lane = lane_id(), wib = warp_id();
-  float* qball = reinterpret_cast<float*>(sm4) + wib * (9 * dp);   // [0]: tile, [1..8]: sub-balls
+  const int n4 = dp / 4;
+  float4* qball = sm4 + wib * (9 * n4);          // [0]: tile, [1..8]: sub-balls
   unsigned* ubits = ubits_all[wib];
   unsigned* wbits = wbits_all[wib];
-  const int n4 = dp / 4;
+  uint8_t *fails = fail_all[wib], *opens = open_all[wib];
+  uint8_t *ulist = ulist_all[wib], *wlist = wlist_all[wib];
+  double* reach = reach_all[wib];
+  const unsigned below = (1u << lane) - 1u;
+  const float4* kc4 = reinterpret_cast<const float4*>(kc);     // interleaved
+  const float4* sc4 = reinterpret_cast<const float4*>(sc);     // interleaved
   const double f = op_scale(prec, ctl);
-  const double f2 = f * f;
   const int64_t warps = int64_t(gridDim.x) * PLAN_WARPS;
   const int nv = 2 * max(1, bn / SUB);          // key sub-balls per key tile
   long long nvis = 0, ntot = 0, nl1 = 0, npt = 0, npr = 0;
-  // tasks = (query tile, block of PLAN_WORDS mask words): the level-2 work of a query tile varies
+  // tasks = (query tile, block of task_words mask words): the level-2 work of a query tile varies
   // widely, so whole tiles per warp would leave most SMs idle behind the slowest few
-  const int nblk = (words + PLAN_WORDS - 1) / PLAN_WORDS;
+  const int nblk = (words + task_words - 1) / task_words;
   const int64_t ntasks = n_items * nblk;
   // consecutive warps take consecutive query tiles of the same key-tile block, so the key-side
   // centres they read are shared through L1
@@ -361,40 +437,53 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
     const int64_t qt = w.qrow0 / QTILE;          // 128-row tile of packed rows
     const int64_t sb0 = int64_t(w.qrow0) / SUB;  // its first 32-row block
     __syncwarp();
-    for (int t = lane; t < dp; t += 32) qball[t] = qc[qt * dp + t];
-    for (int u = 0; u < 8; ++u)
-      for (int t = lane; t < dp; t += 32) qball[(1 + u) * dp + t] = sc[(2 * sb0 + u) * dp + t];
+    for (int t = lane; t < n4; t += 32)
+      qball[t] = reinterpret_cast<const float4*>(qc)[qt * n4 + t];
+    for (int x = lane; x < 8 * n4; x += 32) {       // 8 consecutive balls: 128-byte runs
+      const int t = x >> 3, u = x & 7;
+      qball[(1 + u) * n4 + t] = sc4[inter_at(2 * sb0 + u, n4) + int64_t(t) * INTER];
+    }
     __syncwarp();
     const float rq = qr[qt];
-    double Rq = 0.0;
-    for (int j = 0; j < 4; ++j) Rq = fmax(Rq, rsub[sb0 + j]);    // rsub is >= 0 or +inf
+    // the reach of each 32-row block and of the whole tile
+    if (lane < 4) reach[lane] = ball_reach(rsub[sb0 + lane], f);  // rsub is >= 0 or +inf
+    __syncwarp();
+    const double reach_q = fmax(fmax(reach[0], reach[1]), fmax(reach[2], reach[3]));
     const int nkt = (w.nkeys + bn - 1) / bn;
     const int diag = (w.qrow0 - w.key0) / bn;
     const int lo = max(0, diag - 2), hi = min(nkt - 1, diag + 2);
     uint32_t* out = mask + it * int64_t(words);
-    const int wend = min(words, (wblk + 1) * PLAN_WORDS);
-    for (int base = wblk * PLAN_WORDS * 32; base < wend * 32; base += 32) {
+    const int wend = min(words, (wblk + 1) * task_words);
+    for (int base = wblk * task_words * 32; base < wend * 32; base += 32) {
       const int kt = base + lane;
       bool l1 = false;                           // not separated at level 1
+      bool deep = false;                         // ... and visited without level 2
       if (kt < nkt && (kt < lo || kt > hi)) {
         const int64_t g = (int64_t(w.key0) + int64_t(kt) * bn) / 256;
-        l1 = !separated(qball, rq, Rq, kc + g * dp, kr[g], n4, d, f2);
+        const float d2 = ball_d2<1, INTER>(qball, kc4 + inter_at(g, n4), n4);
+        l1 = !apart(d2, rq, kr[g], reach_q, d);
+        // a key tile whose centre lies within the rows' reach of the query tile's shares its
+        // cluster: level 2 would find open sub-balls (a visit it could have saved costs time only;
+        // at 1.3M x 50 the visits are the same 2.88 M, and level 2 tests half the pairs)
+        deep = l1 && double(d2) <= reach_q * reach_q;
+        l1 = l1 && !deep;
       }
       const uint32_t fm = __ballot_sync(FULL, l1);
-      uint32_t bits = 0u;
+      uint32_t bits = __ballot_sync(FULL, deep);
       if (fm) {
         const int nf = __popc(fm);
         nl1 += nf;
         ubits[lane] = 0u;
         wbits[lane] = 0u;
+        if (l1) fails[__popc(fm & below)] = uint8_t(lane);
         __syncwarp();
         // (a) query sub-ball u of failing tile i
         for (int x = lane; x < 8 * nf; x += 32) {
           const int i = x >> 3, u = x & 7;
-          const int kti = base + __fns(fm, 0, i + 1);
+          const int kti = base + fails[i];
           const int64_t g = (int64_t(w.key0) + int64_t(kti) * bn) / 256;
-          if (!separated(qball + (1 + u) * dp, sr[2 * sb0 + u], rsub[sb0 + (u >> 1)],
-                         kc + g * dp, kr[g], n4, d, f2))
+          if (!separated<1, INTER>(qball + (1 + u) * n4, sr[2 * sb0 + u], reach[u >> 1],
+                                   kc4 + inter_at(g, n4), kr[g], n4, d))
             atomicOr(&ubits[i], 1u << u);
         }
         __syncwarp();
@@ -402,20 +491,23 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
         // open query sub-ball is skipped whatever (b) finds)
         const uint32_t fo = __ballot_sync(FULL, lane < nf && ubits[lane] != 0u);
         const int no = __popc(fo);
+        if ((fo >> lane) & 1u) opens[__popc(fo & below)] = uint8_t(lane);
+        __syncwarp();
         for (int x = lane; x < nv * no; x += 32) {
           const int io = x / nv, v = x - io * nv;
-          const int i = __fns(fo, 0, io + 1);
-          const int kti = base + __fns(fm, 0, i + 1);
+          const int i = opens[io];
+          const int kti = base + fails[i];
           const int64_t kb0 = (int64_t(w.key0) + int64_t(kti) * bn) / SUB;
           const float rw = sr[2 * kb0 + v];
-          if (rw >= 0.f && !separated(qball, rq, Rq, sc + (2 * kb0 + v) * dp, rw, n4, d, f2))
+          if (rw >= 0.f && !separated<1, INTER>(qball, rq, reach_q,
+                                                sc4 + inter_at(2 * kb0 + v, n4), rw, n4, d))
             atomicOr(&wbits[i], 1u << v);
         }
         __syncwarp();
         for (int i = 0; i < nf; ++i) {
           const uint32_t ub = ubits[i], wb = wbits[i];
           if (!ub || !wb) continue;                 // warp-uniform
-          const int kti = base + __fns(fm, 0, i + 1);
+          const int kti = base + fails[i];
           const int64_t kb0 = (int64_t(w.key0) + int64_t(kti) * bn) / SUB;
           const int nu = __popc(ub), npair = nu * __popc(wb);
           // many overlapping sub-ball pairs: the tiles share a cluster, and testing every pair
@@ -426,11 +518,15 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
           }
           ++npt;
           npr += npair;
+          __syncwarp();                             // the previous tile's lists are read
+          if (lane < 8 && ((ub >> lane) & 1u)) ulist[__popc(ub & below)] = uint8_t(lane);
+          if ((wb >> lane) & 1u) wlist[__popc(wb & below)] = uint8_t(lane);
+          __syncwarp();
           bool hit = false;
           for (int pr = lane; pr < npair && !hit; pr += 32) {
-            const int u = __fns(ub, 0, pr % nu + 1), vv = __fns(wb, 0, pr / nu + 1);
-            hit = !separated(qball + (1 + u) * dp, sr[2 * sb0 + u], rsub[sb0 + (u >> 1)],
-                             sc + (2 * kb0 + vv) * dp, sr[2 * kb0 + vv], n4, d, f2);
+            const int u = ulist[pr % nu], vv = wlist[pr / nu];
+            hit = !separated<1, INTER>(qball + (1 + u) * n4, sr[2 * sb0 + u], reach[u >> 1],
+                                       sc4 + inter_at(2 * kb0 + vv, n4), sr[2 * kb0 + vv], n4, d);
           }
           if (__any_sync(FULL, hit)) bits |= 1u << (kti - base);
         }
@@ -806,10 +902,10 @@ visit_order_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, 
         float dist = 0.f, need = F_INF;
         if (rq >= 0.f && rk >= 0.f) {
           const float4* a4 = reinterpret_cast<const float4*>(qcen);
-          const float4* b4 = reinterpret_cast<const float4*>(kc + g * dp);
+          const float4* b4 = reinterpret_cast<const float4*>(kc) + inter_at(g, n4);
           float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
           for (int t = 0; t < n4; ++t) {
-            const float4 x = a4[t], y = b4[t];
+            const float4 x = a4[t], y = b4[t * INTER];
             const float e0 = x.x - y.x, e1 = x.y - y.y, e2 = x.z - y.z, e3 = x.w - y.w;
             s0 = fmaf(e0, e0, s0);
             s1 = fmaf(e1, e1, s1);
@@ -890,9 +986,9 @@ PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items
   const int dp = int(round_up(d, 4));
   w.qc = c.take<float>(size_t(nq) * dp);
   w.qr = c.take<float>(nq);
-  w.kc = c.take<float>(size_t(nk) * dp);
+  w.kc = c.take<float>(size_t(round_up(nk, 32)) * dp);          // interleaved in groups of 32
   w.kr = c.take<float>(nk);
-  w.sc = c.take<float>(size_t(2 * ns) * dp);
+  w.sc = c.take<float>(size_t(round_up(2 * ns, 32)) * dp);      // interleaved in groups of 32
   w.sr = c.take<float>(2 * ns);
   w.rsub = c.take<double>(ns);
   w.mask = c.take<uint32_t>(size_t(n_items) * words);
@@ -973,10 +1069,12 @@ int launch_prune_plan(const float* X, int d, int64_t npacked, const int32_t* per
   }
   const int64_t nq = npacked / QTILE, nk = npacked / 256, ns = npacked / SUB;
   const int dp = int(round_up(d, 4));
-  const int wgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(nq, 8), num_sms() * 16)));
-  group_ball_kernel<QTILE><<<wgrid, PR_T, 0, st>>>(X, d, dp, perm, nq, w.qc, w.qr);
+  const int64_t most = int64_t(num_sms()) * 32;
+  group_ball_kernel<QTILE, false><<<int(std::min(nq, most)), PR_T, 0, st>>>(X, d, dp, perm, nq,
+                                                                           w.qc, w.qr);
   MSC_LAUNCH_CHECK();
-  group_ball_kernel<256><<<wgrid, PR_T, 0, st>>>(X, d, dp, perm, nk, w.kc, w.kr);
+  group_ball_kernel<256, true><<<int(std::min(nk, most)), PR_T, 0, st>>>(X, d, dp, perm, nk, w.kc,
+                                                                         w.kr);
   MSC_LAUNCH_CHECK();
   const int sgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ns, 8), num_sms() * 16)));
   sub_ball_kernel<<<sgrid, PR_T, 0, st>>>(X, d, dp, perm, w.leaf2, w.rpos2, ns, w.sc, w.sr, w.rsub);
@@ -984,13 +1082,16 @@ int launch_prune_plan(const float* X, int d, int64_t npacked, const int32_t* per
   const size_t smem = size_t(PLAN_WARPS) * 9 * dp * sizeof(float);
   int max_pairs = PLAN_MAX_PAIRS;
   if (const char* env = std::getenv("MSC_B200_PLAN_PAIRS")) max_pairs = std::max(0, std::atoi(env));
-  const int64_t ntasks = n_items * ceil_div(words, PLAN_WORDS);
+  const int64_t want = int64_t(num_sms()) * 6 * PLAN_WARPS * PLAN_TASKS;
+  int task_words = PLAN_WORDS_MAX;
+  while (task_words > 1 && n_items * ceil_div(words, task_words) < want) task_words >>= 1;
+  const int64_t ntasks = n_items * ceil_div(words, task_words);
   const int pgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ntasks, PLAN_WARPS),
                                                               int64_t(num_sms()) * 32)));
   plan_kernel<<<pgrid, PLAN_WARPS * 32, smem, st>>>(items, n_items, bn, d, dp, ctl, prec, w.qc,
                                                     w.qr, w.kc, w.kr, w.sc, w.sr, w.rsub, words,
                                                     w.mask, profiling_enabled() ? 1 : 0,
-                                                    max_pairs);
+                                                    max_pairs, task_words);
   MSC_LAUNCH_CHECK();
   // point test of the kept pairs, opt-in (MSC_B200_POINT_TEST=1).  Measured at 1.3M × 50: far
   // tiles kept 2.63 M → 1.63 M and main scan 33.4 → 28.0 ms, but the test itself costs ~15 ms
