@@ -267,7 +267,7 @@ int msc_trim_graph(const int64_t* indptr_dev, const int32_t* indices_dev, const 
 #define MSC_SP_STAT_NONFINITE    0   /* non-finite coordinates (nothing is computed)             */
 #define MSC_SP_STAT_STATUS       1   /* 0 ok, 1 non-finite input, 2 no cell plan                */
 #define MSC_SP_STAT_CELLS        2   /* cells of the grid                                        */
-#define MSC_SP_STAT_CHUNKS       3   /* query chunks (<= 32 points of one cell)                  */
+#define MSC_SP_STAT_CHUNKS       3   /* groups of 32 queries, in cell order                      */
 #define MSC_SP_STAT_EVALS        4   /* candidate distances evaluated                            */
 #define MSC_SP_STAT_EXPANDED     5   /* kNN rows that needed more than one ring of cells         */
 #define MSC_SP_STAT_RING         6   /* radius search: rings of cells around the query's cell    */

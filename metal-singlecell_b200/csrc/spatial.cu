@@ -11,17 +11,19 @@
 // Build, all on the device:
 //   sp_bbox   per-axis minimum / maximum (order-preserving integer atomics), non-finite count
 //   sp_plan   one thread: cell side, cells per axis (at most 4n + 16 cells), FP64 geometry
-//   sp_bin    cell of every point (FP64 floor of (x − o) / cs), cell counts, chunk counts
-//   scans     cell starts, chunk starts
+//   sp_bin    cell of every point (FP64 floor of (x − o) / cs), cell counts
+//   scan      cell starts
 //   sp_place  points in cell order as float4 (x, y, z, index bits)
-//   sp_chunks chunk → (cell, first sorted position); a chunk is ≤ 32 points of one cell
-// Search: one warp per chunk (persistent grid), one lane per query, candidates of a run of
-// cells staged through shared memory and read by every lane (broadcast reads).
-//   kNN: shells R = 0, 1, 2, ... of cells around the chunk's cell; each lane keeps its k − 1
+// Search: one lane per query, the queries in cell order, each lane walking its own cells.  Lanes of
+// one cell read the same points at the same time and lanes of neighbouring cells nearly the same
+// lines.  (A warp per cell with the candidates staged for all its lanes left most lanes without a
+// query where cells hold few points, and so wanted large cells, whose candidates are mostly too
+// far.  1M spots, k = 7, whole search: 1.86 ms, now 0.55.)
+//   kNN: the 3^d cells around the query's cell, then larger boxes; a lane keeps its k − 1
 //        best (distance, index) keys sorted in registers; it is done once its (k−1)-th distance
 //        is provably below the distance to every cell outside the scanned box (FP64 bound with a
 //        margin that covers float32 rounding), so every row is exact without a fallback pass.
-//   radius: every cell within ring = ceil(D / cs) of the chunk's cell, D = radius plus a margin
+//   radius: every cell within ring = ceil(D / cs) of the query's cell, D = radius plus a margin
 //        that covers rounding; a count pass, a scan, a fill pass in the same walk order, then
 //        each row's columns put in ascending order (rank sort).
 #include <climits>
@@ -34,7 +36,8 @@ namespace {
 
 constexpr int SP_T = 128;                 // threads per block of the search kernels
 constexpr int SP_W = SP_T / 32;
-constexpr int SP_STAGE = 64;              // candidates staged per warp per round
+constexpr int LANE_R = 4;                 // kNN: largest box of cells one lane walks
+constexpr double CELL_PER_K = 0.33;       // kNN in the plane: points per cell / k
 constexpr int SORT_TILE = 256;            // columns staged per warp by the row sort
 constexpr int SORT_E = 4;                 // entries ranked per lane per group
 
@@ -81,13 +84,26 @@ __global__ void sp_bbox_kernel(const float* __restrict__ X, int64_t n, int d,
     }
   }
   for (int off = 16; off > 0; off >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, off);
+  // one set of atomics per block (one per warp took 53 us at 1M points)
+  __shared__ float slo[3][32], shi[3][32];
+  __shared__ unsigned long long sbad[32];
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if ((threadIdx.x & 31) == 0) {
-    for (int a = 0; a < d; ++a) {
-      if (lo[a] <= hi[a]) {
-        atomicMin(&mm[a], f2o(lo[a]));
-        atomicMax(&mm[3 + a], f2o(hi[a]));
-      }
+    for (int a = 0; a < 3; ++a) { slo[a][w] = lo[a]; shi[a][w] = hi[a]; }
+    sbad[w] = bad;
+  }
+  __syncthreads();
+  if (threadIdx.x < d) {
+    const int a = threadIdx.x;
+    float l = slo[a][0], h = shi[a][0];
+    for (int i = 1; i < nw; ++i) { l = fminf(l, slo[a][i]); h = fmaxf(h, shi[a][i]); }
+    if (l <= h) {
+      atomicMin(&mm[a], f2o(l));
+      atomicMax(&mm[3 + a], f2o(h));
     }
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < nw; ++i) bad += sbad[i];
     if (bad) atomicAdd(nonfinite, bad);
   }
 }
@@ -121,7 +137,12 @@ __global__ void sp_plan_kernel(const unsigned* __restrict__ mm,
     } else {
       double vol = 1.0;
       for (int a = 0; a < 3; ++a) if (ext[a] > 0) vol *= ext[a];
-      const double target = double(k > 4 ? 2 * k : 8);
+      // points per cell on average: of the 3^d cells scanned first a circle (ball) of one cell
+      // side around the query is certain to be covered, so about k/3 points a cell in the plane and
+      // k/4 in space end most walks there where the points are as dense as on average; in denser
+      // regions, where most points are, cells hold more.  (1M spots of uneven density, k = 7: whole
+      // search 0.67 ms at 0.33 k points a cell, 0.79 at 0.5 k.)
+      const double target = fmax(1.0, eff == 3 ? 0.25 * k : CELL_PER_K * k);
       cs = pow(target * vol / double(n), 1.0 / eff);
     }
   } else {
@@ -181,14 +202,6 @@ __global__ void sp_bin_kernel(const float* __restrict__ X, int64_t n, int d,
   }
 }
 
-__global__ void sp_chunk_count_kernel(const int32_t* __restrict__ count, const SpGrid* __restrict__ G,
-                                      int32_t* __restrict__ nchunk) {
-  const int64_t nc = G->status ? 0 : G->ncells;
-  for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nc;
-       c += int64_t(gridDim.x) * blockDim.x)
-    nchunk[c] = (count[c] + 31) >> 5;
-}
-
 __global__ void sp_place_kernel(const float* __restrict__ X, int64_t n, int d,
                                 const SpGrid* __restrict__ G, const int64_t* __restrict__ cell,
                                 const int64_t* __restrict__ cell_start, int32_t* __restrict__ cursor,
@@ -200,23 +213,6 @@ __global__ void sp_place_kernel(const float* __restrict__ X, int64_t n, int d,
     const int64_t pos = cell_start[c] + atomicAdd(&cursor[c], 1);
     const float* p = X + i * d;
     pts[pos] = make_float4(p[0], p[1], d == 3 ? p[2] : 0.f, __int_as_float(int(i)));
-  }
-}
-
-// chunk j → (its cell, its first sorted position): the cell is the last c with
-// chunk_start[c] <= j (binary search), so a cell with many points spreads over many threads
-__global__ void sp_chunks_kernel(const int64_t* __restrict__ cell_start,
-                                 const int64_t* __restrict__ chunk_start, int64_t cap,
-                                 int2* __restrict__ chunks) {
-  const int64_t total = chunk_start[cap];
-  for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < total;
-       j += int64_t(gridDim.x) * blockDim.x) {
-    int64_t lo = 0, hi = cap;                 // chunk_start[lo] <= j < chunk_start[hi]
-    while (hi - lo > 1) {
-      const int64_t mid = lo + (hi - lo) / 2;
-      if (chunk_start[mid] <= j) lo = mid; else hi = mid;
-    }
-    chunks[j] = make_int2(int(lo), int(cell_start[lo] + (j - chunk_start[lo]) * 32));
   }
 }
 
@@ -245,45 +241,39 @@ __device__ __forceinline__ float prefilter(float top) {
   return __fmul_ru(up, up);
 }
 
-// Stage the points [a, b) through the warp's shared buffer; f(candidate) runs on every lane.
+// f(point) for the points [a, b), four loads in flight
 template <class F>
 __device__ __forceinline__ void scan_run(const float4* __restrict__ pts, int64_t a, int64_t b,
-                                         float4* stage, int lane, F&& f) {
-  for (int64_t base = a; base < b; base += SP_STAGE) {
-    const int cnt = int(imin64(SP_STAGE, b - base));
-    __syncwarp();
-    for (int j = lane; j < cnt; j += 32) stage[j] = pts[base + j];
-    __syncwarp();
-    for (int t = 0; t < cnt; ++t) f(stage[t]);
+                                         F&& f) {
+  for (; a + 4 <= b; a += 4) {
+    const float4 p0 = pts[a], p1 = pts[a + 1], p2 = pts[a + 2], p3 = pts[a + 3];
+    f(p0);
+    f(p1);
+    f(p2);
+    f(p3);
   }
+  for (; a < b; ++a) f(pts[a]);
 }
 
+// blocks per SM by list length: latency-bound walks want warps (K = 8: 0.67 -> 0.55 ms at 10 blocks)
+constexpr int knn_blocks(int K) { return K <= 8 ? 10 : (K <= 16 ? 6 : (K <= 32 ? 4 : 2)); }
 template <int K, int D>
-__global__ void __launch_bounds__(SP_T)
+__global__ void __launch_bounds__(SP_T, knn_blocks(K))
 sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_start,
-              const int2* __restrict__ chunks, const int64_t* __restrict__ chunk_start,
-              const SpGrid* __restrict__ G, int k, int32_t* __restrict__ out_idx,
-              float* __restrict__ out_dist, unsigned long long* __restrict__ counters) {
-  __shared__ float4 stage_all[SP_W][SP_STAGE];
+              const SpGrid* __restrict__ G, int64_t n, int k, int32_t* __restrict__ out_idx,
+              float* __restrict__ out_dist, unsigned long long* __restrict__ counters,
+              int32_t* __restrict__ far_rows, int32_t* __restrict__ n_far) {
   const SpGrid g = *G;
   if (g.status) return;
   const int lane = threadIdx.x & 31;
-  float4* stage = stage_all[threadIdx.x >> 5];
-  const int64_t nchunks = chunk_start[g.ncells];
-  const int64_t wid = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int m = k - 1;
   unsigned long long evals = 0, expanded = 0;
-  for (int64_t ch = wid; ch < nchunks; ch += nw) {
-    const int2 c = chunks[ch];
-    const int64_t qend = imin64(int64_t(c.y) + 32, cell_start[int64_t(c.x) + 1]);
-    const int64_t qpos = int64_t(c.y) + lane;
-    const bool active = qpos < qend;
-    const float4 q = active ? pts[qpos] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int qi = active ? __float_as_int(q.w) : -1;
-    const int cx = int(int64_t(c.x) % g.g[0]);
-    const int cy = int((int64_t(c.x) / g.g[0]) % g.g[1]);
-    const int cz = int(int64_t(c.x) / (int64_t(g.g[0]) * g.g[1]));
+  for (int64_t pos = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; pos < n;
+       pos += int64_t(gridDim.x) * blockDim.x) {
+    const float4 q = pts[pos];
+    const int qi = __float_as_int(q.w);
+    const int cx = cell_axis(q.x, g, 0), cy = cell_axis(q.y, g, 1);
+    const int cz = D == 3 ? cell_axis(q.z, g, 2) : 0;
     float s[K];
     int id[K];
 #pragma unroll
@@ -293,14 +283,11 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
       id[j] = sent ? -1 : INT_MAX;
     }
     float t2 = prefilter(s[K - 1]);
-    bool done = !active;
     const int rmax = max(max(cx, g.g[0] - 1 - cx),
                          max(max(cy, g.g[1] - 1 - cy), D == 3 ? max(cz, g.g[2] - 1 - cz) : 0));
     auto visit = [&](const float4& p) {
-      if (done) return;
       const float d2 = sq_dist<D>(p, q);
       const int pid = __float_as_int(p.w);
-      ++evals;
       if (d2 <= t2 && pid != qi) {
         const float sd = __fsqrt_rn(d2);
         if (key_less(sd, pid, s[K - 1], id[K - 1])) {
@@ -323,55 +310,77 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
       x1 = min(x1, g.g[0] - 1);
       if (x0 > x1 || y < 0 || y >= g.g[1] || z < 0 || z >= g.g[2]) return;
       const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
-      scan_run(pts, cell_start[row + x0], cell_start[row + x1 + 1], stage, lane, visit);
+      const int64_t a = cell_start[row + x0], b = cell_start[row + x1 + 1];
+      evals += b - a;
+      scan_run(pts, a, b, visit);
     };
-    for (int R = 0;; ++R) {
-      const int zlo = D == 3 ? -R : 0, zhi = D == 3 ? R : 0;
+    // Boxes of cells |d| <= R around the query's cell, R = 1 first; the cells of the last box (P) are
+    // left out of the next, and rows of cells beyond the list's last distance r are skipped.  r says
+    // which box is enough; a query that is not done within LANE_R (far from other points) goes to
+    // the warp pass: its one lane would walk thousands of row ranges while the launch waits.
+    bool defer = false;
+    for (int P = -1, R = 1;;) {
+      const int zlo = D == 3 ? max(-R, -cz) : 0, zhi = D == 3 ? min(R, g.g[2] - 1 - cz) : 0;
       for (int dz = zlo; dz <= zhi; ++dz) {
-        for (int dy = -R; dy <= R; ++dy) {
-          const bool full = (dy == -R || dy == R || (D == 3 && (dz == -R || dz == R)));
-          if (full) {
+        for (int dy = max(-R, -cy); dy <= min(R, g.g[1] - 1 - cy); ++dy) {
+          if (P >= 1) {
+            const double far = double(s[K - 1]) * (1.0 + 4e-6) + g.eps_abs;
+            const double ly = g.o[1] + double(cy + dy) * g.cs;           // the row's lower face
+            if (ly - double(q.y) > far || double(q.y) - (ly + g.cs) > far) continue;
+            if (D == 3) {
+              const double lz = g.o[2] + double(cz + dz) * g.cs;
+              if (lz - double(q.z) > far || double(q.z) - (lz + g.cs) > far) continue;
+            }
+          }
+          if (abs(dy) > P || (D == 3 && abs(dz) > P)) {
             run(cy + dy, cz + dz, cx - R, cx + R);
           } else {
-            run(cy + dy, cz + dz, cx - R, cx - R);
-            run(cy + dy, cz + dz, cx + R, cx + R);
+            run(cy + dy, cz + dz, cx - R, cx - P - 1);
+            run(cy + dy, cz + dz, cx + P + 1, cx + R);
           }
         }
       }
-      if (!done) {
-        // distance from the query to the nearest face of the box of cells within R that has
-        // points beyond it; a box that reaches the grid's edge on a side bounds nothing there
-        double bound = INFINITY;
-        const int cc[3] = {cx, cy, cz};
-        const float qq[3] = {q.x, q.y, q.z};
+      // distance from the query to the nearest face of the box of cells within R that has
+      // points beyond it; a box that reaches the grid's edge on a side bounds nothing there
+      double bound = INFINITY;
+      const int cc[3] = {cx, cy, cz};
+      const float qq[3] = {q.x, q.y, q.z};
 #pragma unroll
-        for (int a = 0; a < D; ++a) {
-          if (cc[a] - R > 0)
-            bound = fmin(bound, double(qq[a]) - (g.o[a] + double(cc[a] - R) * g.cs));
-          if (cc[a] + R < g.g[a] - 1)
-            bound = fmin(bound, (g.o[a] + double(cc[a] + R + 1) * g.cs) - double(qq[a]));
-        }
-        if (isinf(bound) || double(s[K - 1]) < bound * (1.0 - 4e-6) - g.eps_abs) {
-          done = true;
-          if (R >= 2) ++expanded;
-        }
+      for (int a = 0; a < D; ++a) {
+        if (cc[a] - R > 0)
+          bound = fmin(bound, double(qq[a]) - (g.o[a] + double(cc[a] - R) * g.cs));
+        if (cc[a] + R < g.g[a] - 1)
+          bound = fmin(bound, (g.o[a] + double(cc[a] + R + 1) * g.cs) - double(qq[a]));
       }
-      if (__all_sync(0xffffffffu, done) || R >= rmax) break;
+      const double r = double(s[K - 1]);
+      if (isinf(bound) || r < bound * (1.0 - 4e-6) - g.eps_abs || R >= rmax) {
+        if (R >= 2) ++expanded;
+        break;
+      }
+      P = R;
+      // the faces of box R lie at least R·cs away, so R > r / cs ends the walk
+      const double want = isinf(r) ? double(R + 1) : r * (1.0 + 1e-5) / g.cs + 1.0;
+      R = max(R + 1, int(fmin(want, double(rmax))));
+      if (R > LANE_R) { defer = true; break; }
     }
-    if (active) {
-      int32_t* oi = out_idx + int64_t(qi) * k;
-      float* od = out_dist + int64_t(qi) * k;
-      oi[0] = qi;
-      od[0] = 0.f;
+    if (defer) {
+      far_rows[atomicAdd(n_far, 1)] = int32_t(pos);
+      ++expanded;
+      continue;
+    }
+    int32_t* oi = out_idx + int64_t(qi) * k;
+    float* od = out_dist + int64_t(qi) * k;
+    oi[0] = qi;
+    od[0] = 0.f;
 #pragma unroll
-      for (int j = 0; j < K; ++j) {
-        if (j >= K - m) {
-          oi[1 + j - (K - m)] = id[j];
-          od[1 + j - (K - m)] = s[j];
-        }
+    for (int j = 0; j < K; ++j) {
+      if (j >= K - m) {
+        oi[1 + j - (K - m)] = id[j];
+        od[1 + j - (K - m)] = s[j];
       }
     }
   }
+  __syncwarp();
   for (int off = 16; off > 0; off >>= 1) {
     evals += __shfl_xor_sync(0xffffffffu, evals, off);
     expanded += __shfl_xor_sync(0xffffffffu, expanded, off);
@@ -382,43 +391,153 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
   }
 }
 
+// The queries the lane pass left open, a warp each: the lanes share a box's rows of cells.  First the
+// smallest box of a doubling sequence that holds k points (from the cell starts alone), then that
+// box's (k-1)-th distance r, then the rows and cells within r: every point that can be nearer.
+// Each lane keeps a sorted list of what it sees; the warp takes the smallest head m times.
+template <int K, int D>
+__global__ void __launch_bounds__(SP_T)
+sp_knn_far_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_start,
+                  const SpGrid* __restrict__ G, int k, const int32_t* __restrict__ far_rows,
+                  const int32_t* __restrict__ n_far, int32_t* __restrict__ out_idx,
+                  float* __restrict__ out_dist, unsigned long long* __restrict__ counters) {
+  const SpGrid g = *G;
+  if (g.status) return;
+  const int lane = threadIdx.x & 31;
+  const int m = k - 1, total = *n_far;
+  unsigned long long evals = 0;
+  for (int w = int((blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5); w < total;
+       w += int((int64_t(gridDim.x) * blockDim.x) >> 5)) {
+    const float4 q = pts[far_rows[w]];
+    const int qi = __float_as_int(q.w);
+    const int c[3] = {cell_axis(q.x, g, 0), cell_axis(q.y, g, 1),
+                      D == 3 ? cell_axis(q.z, g, 2) : 0};
+    const float qq[3] = {q.x, q.y, q.z};
+    int rmax = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a) rmax = max(rmax, max(c[a], g.g[a] - 1 - c[a]));
+    // f(first, last + 1) for the lane's rows of box R, cut to the cells within r
+    auto rows = [&](int R, double r, auto&& f) {
+      const int y0 = max(c[1] - R, 0), y1 = min(c[1] + R, g.g[1] - 1), ny = y1 - y0 + 1;
+      const int z0 = D == 3 ? max(c[2] - R, 0) : 0, z1 = D == 3 ? min(c[2] + R, g.g[2] - 1) : 0;
+      for (int64_t e = lane; e < int64_t(ny) * (z1 - z0 + 1); e += 32) {
+        const int y = y0 + int(e % ny), z = z0 + int(e / ny);
+        double rest = r * r;                       // (reach along x)², from the row's distance
+        const double ly = g.o[1] + double(y) * g.cs;
+        const double ey = fmax(0.0, fmax(ly - double(qq[1]), double(qq[1]) - (ly + g.cs)));
+        rest -= ey * ey;
+        if (D == 3) {
+          const double lz = g.o[2] + double(z) * g.cs;
+          const double ez = fmax(0.0, fmax(lz - double(qq[2]), double(qq[2]) - (lz + g.cs)));
+          rest -= ez * ez;
+        }
+        if (rest < 0.0) continue;
+        int x0 = max(c[0] - R, 0), x1 = min(c[0] + R, g.g[0] - 1);
+        if (rest < 1e300) {                        // one cell to spare on either side
+          const double h = sqrt(rest) / g.cs + 1.0;
+          const double at = (double(qq[0]) - g.o[0]) / g.cs;
+          x0 = max(x0, int(fmax(floor(at - h), 0.0)));
+          x1 = min(x1, int(fmin(floor(at + h), double(g.g[0] - 1))));
+        }
+        if (x0 > x1) continue;
+        const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
+        f(cell_start[row + x0], cell_start[row + x1 + 1]);
+      }
+    };
+    int R = LANE_R;
+    for (;; R *= 2) {
+      long long have = 0;
+      rows(min(R, rmax), INFINITY, [&](int64_t a, int64_t b) { have += b - a; });
+      for (int off = 16; off > 0; off >>= 1) have += __shfl_xor_sync(0xffffffffu, have, off);
+      if (have >= k || R >= rmax) break;
+    }
+    float s[K];
+    int id[K];
+    double r = INFINITY;
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) { s[j] = INFINITY; id[j] = INT_MAX; }
+      rows(min(R, rmax), r, [&](int64_t a, int64_t b) {
+        evals += b - a;
+        for (; a < b; ++a) {
+          const float4 p = pts[a];
+          const int pid = __float_as_int(p.w);
+          const float sd = __fsqrt_rn(sq_dist<D>(p, q));
+          if (pid == qi || !key_less(sd, pid, s[K - 1], id[K - 1])) continue;
+#pragma unroll
+          for (int j = K - 1; j > 0; --j) {
+            const bool lp = key_less(sd, pid, s[j - 1], id[j - 1]);
+            const bool lc = key_less(sd, pid, s[j], id[j]);
+            const float ns = lp ? s[j - 1] : (lc ? sd : s[j]);
+            const int ni = lp ? id[j - 1] : (lc ? pid : id[j]);
+            s[j] = ns;
+            id[j] = ni;
+          }
+          if (key_less(sd, pid, s[0], id[0])) { s[0] = sd; id[0] = pid; }
+        }
+      });
+      // the m smallest heads of the lanes' sorted lists, in order
+      float last = INFINITY;
+      for (int t = 0; t < m; ++t) {
+        float bs = s[0];
+        int bi = id[0];
+        for (int off = 16; off > 0; off >>= 1) {
+          const float os = __shfl_xor_sync(0xffffffffu, bs, off);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+          if (key_less(os, oi, bs, bi)) { bs = os; bi = oi; }
+        }
+        if (id[0] == bi && s[0] == bs && bi != INT_MAX) {
+#pragma unroll
+          for (int j = 0; j + 1 < K; ++j) { s[j] = s[j + 1]; id[j] = id[j + 1]; }
+          s[K - 1] = INFINITY;
+          id[K - 1] = INT_MAX;
+        }
+        last = bs;
+        if (pass == 1 && lane == 0) {
+          out_idx[int64_t(qi) * k + 1 + t] = bi;
+          out_dist[int64_t(qi) * k + 1 + t] = bs;
+        }
+      }
+      // every point within r of the query lies in the cells within r (margin: float32 and FP64
+      // rounding, as in the lane pass)
+      r = double(last) * (1.0 + 8e-6) + 2.0 * g.eps_abs;
+      const double need = r / g.cs + 1.0;
+      R = isinf(last) || need >= double(rmax) ? rmax : max(1, int(need));
+    }
+    if (lane == 0) {
+      out_idx[int64_t(qi) * k] = qi;
+      out_dist[int64_t(qi) * k] = 0.f;
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) evals += __shfl_xor_sync(0xffffffffu, evals, off);
+  if (lane == 0 && evals) atomicAdd(&counters[0], evals);
+}
+
 // Radius search.  pass 0 counts into count[qi]; pass 1 writes (column, distance) from
 // indptr[qi] in the same walk order.
 template <int D>
 __global__ void __launch_bounds__(SP_T)
 sp_radius_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_start,
-                 const int2* __restrict__ chunks, const int64_t* __restrict__ chunk_start,
-                 const SpGrid* __restrict__ G, float r2lo, float r2hi, int pass,
+                 const SpGrid* __restrict__ G, int64_t n, float r2lo, float r2hi, int pass,
                  int32_t* __restrict__ count, const int64_t* __restrict__ indptr,
                  int32_t* __restrict__ col, float* __restrict__ val,
                  unsigned long long* __restrict__ counters) {
-  __shared__ float4 stage_all[SP_W][SP_STAGE];
   const SpGrid g = *G;
   if (g.status) return;
   const int lane = threadIdx.x & 31;
-  float4* stage = stage_all[threadIdx.x >> 5];
-  const int64_t nchunks = chunk_start[g.ncells];
-  const int64_t wid = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int R = g.ring;
   unsigned long long evals = 0;
-  for (int64_t ch = wid; ch < nchunks; ch += nw) {
-    const int2 c = chunks[ch];
-    const int64_t qend = imin64(int64_t(c.y) + 32, cell_start[int64_t(c.x) + 1]);
-    const int64_t qpos = int64_t(c.y) + lane;
-    const bool active = qpos < qend;
-    const float4 q = active ? pts[qpos] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int qi = active ? __float_as_int(q.w) : -1;
-    const int cx = int(int64_t(c.x) % g.g[0]);
-    const int cy = int((int64_t(c.x) / g.g[0]) % g.g[1]);
-    const int cz = int(int64_t(c.x) / (int64_t(g.g[0]) * g.g[1]));
-    int64_t w = (pass == 1 && active) ? indptr[qi] : 0;
+  for (int64_t pos = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; pos < n;
+       pos += int64_t(gridDim.x) * blockDim.x) {
+    const float4 q = pts[pos];
+    const int qi = __float_as_int(q.w);
+    const int cx = cell_axis(q.x, g, 0), cy = cell_axis(q.y, g, 1);
+    const int cz = D == 3 ? cell_axis(q.z, g, 2) : 0;
+    int64_t w = pass == 1 ? indptr[qi] : 0;
     int32_t cnt = 0;
     auto visit = [&](const float4& p) {
-      if (!active) return;
       const float d2 = sq_dist<D>(p, q);
       const int pid = __float_as_int(p.w);
-      ++evals;
       if (pid != qi && d2 <= r2hi && d2 >= r2lo) {
         if (pass == 1) {
           col[w] = pid;
@@ -433,11 +552,14 @@ sp_radius_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cel
     for (int z = zlo; z <= zhi; ++z) {
       for (int y = max(cy - R, 0); y <= min(cy + R, g.g[1] - 1); ++y) {
         const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
-        scan_run(pts, cell_start[row + x0], cell_start[row + x1 + 1], stage, lane, visit);
+        const int64_t a = cell_start[row + x0], b = cell_start[row + x1 + 1];
+        evals += b - a;
+        scan_run(pts, a, b, visit);
       }
     }
-    if (pass == 0 && active) count[qi] = cnt;
+    if (pass == 0) count[qi] = cnt;
   }
+  __syncwarp();
   for (int off = 16; off > 0; off >>= 1) evals += __shfl_xor_sync(0xffffffffu, evals, off);
   if (lane == 0) atomicAdd(&counters[0], evals);
 }
@@ -456,6 +578,17 @@ sp_sort_rows_kernel(const int64_t* __restrict__ indptr, int64_t n, const int32_t
   for (int64_t row = wid; row < n; row += nw) {
     const int64_t a = indptr[row];
     const int64_t m = indptr[row + 1] - a;
+    if (m <= 32) {                                      // one entry a lane
+      const int32_t mine = lane < m ? col_in[a + lane] : INT_MAX;
+      const float v = lane < m ? val_in[a + lane] : 0.f;
+      int rank = 0;
+      for (int t = 0; t < int(m); ++t) rank += __shfl_sync(0xffffffffu, mine, t) < mine;
+      if (lane < m) {
+        col_out[a + rank] = mine;
+        val_out[a + rank] = v;
+      }
+      continue;
+    }
     for (int64_t g0 = 0; g0 < m; g0 += 32 * SORT_E) {
       int32_t mine[SORT_E];
       int64_t rank[SORT_E];
@@ -511,20 +644,21 @@ __global__ void sp_edge_len_kernel(const double* __restrict__ X, int d,
   }
 }
 
-__global__ void sp_init_kernel(unsigned* mm, unsigned long long* nonfinite, unsigned long long* counters) {
+__global__ void sp_init_kernel(unsigned* mm, unsigned long long* nonfinite,
+                               unsigned long long* counters, int32_t* n_far) {
   if (threadIdx.x < 3) { mm[threadIdx.x] = 0xffffffffu; mm[3 + threadIdx.x] = 0u; }
-  if (threadIdx.x == 0) { *nonfinite = 0; counters[0] = 0; counters[1] = 0; }
+  if (threadIdx.x == 0) { *nonfinite = 0; *n_far = 0; counters[0] = 0; counters[1] = 0; }
 }
 
 __global__ void sp_stats_kernel(const SpGrid* __restrict__ G, const unsigned long long* __restrict__ nonfinite,
-                                const unsigned long long* __restrict__ counters,
-                                const int64_t* __restrict__ chunk_start, int64_t* __restrict__ stats) {
+                                const unsigned long long* __restrict__ counters, int64_t n,
+                                int64_t* __restrict__ stats) {
   if (threadIdx.x != 0) return;
   const SpGrid g = *G;
   stats[MSC_SP_STAT_NONFINITE] = int64_t(*nonfinite);
   stats[MSC_SP_STAT_STATUS] = g.status;
   stats[MSC_SP_STAT_CELLS] = g.status ? 0 : g.ncells;
-  stats[MSC_SP_STAT_CHUNKS] = g.status ? 0 : chunk_start[g.ncells];
+  stats[MSC_SP_STAT_CHUNKS] = g.status ? 0 : (n + 31) / 32;
   stats[MSC_SP_STAT_EVALS] = int64_t(counters[0]);
   stats[MSC_SP_STAT_EXPANDED] = int64_t(counters[1]);
   stats[MSC_SP_STAT_RING] = g.status ? 0 : g.ring;
@@ -538,13 +672,12 @@ struct SpWs {
   unsigned long long* counters;
   int64_t* cell;          // [n]
   int32_t* count;         // [cap]
-  int32_t* cursor;        // [cap]
-  int32_t* nchunk;        // [cap]
+  int32_t* cursor;        // [cap], right behind count
   int64_t* cell_start;    // [cap + 1]
-  int64_t* chunk_start;   // [cap + 1]
   int64_t* scan_scratch;
   float4* pts;            // [n]
-  int2* chunks;           // [cap + n / 32 + 1]
+  int32_t* far_rows;      // [n] queries of the warp pass
+  int32_t* n_far;
 };
 
 int64_t cell_cap(int64_t n) { return 4 * n + 16; }
@@ -559,12 +692,11 @@ SpWs carve(Carver& c, int64_t n) {
   w.cell = c.take<int64_t>(n);
   w.count = c.take<int32_t>(cap);
   w.cursor = c.take<int32_t>(cap);
-  w.nchunk = c.take<int32_t>(cap);
   w.cell_start = c.take<int64_t>(cap + 1);
-  w.chunk_start = c.take<int64_t>(cap + 1);
   w.scan_scratch = c.take<int64_t>(scan_i32_scratch_elems(cap));
   w.pts = c.take<float4>(n);
-  w.chunks = c.take<int2>(cap + n / 32 + 1);
+  w.far_rows = c.take<int32_t>(n);
+  w.n_far = c.take<int32_t>(1);
   return w;
 }
 
@@ -574,54 +706,53 @@ unsigned flat_grid(int64_t items, int threads) {
   return unsigned(std::max<int64_t>(1, std::min<int64_t>(b, int64_t(num_sms()) * 16)));
 }
 
-// The grid: bounding box, plan, binning, cell-ordered points, chunks.  The cell table is sized
+// The grid: bounding box, plan, binning, cell-ordered points.  The cell table is sized
 // for the cap; the plan never uses more cells than that.
 int build_grid(const float* X, int64_t n, int d, int mode, int k, double reach, const SpWs& w,
                cudaStream_t st) {
   const int64_t cap = cell_cap(n);
-  sp_init_kernel<<<1, 32, 0, st>>>(w.mm, w.nonfinite, w.counters);
+  sp_init_kernel<<<1, 32, 0, st>>>(w.mm, w.nonfinite, w.counters, w.n_far);
   MSC_LAUNCH_CHECK();
   sp_bbox_kernel<<<flat_grid(n, 256), 256, 0, st>>>(X, n, d, w.mm, w.nonfinite);
   MSC_LAUNCH_CHECK();
   sp_plan_kernel<<<1, 32, 0, st>>>(w.mm, w.nonfinite, n, d, mode, k, reach, w.G);
   MSC_LAUNCH_CHECK();
-  MSC_CUDA_TRY(cudaMemsetAsync(w.count, 0, sizeof(int32_t) * cap, st));
-  MSC_CUDA_TRY(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * cap, st));
-  MSC_CUDA_TRY(cudaMemsetAsync(w.nchunk, 0, sizeof(int32_t) * cap, st));
+  // counts and cursors lie one behind the other: one memset
+  MSC_CUDA_TRY(cudaMemsetAsync(w.count, 0, reinterpret_cast<char*>(w.cursor + cap) -
+                                               reinterpret_cast<char*>(w.count), st));
   sp_bin_kernel<<<flat_grid(n, 256), 256, 0, st>>>(X, n, d, w.G, w.cell, w.count);
   MSC_LAUNCH_CHECK();
-  sp_chunk_count_kernel<<<flat_grid(cap, 256), 256, 0, st>>>(w.count, w.G, w.nchunk);
-  MSC_LAUNCH_CHECK();
-  // scans over the whole cap: cells the plan does not use hold zero counts, so
-  // cell_start[ncells] = n and chunk_start[ncells] = the number of chunks
+  // a scan over the whole cap: cells the plan does not use hold zero counts, so
+  // cell_start[ncells] = n
   MSC_TRY(scan_excl_i32(w.count, cap, w.cell_start, w.scan_scratch, st));
-  MSC_TRY(scan_excl_i32(w.nchunk, cap, w.chunk_start, w.scan_scratch, st));
   sp_place_kernel<<<flat_grid(n, 256), 256, 0, st>>>(X, n, d, w.G, w.cell, w.cell_start, w.cursor,
                                                       w.pts);
-  MSC_LAUNCH_CHECK();
-  sp_chunks_kernel<<<flat_grid(cap + n / 32 + 1, 256), 256, 0, st>>>(w.cell_start, w.chunk_start,
-                                                                       cap, w.chunks);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
 
+// one lane per query; as many blocks as there are queries, up to four waves of full SMs
 unsigned search_grid(int64_t n) {
-  // persistent: enough warps for every chunk of a uniform layout, at most 8 blocks per SM
-  const int64_t warps = n / 16 + 1;
-  const int64_t blocks = (warps + SP_W - 1) / SP_W;
-  return unsigned(std::max<int64_t>(1, std::min<int64_t>(blocks, int64_t(num_sms()) * 8)));
+  const int64_t blocks = (n + SP_T - 1) / SP_T;
+  return unsigned(std::max<int64_t>(1, std::min<int64_t>(blocks, int64_t(num_sms()) * 64)));
 }
 
 template <int K>
 int launch_knn_k(const SpWs& w, int64_t n, int d, int k, int32_t* idx, float* dist, cudaStream_t st) {
   if (d == 2)
-    sp_knn_kernel<K, 2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                         w.chunk_start, w.G, k, idx, dist,
-                                                         w.counters);
+    sp_knn_kernel<K, 2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, k, idx,
+                                                         dist, w.counters, w.far_rows, w.n_far);
   else
-    sp_knn_kernel<K, 3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                         w.chunk_start, w.G, k, idx, dist,
-                                                         w.counters);
+    sp_knn_kernel<K, 3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, k, idx,
+                                                         dist, w.counters, w.far_rows, w.n_far);
+  MSC_LAUNCH_CHECK();
+  const unsigned gf = search_grid(std::min<int64_t>(n * 32, int64_t(num_sms()) * 16 * SP_T));
+  if (d == 2)
+    sp_knn_far_kernel<K, 2><<<gf, SP_T, 0, st>>>(w.pts, w.cell_start, w.G, k, w.far_rows, w.n_far,
+                                                 idx, dist, w.counters);
+  else
+    sp_knn_far_kernel<K, 3><<<gf, SP_T, 0, st>>>(w.pts, w.cell_start, w.G, k, w.far_rows, w.n_far,
+                                                 idx, dist, w.counters);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
@@ -644,7 +775,7 @@ int launch_spatial_knn(const float* X, int64_t n, int d, int k, int32_t* idx, fl
   else if (m <= 16) MSC_TRY(launch_knn_k<16>(w, n, d, k, idx, dist, st));
   else if (m <= 32) MSC_TRY(launch_knn_k<32>(w, n, d, k, idx, dist, st));
   else MSC_TRY(launch_knn_k<64>(w, n, d, k, idx, dist, st));
-  sp_stats_kernel<<<1, 32, 0, st>>>(w.G, w.nonfinite, w.counters, w.chunk_start, stats);
+  sp_stats_kernel<<<1, 32, 0, st>>>(w.G, w.nonfinite, w.counters, n, stats);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
@@ -666,16 +797,16 @@ int launch_spatial_radius_count(const float* X, int64_t n, int d, double radius,
   MSC_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, sizeof(int32_t) * n, st));
   const float r2hi = float(radius * radius), r2lo = float(min_radius * min_radius);
   if (d == 2)
-    sp_radius_kernel<2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                         w.chunk_start, w.G, r2lo, r2hi, 0, rowcnt,
-                                                         nullptr, nullptr, nullptr, w.counters);
+    sp_radius_kernel<2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, r2lo,
+                                                         r2hi, 0, rowcnt, nullptr, nullptr,
+                                                         nullptr, w.counters);
   else
-    sp_radius_kernel<3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                         w.chunk_start, w.G, r2lo, r2hi, 0, rowcnt,
-                                                         nullptr, nullptr, nullptr, w.counters);
+    sp_radius_kernel<3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, r2lo,
+                                                         r2hi, 0, rowcnt, nullptr, nullptr,
+                                                         nullptr, w.counters);
   MSC_LAUNCH_CHECK();
   MSC_TRY(scan_excl_i32(rowcnt, n, indptr, w.scan_scratch, st));
-  sp_stats_kernel<<<1, 32, 0, st>>>(w.G, w.nonfinite, w.counters, w.chunk_start, stats);
+  sp_stats_kernel<<<1, 32, 0, st>>>(w.G, w.nonfinite, w.counters, n, stats);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
@@ -698,17 +829,15 @@ int launch_spatial_radius_fill(int64_t n, int d, double radius, double min_radiu
   const float r2hi = float(radius * radius), r2lo = float(min_radius * min_radius);
   if (nnz > 0) {
     if (d == 2)
-      sp_radius_kernel<2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                           w.chunk_start, w.G, r2lo, r2hi, 1,
-                                                           nullptr, indptr, col_tmp, val_tmp,
-                                                           w.counters);
+      sp_radius_kernel<2><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, r2lo,
+                                                           r2hi, 1, nullptr, indptr, col_tmp,
+                                                           val_tmp, w.counters);
     else
-      sp_radius_kernel<3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.chunks,
-                                                           w.chunk_start, w.G, r2lo, r2hi, 1,
-                                                           nullptr, indptr, col_tmp, val_tmp,
-                                                           w.counters);
+      sp_radius_kernel<3><<<search_grid(n), SP_T, 0, st>>>(w.pts, w.cell_start, w.G, n, r2lo,
+                                                           r2hi, 1, nullptr, indptr, col_tmp,
+                                                           val_tmp, w.counters);
     MSC_LAUNCH_CHECK();
-    sp_sort_rows_kernel<<<search_grid(n * 8), SP_T, 0, st>>>(indptr, n, col_tmp, val_tmp, cols,
+    sp_sort_rows_kernel<<<search_grid(n * 32), SP_T, 0, st>>>(indptr, n, col_tmp, val_tmp, cols,
                                                              dist);
     MSC_LAUNCH_CHECK();
   }
