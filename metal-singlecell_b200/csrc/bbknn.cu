@@ -19,10 +19,17 @@
 //            cells it cannot certify take an FP64 scan of the batch;
 //   merge    every cell's K entries sorted by (float32 distance, index).
 //
+// Large inputs (BbPlan::ordered): the cells go into locality order first, queries and each batch's
+// keys alike; a near pass scans every query tile's nearest key tile of each batch, and its radii give
+// masks of the key tiles that can still matter (prune.cu), so that a query tile visits a few tiles
+// of a batch instead of all.  All batches run in one launch per stage.  200,000 x 50, 8 batches, 3
+// neighbours in each: the graph 38.0 ms batch by batch, 13.3 ordered.
+//
 // The distances graph drops the diagonal and every zero distance (neighbors.py:554-557); the
 // trimming keeps an entry (i, j) of value v when v != 0, v >= θ_i and v >= θ_j, θ_i being the
 // trim-th largest stored value of row i when the row stores more than `trim` entries, else 0.
 #include <algorithm>
+#include <cstdlib>
 
 #include "kernels.cuh"
 #include "msc_warpsort.cuh"
@@ -70,6 +77,70 @@ __global__ void bb_place_kernel(const int32_t* __restrict__ codes, int64_t n, in
   }
 }
 
+// the same from the cells in locality order (positions j, cells gperm[j])
+__global__ void bb_flag_order_kernel(const int32_t* __restrict__ codes,
+                                     const int32_t* __restrict__ gperm, int64_t n, int b,
+                                     int32_t* __restrict__ flag) {
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n;
+       j += int64_t(gridDim.x) * blockDim.x)
+    flag[j] = codes[gperm[j]] == b ? 1 : 0;
+}
+__global__ void bb_place_order_kernel(const int32_t* __restrict__ flag,
+                                      const int32_t* __restrict__ gperm,
+                                      const int32_t* __restrict__ gleaf, int64_t n,
+                                      const int64_t* __restrict__ S, int64_t poff, int64_t nb,
+                                      int32_t* __restrict__ perm, int32_t* __restrict__ leaf) {
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n;
+       j += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t r = S[j];
+    if (flag[j] && r < nb) {
+      perm[poff + r] = gperm[j];
+      leaf[poff + r] = gleaf[j];
+    }
+  }
+}
+__global__ void bb_query_order_kernel(const int32_t* __restrict__ gperm,
+                                      const int32_t* __restrict__ gleaf, int64_t n, int64_t p1,
+                                      int32_t* __restrict__ perm, int32_t* __restrict__ leaf,
+                                      int32_t* __restrict__ qmap) {
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < n;
+       j += int64_t(gridDim.x) * blockDim.x) {
+    perm[p1 + j] = gperm[j];
+    leaf[p1 + j] = gleaf[j];
+    qmap[j] = int32_t(p1 + j);
+  }
+}
+
+// the batches of one launch
+constexpr int BB_GROUP = 64;
+struct BbBatches {
+  int32_t poff[BB_GROUP], nb[BB_GROUP], kk[BB_GROUP], col0[BB_GROUP];
+};
+
+// batch-major items of a group: scan items (query rows of the list) and plan items (packed rows)
+__global__ void bb_group_items_kernel(const BbBatches B, int nb, int64_t n, int64_t p1,
+                                      WorkItem* __restrict__ items,
+                                      WorkItem* __restrict__ pitems) {
+  const int64_t nt = (n + QTILE - 1) / QTILE;
+  for (int64_t x = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; x < nt * nb;
+       x += int64_t(gridDim.x) * blockDim.x) {
+    const int b = int(x / nt);
+    const int64_t t = x - b * nt;
+    WorkItem w;
+    w.qrow0 = int32_t(t * QTILE);
+    w.nq = int32_t(min64(QTILE, n - t * QTILE));
+    w.key0 = B.poff[b];
+    w.nkeys = B.nb[b];
+    w.orig_off = 0;
+    w.qorig0 = 0;
+    w.pad0 = b;
+    w.pad1 = 0;
+    items[x] = w;
+    w.qrow0 += int32_t(p1);
+    pitems[x] = w;
+  }
+}
+
 __global__ void bb_set_i32_kernel(int32_t* __restrict__ p, int32_t v) { *p = v; }
 
 // query tiles of batch b: 128 listed cells each against the batch's keys
@@ -107,6 +178,82 @@ __device__ __forceinline__ float bb_d2_f32(const float* xs, const float* __restr
     acc = fmaf(df, df, acc);
   }
   return acc;
+}
+
+// the same for the scans: eight loads in flight (a scanned row waits for little else)
+__device__ __forceinline__ double bb_d2_f64_scan(const float* xs, const float* __restrict__ y,
+                                                 int d) {
+  double acc = 0.0;
+#pragma unroll 8
+  for (int t = 0; t < d; ++t) {
+    const double df = double(xs[t]) - double(y[t]);
+    acc += df * df;
+  }
+  return acc;
+}
+
+// four lanes' shares of an FP32 squared distance (part = lane & 3 takes every fourth 8-byte pair, or
+// every fourth element of a row that is not 8-byte aligned); any order of the sum stays within the
+// (d+4)·2^-24 the windows assume
+__device__ __forceinline__ float bb_part_d2_f32(const float* xs, const float* __restrict__ y,
+                                                int d, int part) {
+  float a0 = 0.f, a1 = 0.f;
+  if ((reinterpret_cast<uintptr_t>(y) & 7) == 0) {
+    const float2* y2 = reinterpret_cast<const float2*>(y);
+    const float2* x2 = reinterpret_cast<const float2*>(xs);
+    const int h = d >> 1;
+    for (int t = part; t < h; t += 4) {
+      const float2 u = y2[t], p = x2[t];
+      const float e0 = p.x - u.x, e1 = p.y - u.y;
+      a0 = fmaf(e0, e0, a0);
+      a1 = fmaf(e1, e1, a1);
+    }
+    if ((d & 1) && part == 0) {
+      const float e = xs[d - 1] - y[d - 1];
+      a0 = fmaf(e, e, a0);
+    }
+  } else {
+    for (int t = part; t < d; t += 4) {
+      const float e = xs[t] - y[t];
+      a0 = fmaf(e, e, a0);
+    }
+  }
+  return a0 + a1;
+}
+
+// a warp's FP64 scan of one batch (keys perm[0..nb)) for cell i: the kk <= 128 nearest by
+// (d², index) to oi / od
+__device__ __forceinline__ void bb_scan_row(const float* __restrict__ X, int d, int64_t i,
+                                            const int32_t* __restrict__ perm, int64_t nb, int kk,
+                                            float* xs, int32_t* oi, float* od) {
+  const int lane = lane_id();
+  const double INF = __longlong_as_double(0x7ff0000000000000ll);
+  for (int t = lane; t < d; t += 32) xs[t] = X[i * d + t];
+  __syncwarp();
+  WarpTop128 top;
+  top.init();
+  for (int64_t base = 0; base < nb; base += 32) {
+    const int64_t jj = base + lane;
+    double v = INF;
+    int vi = INT32_MAX;
+    if (jj < nb) {
+      const int32_t c = perm[jj];
+      if (c >= 0) {
+        v = bb_d2_f64_scan(xs, X + int64_t(c) * d, d);
+        vi = c;
+      }
+    }
+    top.offer(v, vi, kk);
+  }
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int r = s * 32 + lane;
+    if (r < kk) {
+      oi[r] = top.ai[s] == INT32_MAX ? int32_t(i) : top.ai[s];
+      od[r] = __double2float_rn(sqrt(top.a[s]));
+    }
+  }
+  __syncwarp();
 }
 
 // One warp per cell i: its k' candidates in batch b (original rows, -1 = none) → the kk nearest
@@ -176,6 +323,125 @@ bb_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1,
     atomicAdd(reinterpret_cast<unsigned long long*>(n_cert_out), (unsigned long long)n_cert);
 }
 
+// One warp per cell of the order and group of batches: its k' <= 32 candidates of each batch, as in
+// rerank.cu: FP32 distances with four lanes a candidate, the kk-th from a sort of the values alone,
+// FP64 for the few within its rounding bound, placed by counting.  (The kernel above reads a
+// candidate's row with one lane and sorts 64 FP64 pairs twice: 7.7 ms for 8 batches of 200,000
+// cells, 2.7 here.)  Cells it cannot certify, or with more than 32 candidates inside the bound
+// or NaN distances, are listed for the FP64 scan.
+__global__ void __launch_bounds__(BB_T)
+bb_group_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1,
+                       const int32_t* __restrict__ perm, const BbBatches B, int nb,
+                       const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_thr,
+                       int kprime, const QStat* __restrict__ qs, const KeyMax* __restrict__ km,
+                       const Ctl* __restrict__ ctl, int prec, int kmma, int K,
+                       int32_t* __restrict__ knn_idx, float* __restrict__ knn_dist,
+                       int32_t* __restrict__ fail_rows, int32_t* __restrict__ fail_bat,
+                       int32_t* __restrict__ nfail, int64_t* __restrict__ n_cert_out) {
+  __shared__ __align__(16) float xs_all[BB_WARPS][MSC_MAX_D];
+  __shared__ int win_all[BB_WARPS][32];
+  const int lane = lane_id(), wib = warp_id();
+  float* xs = xs_all[wib];
+  int* win = win_all[wib];
+  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  const KeyMax kmv = *km;
+  const double f = op_scale(prec, ctl);
+  const double f2 = f * f;
+  const double delta = double(d + 4) * 0x1p-24;
+  const double INF = __longlong_as_double(0x7ff0000000000000ll);
+  const unsigned lt = (1u << lane) - 1u;
+  int64_t n_cert = 0;
+  for (int64_t j = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; j < n; j += nwarps) {
+    const int64_t i = perm[p1 + j];
+    __syncwarp();
+    for (int t = lane; t < d; t += 32) xs[t] = X[i * d + t];
+    __syncwarp();
+    const QStat q = qs[p1 + j];
+    const double eps = cert_eps(q, kmv, prec, kmma, d);
+    for (int b = 0; b < nb; ++b) {
+      const int kk = B.kk[b];
+      const int c = lane < kprime ? cand_idx[(i * nb + b) * kprime + lane] : -1;
+      float e = F_INF;
+      for (int r = 0; r < kprime; r += 8) {              // eight candidates, four lanes each
+        const int s = r + (lane >> 2);
+        const int cid = __shfl_sync(FULL, c, s & 31);
+        const bool have = s < kprime && cid >= 0;
+        float v = have ? bb_part_d2_f32(xs, X + int64_t(cid) * d, d, lane & 3) : 0.f;
+        v += __shfl_xor_sync(FULL, v, 1);
+        v += __shfl_xor_sync(FULL, v, 2);
+        if (!have) v = F_INF;
+        const float got = __shfl_sync(FULL, v, ((lane - r) & 7) * 4);
+        if (lane >= r && lane < r + 8) e = got;
+      }
+      bool ok = !__any_sync(FULL, isnan(e));
+      float sv = e;
+      warp_sort32_f(sv);
+      const double lim = double(__shfl_sync(FULL, sv, kk - 1)) * (1.0 + 3.0 * delta) + 1e-300;
+      const bool in = c >= 0 && double(e) <= lim;
+      const unsigned m = __ballot_sync(FULL, in);
+      const int nw = __popc(m);
+      ok = ok && nw >= kk;
+      if (ok) {                                          // warp-uniform
+        if (in) win[__popc(m & lt)] = c;
+        __syncwarp();
+        const int id = lane < nw ? win[lane] : INT32_MAX;
+        const double g = lane < nw ? bb_d2_f64(xs, X + int64_t(id) * d, d) : INF;
+        int rank = 0;
+        for (int x = 0; x < nw; ++x) {
+          const double og = __shfl_sync(FULL, g, x);
+          const int oi = __shfl_sync(FULL, id, x);
+          rank += dless(og, oi, g, id);
+        }
+        // every key outside the list has an approximate value at or above T
+        const double T = double(cand_thr[b * n + i]);
+        const bool mine = lane < nw && rank == kk - 1 &&
+                          (B.nb[b] <= kprime || f2 * g < q.sq + T - eps);
+        ok = __any_sync(FULL, mine);
+        if (lane < nw && rank < kk) {
+          knn_idx[i * K + B.col0[b] + rank] = id;
+          knn_dist[i * K + B.col0[b] + rank] = __double2float_rn(sqrt(g));
+        }
+        __syncwarp();
+      }
+      if (lane == 0) {
+        if (ok) {
+          ++n_cert;
+        } else {
+          const int at = atomicAdd(nfail, 1);
+          fail_rows[at] = int32_t(i);
+          fail_bat[at] = b;
+        }
+      }
+    }
+  }
+  if (lane == 0 && n_cert)
+    atomicAdd(reinterpret_cast<unsigned long long*>(n_cert_out), (unsigned long long)n_cert);
+}
+
+// FP64 scan of the listed (cell, batch) pairs of a group
+__global__ void __launch_bounds__(BB_T)
+bb_group_scan_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ perm,
+                     const BbBatches B, const int32_t* __restrict__ rows,
+                     const int32_t* __restrict__ bats, const int32_t* __restrict__ nrows, int K,
+                     int32_t* __restrict__ knn_idx, float* __restrict__ knn_dist,
+                     int64_t* __restrict__ n_scanned) {
+  __shared__ __align__(16) float xs_all[BB_WARPS][MSC_MAX_D];
+  const int lane = lane_id(), wib = warp_id();
+  const int64_t count = *nrows;
+  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  int64_t done = 0;
+  for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w < count;
+       w += nwarps) {
+    const int b = bats[w];
+    bb_scan_row(X, d, rows[w], perm + B.poff[b], B.nb[b], B.kk[b], xs_all[wib],
+                knn_idx + int64_t(rows[w]) * K + B.col0[b],
+                knn_dist + int64_t(rows[w]) * K + B.col0[b]);
+    ++done;
+  }
+  if (lane == 0 && done)
+    atomicAdd(reinterpret_cast<unsigned long long*>(n_scanned), (unsigned long long)done);
+}
+
 // FP64 scan of batch b for the listed cells (every cell when rows == nullptr): the kk (<= 128)
 // nearest keys by (d², index) into columns [col0, col0 + kk)
 __global__ void __launch_bounds__(BB_T)
@@ -186,43 +452,15 @@ bb_scan_kernel(const float* __restrict__ X, int d, int64_t n, const int32_t* __r
                int64_t* __restrict__ n_scanned) {
   __shared__ __align__(16) float xs_all[BB_WARPS][MSC_MAX_D];
   const int lane = lane_id(), wib = warp_id();
-  float* xs = xs_all[wib];
   const int64_t count = rows ? int64_t(*nrows) : n;
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  const double INF = __longlong_as_double(0x7ff0000000000000ll);
   int64_t done = 0;
   for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w < count;
        w += nwarps) {
     const int64_t i = rows ? int64_t(rows[w]) : w;
-    for (int t = lane; t < d; t += 32) xs[t] = X[i * d + t];
-    __syncwarp();
-    WarpTop128 top;
-    top.init();
-    for (int64_t base = 0; base < nb; base += 32) {
-      const int64_t jj = base + lane;
-      double v = INF;
-      int vi = INT32_MAX;
-      if (jj < nb) {
-        const int32_t c = perm[poff + jj];
-        if (c >= 0) {
-          v = bb_d2_f64(xs, X + int64_t(c) * d, d);
-          vi = c;
-        }
-      }
-      top.offer(v, vi, kk);
-    }
-    int32_t* oi = knn_idx + i * K + col0;
-    float* od = knn_dist + i * K + col0;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int r = s * 32 + lane;
-      if (r < kk) {
-        oi[r] = top.ai[s] == INT32_MAX ? int32_t(i) : top.ai[s];
-        od[r] = __double2float_rn(sqrt(top.a[s]));
-      }
-    }
+    bb_scan_row(X, d, i, perm + poff, nb, kk, xs_all[wib], knn_idx + i * K + col0,
+                knn_dist + i * K + col0);
     ++done;
-    __syncwarp();
   }
   if (lane == 0 && done)
     atomicAdd(reinterpret_cast<unsigned long long*>(n_scanned), (unsigned long long)done);
@@ -345,13 +583,17 @@ __global__ void trim_count_kernel(const int64_t* __restrict__ indptr,
                                   const int32_t* __restrict__ indices,
                                   const float* __restrict__ data, int64_t n,
                                   const float* __restrict__ theta, int32_t* __restrict__ cnt) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x) {
+  // a warp per row: a thread per row read its row entry by entry, 0.31 ms for 7 M entries
+  const int lane = lane_id();
+  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t i = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; i < n; i += nwarps) {
     const float ti = theta[i];
+    const int64_t b = indptr[i + 1];
     int c = 0;
-    for (int64_t e = indptr[i]; e < indptr[i + 1]; ++e)
+    for (int64_t e = indptr[i] + lane; e < b; e += 32)
       c += trim_kept(data[e], ti, theta[indices[e]]) ? 1 : 0;
-    cnt[i] = c;
+    c = __reduce_add_sync(FULL, c);
+    if (lane == 0) cnt[i] = c;
   }
 }
 
@@ -397,6 +639,11 @@ int grid_for(int64_t units, int per_block) {
 
 // ---- host side ---------------------------------------------------------------------------------
 
+namespace {
+constexpr int64_t BB_ORDER_MIN = 32768;
+constexpr int BB_ORDER_LEAF = 256;
+}  // namespace
+
 BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int prec) {
   BbPlan P;
   P.n = n;
@@ -421,15 +668,33 @@ BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int pre
   P.kprime = 0;
   if (P.candidates) {
     // over-fetch: the certificate compares the kk-th neighbour with the k'-th candidate, a wide
-    // margin already at k' = 32 for the usual kk = 3 (the self path's k' = 48 is sized for the
-    // 15th neighbour); wider lists for larger kk
-    P.kprime = prec == PREC_BF16X3 ? std::min(64, std::max(32, P.kk_max + 9))
-                                   : std::min(64, std::max(32, P.kk_max + 16));
+    // margin already at k' = 24 for the usual kk = 3 (the self path's k' = 48 is sized for the
+    // 15th neighbour); wider lists for larger kk.  8 batches of 200,000 x 50: k' = 32 no cell
+    // uncertified, 14.3 ms; 24 none, 13.3 ms; 16 two to eleven of 1.6 M, each an FP64 scan
+    P.kprime = prec == PREC_BF16X3 ? std::min(64, std::max(24, P.kk_max + 9))
+                                   : std::min(64, std::max(24, P.kk_max + 16));
     P.L = op_layout(prec, d);
     P.cfg = tc_default_config(prec, d, P.kprime);
     if (P.cfg.pair || !tc_config_ok(P.cfg, P.L.kp, P.kprime)) P.candidates = false;
   }
   P.ntiles = ceil_div(n, QTILE);
+  // the ordered scan: lists the group re-rank takes, 256-key tiles, and enough cells that the order
+  // and the plan cost less than the tiles they save: 16,384 cells in 8 batches 2.17 ms plain, 2.21
+  // ordered; 30,000 in 4 batches 2.20 / 2.29; 60,000 in 8 8.0 / 4.9.  MSC_B200_BB_ORDER=<cells>
+  // moves the line (tests; 0: always, negative: never).
+  int64_t least = BB_ORDER_MIN;
+  if (const char* e = std::getenv("MSC_B200_BB_ORDER")) {
+    least = std::atoll(e);
+    if (least < 0) least = INT64_MAX;
+  }
+  P.words = prune_mask_words(std::max<int64_t>(P.max_nb, 1), 256);
+  P.npg = round_up(n, 256);
+  // candidate lists of a launch within 1 GB (and the batches its parameters hold)
+  P.group = int(std::min<int64_t>(std::min(nb, BB_GROUP),
+                                  std::max<int64_t>(1, (int64_t(1) << 28) /
+                                                           std::max<int64_t>(1, n * P.kprime))));
+  P.ordered = P.candidates && P.kprime <= 32 && P.cfg.bn == 256 && d <= MSC_MAX_D && n >= least &&
+              n >= 1024;
   return P;
 }
 
@@ -458,9 +723,19 @@ size_t bb_carve(const BbPlan& P, void* base, BbWs& w) {
     w.Aop = c.take<char>(size_t(round_up(P.n, QTILE)) * P.L.kp * el);
     w.Bop = c.take<char>(size_t(P.p1) * P.L.kp * el);
     w.qs = c.take<QStat>(P.npk);
-    w.items = c.take<WorkItem>(std::max<int64_t>(P.ntiles, 1));
-    w.cand_idx = c.take<int32_t>(size_t(P.n) * P.kprime);
-    w.cand_thr = c.take<float>(P.n);
+    const int lists = P.ordered ? P.group : 1;
+    w.items = c.take<WorkItem>(std::max<int64_t>(P.ntiles * lists, 1));
+    w.cand_idx = c.take<int32_t>(size_t(P.n) * P.kprime * lists);
+    w.cand_thr = c.take<float>(size_t(P.n) * lists);
+    if (P.ordered) {
+      w.gperm = c.take<int32_t>(P.npg);
+      w.order_bytes = order_workspace_bytes(P.npg, P.d, BB_ORDER_LEAF);
+      w.order_ws = c.take<char>(w.order_bytes);
+      w.pitems = c.take<WorkItem>(P.ntiles * lists);
+      w.pr = carve_query_prune(c, P.n, P.npk, P.p1, P.d, lists, P.ntiles * lists, P.words);
+      w.fail_rows = c.take<int32_t>(size_t(P.n) * lists);
+      w.fail_bat = c.take<int32_t>(size_t(P.n) * lists);
+    }
   } else {
     w.Aop = w.Bop = nullptr;
     w.qs = nullptr;
@@ -471,6 +746,113 @@ size_t bb_carve(const BbPlan& P, void* base, BbWs& w) {
   return c.bytes();
 }
 
+namespace {
+// one centring and one scale, the operands of both sides (perm, qmap in place)
+int bb_operands(const BbPlan& P, const BbWs& w, const float* X, cudaStream_t st) {
+  MSC_TRY(launch_single_segment(w.seg, P.n, st));
+  MSC_TRY(launch_colmean(X, w.seg, 1, P.n, P.d, w.partial, BB_COLMEAN_NB, w.mean,
+                         &w.ctl->stats[MSC_STAT_NONFINITE], st));
+  if (P.prec == PREC_FP16) MSC_TRY(launch_maxnorm(X, w.seg, 1, w.mean, P.d, P.n, w.ctl, st));
+  MSC_TRY(launch_pack_tc(P.prec, X, w.perm, w.seg, 1, w.mean, P.d, P.p1, nullptr, nullptr, 0,
+                         nullptr, w.Bop, w.qs, w.km, w.ctl, st));
+  // the query operand: every cell, listed through qmap (the listed-row count in ctl)
+  bb_set_i32_kernel<<<1, 1, 0, st>>>(&w.ctl->n_refine, int32_t(P.n));
+  MSC_LAUNCH_CHECK();
+  const size_t row = size_t(P.L.kp) * (P.prec == PREC_FP16 ? sizeof(__half) : sizeof(__nv_bfloat16));
+  const int64_t tail = round_up(P.n, QTILE) - P.n;        // the operand's rows past the last query
+  if (tail > 0)
+    MSC_CUDA_TRY(cudaMemsetAsync(static_cast<char*>(w.Aop) + size_t(P.n) * row, 0, tail * row, st));
+  return launch_pack_tc(P.prec, X, w.perm, w.seg, 1, w.mean, P.d, P.npk, w.qmap,
+                        &w.ctl->n_refine, P.n, w.Aop, nullptr, w.qs, nullptr, w.ctl, st);
+}
+
+int run_bbknn_ordered(const BbPlan& P, const BbWs& w, const float* X, const int32_t* codes,
+                      const int64_t* counts, int32_t* knn_idx, float* knn_dist,
+                      cudaStream_t st) {
+  const int g = grid_for(P.n, BB_T);
+  // all cells in locality order, cells of no dense region last
+  MSC_TRY(launch_single_segment(w.seg, P.n, st));
+  int levels = 4;
+  while ((int64_t(BB_ORDER_LEAF) << (levels - 4)) < P.n) ++levels;
+  MSC_TRY(launch_order(X, P.d, w.seg, 1, P.npg, levels, BB_ORDER_LEAF, w.gperm, w.pr.leaf,
+                       w.order_ws, w.order_bytes, st, P.n));
+  MSC_TRY(launch_order_outliers(X, P.d, w.seg, P.n, P.npg, w.gperm, w.pr.leaf, w.pr, st));
+  // layout: every batch's keys in that order, then the queries
+  int32_t* leaf = w.pr.leaf2;                             // by packed row
+  MSC_CUDA_TRY(cudaMemsetAsync(leaf, 0xFF, sizeof(int32_t) * P.npk, st));
+  int64_t poff = 0;
+  for (int b = 0; b < P.nb; ++b) {
+    bb_flag_order_kernel<<<g, BB_T, 0, st>>>(codes, w.gperm, P.n, b, w.flag);
+    MSC_LAUNCH_CHECK();
+    MSC_TRY(scan_excl_i32(w.flag, P.n, w.S, w.scan, st));
+    bb_place_order_kernel<<<g, BB_T, 0, st>>>(w.flag, w.gperm, w.pr.leaf, P.n, w.S, poff,
+                                              counts[b], w.perm, leaf);
+    MSC_LAUNCH_CHECK();
+    poff += round_up(std::max<int64_t>(counts[b], 1), SEG_PAD);
+  }
+  bb_query_order_kernel<<<g, BB_T, 0, st>>>(w.gperm, w.pr.leaf, P.n, P.p1, w.perm, leaf, w.qmap);
+  MSC_LAUNCH_CHECK();
+  MSC_TRY(bb_operands(P, w, X, st));
+  MSC_CUDA_TRY(cudaMemsetAsync(w.pr.rpos, 0, sizeof(double) * P.npk, st));
+  MSC_TRY(launch_query_balls(X, P.d, P.npk, P.p1, P.ntiles, w.perm, leaf, w.pr.rpos, w.pr, st));
+  const int64_t arows = round_up(P.n, QTILE);
+  const int gw = grid_for(P.n, BB_WARPS);
+  poff = 0;
+  int col0 = 0, b = 0;
+  while (b < P.nb) {
+    BbBatches B{};
+    int m = 0;
+    for (; b < P.nb && m < P.group; ++b) {
+      const int kk = int(std::min<int64_t>(P.kwb, counts[b]));
+      if (kk > 0) {
+        B.poff[m] = int32_t(poff);
+        B.nb[m] = int32_t(counts[b]);
+        B.kk[m] = kk;
+        B.col0[m] = col0;
+        ++m;
+      }
+      col0 += kk;
+      poff += round_up(std::max<int64_t>(counts[b], 1), SEG_PAD);
+    }
+    if (m == 0) continue;
+    const int64_t n_items = P.ntiles * m;
+    bb_group_items_kernel<<<grid_for(n_items, BB_T), BB_T, 0, st>>>(B, m, P.n, P.p1, w.items,
+                                                                   w.pitems);
+    MSC_LAUNCH_CHECK();
+    // near pass, radii, plan, main scan
+    MSC_TRY(launch_nearest_tiles(w.pitems, n_items, P.d, w.pr, P.words, st));
+    auto scan = [&](bool main_scan) {
+      int32_t* counter = &w.ctl->tc_counter[main_scan ? 0 : 2];
+      MSC_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int32_t), st));
+      return launch_knn_tc(P.prec, P.cfg, w.Aop, w.Bop, arows, P.p1, P.L.kp, P.L.kmma, w.items,
+                           n_items, w.perm, w.qmap, nullptr, counter, w.ctl, P.kprime, w.cand_idx,
+                           w.cand_thr, P.kprime * m, st, w.pr.mask, P.words, false, false,
+                           main_scan ? w.pr.seed : nullptr, nullptr, nullptr, nullptr,
+                           main_scan ? w.pr.claim : nullptr, 1, P.n);
+    };
+    MSC_TRY(scan(false));
+    MSC_TRY(launch_query_plan(P.d, w.perm, P.p1, P.n, m, w.pitems, n_items, w.cand_thr, w.qs,
+                              w.km, w.ctl, P.prec, P.L.kmma, w.pr, P.words, st));
+    MSC_TRY(launch_claim_order(n_items, P.words, w.pr, st));
+    MSC_TRY(scan(true));
+    MSC_CUDA_TRY(cudaMemsetAsync(w.nfail, 0, sizeof(int32_t), st));
+    bb_group_rerank_kernel<<<gw, BB_T, 0, st>>>(X, P.d, P.n, P.p1, w.perm, B, m, w.cand_idx,
+                                                w.cand_thr, P.kprime, w.qs, w.km, w.ctl, P.prec,
+                                                P.L.kmma, P.K, knn_idx, knn_dist, w.fail_rows,
+                                                w.fail_bat, w.nfail,
+                                                &w.ctl->stats[MSC_STAT_CERTIFIED]);
+    MSC_LAUNCH_CHECK();
+    bb_group_scan_kernel<<<gw, BB_T, 0, st>>>(X, P.d, w.perm, B, w.fail_rows, w.fail_bat, w.nfail,
+                                              P.K, knn_idx, knn_dist,
+                                              &w.ctl->stats[MSC_STAT_RESCANNED]);
+    MSC_LAUNCH_CHECK();
+  }
+  bb_merge_kernel<<<gw, BB_T, 0, st>>>(P.n, P.K, knn_idx, knn_dist);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+}  // namespace
+
 int run_bbknn(const BbPlan& P, const BbWs& w, const float* X, const int32_t* codes,
               const int64_t* counts, int32_t* knn_idx, float* knn_dist, cudaStream_t st) {
   MSC_CUDA_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), st));
@@ -478,6 +860,7 @@ int run_bbknn(const BbPlan& P, const BbWs& w, const float* X, const int32_t* cod
   MSC_CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(int32_t) * std::max(P.nb, 1), st));
   MSC_CUDA_TRY(cudaMemsetAsync(w.perm, 0xFF, sizeof(int32_t) * P.npk, st));
   const int g = grid_for(P.n, BB_T);
+  if (P.ordered) return run_bbknn_ordered(P, w, X, codes, counts, knn_idx, knn_dist, st);
   // layout: batch segments, then the query region
   int64_t poff = 0;
   for (int b = 0; b < P.nb; ++b) {
@@ -492,22 +875,7 @@ int run_bbknn(const BbPlan& P, const BbWs& w, const float* X, const int32_t* cod
   MSC_LAUNCH_CHECK();
   const int gw = grid_for(P.n, BB_WARPS);                 // one warp per cell
   if (P.candidates) {
-    // one centring and one scale for both sides
-    MSC_TRY(launch_single_segment(w.seg, P.n, st));
-    MSC_TRY(launch_colmean(X, w.seg, 1, P.n, P.d, w.partial, BB_COLMEAN_NB, w.mean,
-                           &w.ctl->stats[MSC_STAT_NONFINITE], st));
-    if (P.prec == PREC_FP16) MSC_TRY(launch_maxnorm(X, w.seg, 1, w.mean, P.d, P.n, w.ctl, st));
-    MSC_TRY(launch_pack_tc(P.prec, X, w.perm, w.seg, 1, w.mean, P.d, P.p1, nullptr, nullptr, 0,
-                           nullptr, w.Bop, w.qs, w.km, w.ctl, st));
-    // the query operand: every cell, listed through qmap (the listed-row count in ctl)
-    bb_set_i32_kernel<<<1, 1, 0, st>>>(&w.ctl->n_refine, int32_t(P.n));
-    MSC_LAUNCH_CHECK();
-    MSC_CUDA_TRY(cudaMemsetAsync(w.Aop, 0,
-                                 size_t(round_up(P.n, QTILE)) * P.L.kp *
-                                     (P.prec == PREC_FP16 ? sizeof(__half) : sizeof(__nv_bfloat16)),
-                                 st));
-    MSC_TRY(launch_pack_tc(P.prec, X, w.perm, w.seg, 1, w.mean, P.d, P.npk, w.qmap,
-                           &w.ctl->n_refine, P.n, w.Aop, nullptr, w.qs, nullptr, w.ctl, st));
+    MSC_TRY(bb_operands(P, w, X, st));
   }
   poff = 0;
   int col0 = 0;
@@ -586,7 +954,7 @@ int launch_trim(const int64_t* indptr, const int32_t* indices, const float* data
   int64_t* scan = c.take<int64_t>(scan_i32_scratch_elems(n));
   trim_theta_kernel<<<grid_for(n, BB_WARPS), BB_T, 0, st>>>(indptr, data, n, trim, theta);
   MSC_LAUNCH_CHECK();
-  trim_count_kernel<<<grid_for(n, BB_T), BB_T, 0, st>>>(indptr, indices, data, n, theta, cnt);
+  trim_count_kernel<<<grid_for(n, BB_WARPS), BB_T, 0, st>>>(indptr, indices, data, n, theta, cnt);
   MSC_LAUNCH_CHECK();
   MSC_TRY(scan_excl_i32(cnt, n, out_ptr, scan, st));
   trim_fill_kernel<<<grid_for(n, BB_WARPS), BB_T, 0, st>>>(indptr, indices, data, n, theta,

@@ -201,6 +201,27 @@ int launch_refine_merge(const WorkItem* items3, const int32_t* n_items3, const C
                         const PruneWs& w, int kprime, int32_t* cand_idx, float* cand_thr,
                         cudaStream_t st);
 constexpr int REFINE_SPLIT = 8;
+// Batch-balanced scans (bbknn.cu): the queries are a region of their own behind the keys, at packed
+// rows p1 .. p1 + n, items carry their batch in pad0 and queries as packed rows, and seeds, radii
+// and thresholds are per (batch, query).
+PruneWs carve_query_prune(Carver& c, int64_t n, int64_t npk, int64_t p1, int d, int nb,
+                          int64_t n_items, int words);
+// rows far from their tile's mean to the end of the order (perm and leaf rewritten)
+int launch_order_outliers(const float* X, int d, const SegDesc* seg, int64_t n, int64_t npacked,
+                          int32_t* perm, int32_t* leaf, const PruneWs& w, cudaStream_t st);
+// balls of the key tiles, the query tiles and the 32-row blocks of both (zeros: npk doubles read
+// as radii and not used)
+int launch_query_balls(const float* X, int d, int64_t npk, int64_t p1, int64_t nq,
+                       const int32_t* perm, const int32_t* leaf, const double* zeros,
+                       const PruneWs& w, cudaStream_t st);
+// masks of the near pass: every item's nearest key tile
+int launch_nearest_tiles(const WorkItem* items, int64_t n_items, int d, const PruneWs& w,
+                         int words, cudaStream_t st);
+// after the near pass: radii, seeds and the masks of the main scan
+int launch_query_plan(int d, const int32_t* perm, int64_t p1, int64_t n, int nb,
+                      const WorkItem* items, int64_t n_items, const float* cand_thr,
+                      const QStat* qs, const KeyMax* km, const Ctl* ctl, int prec, int kmma,
+                      const PruneWs& w, int words, cudaStream_t st);
 int prune_counters(unsigned long long* out);
 int prune_counters_clear();
 
@@ -371,6 +392,11 @@ struct BbPlan {
   int kprime;
   OpLayout L;
   TcConfig cfg;
+  // large inputs: cells in locality order, all batches (of a group) in one launch, key tiles pruned
+  bool ordered;
+  int group;          // batches per launch
+  int words;          // mask words per item
+  int64_t npg;        // rows of the global order (n padded to 256)
 };
 struct BbWs {
   Ctl* ctl;
@@ -392,6 +418,13 @@ struct BbWs {
   WorkItem* items;
   int32_t* cand_idx;
   float* cand_thr;
+  // ordered
+  int32_t* gperm;
+  void* order_ws;
+  size_t order_bytes;
+  WorkItem* pitems;   // the items with packed query rows
+  PruneWs pr;
+  int32_t* fail_bat;
 };
 BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int prec);
 size_t bb_carve(const BbPlan& P, void* base, BbWs& w);

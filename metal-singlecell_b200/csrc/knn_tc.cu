@@ -939,7 +939,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int nq = min(BM, w.nq - int(rank) * BM);   // this CTA's valid query rows (may be <= 0)
       const int qrow = w.qrow0 + int(rank) * BM;
       const int self = P.qmap ? (row < nq ? P.qmap[qrow + row] : -1) : qrow + row;
-      sel.set_seed((P.seed && row < nq) ? P.seed[qrow + row] : F_INF);
+      // pad0: the item's batch (batch-balanced scans), which has its own seeds and candidate slots
+      sel.set_seed((P.seed && row < nq) ? P.seed[w.pad0 * P.thr_stride + qrow + row] : F_INF);
       if (P.init_val) {
         // both column halves start from the near pass's lists (merge_from skips the copies)
         const int nv = min(32, nq - q * 32);
@@ -1101,7 +1102,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int wrow0 = q * 32;
       const int nvalid = min(32, nq - wrow0);
       auto write_out = [&]() {
-        const int sidx = S > 1 ? it % S : 0;
+        const int sidx = (S > 1 ? it % S : 0) + w.pad0;
         if (S > 1 && P.part)
           sel.finish_partial(P.part, P.part_thr, int64_t(it) * BM + wrow0, P.perm, nvalid,
                              P.kprime);

@@ -89,7 +89,8 @@ struct WorkItem {
   int32_t nkeys;      // valid keys of the sample (n_s)
   int32_t orig_off;   // original row of the sample's first cell
   int32_t qorig0;     // original row of the tile's first query (orig_off + qrow0 - key0)
-  int32_t pad0, pad1;
+  int32_t pad0;       // batch of a batch-balanced scan, else 0
+  int32_t pad1;
 };
 
 // per-row statistics of the query operand, for the certification bound

@@ -400,7 +400,7 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
             const float* __restrict__ kc, const float* __restrict__ kr,
             const float* __restrict__ sc, const float* __restrict__ sr,
             const double* __restrict__ rsub, int words, uint32_t* __restrict__ mask, int prof,
-            int max_pairs, int task_words) {
+            int max_pairs, int task_words, int near, int64_t rsub_stride) {
   extern __shared__ float4 sm4[];
   __shared__ unsigned ubits_all[PLAN_WARPS][32], wbits_all[PLAN_WARPS][32];
   // positions of set bits, written by the lanes that hold them: the failing tiles of a chunk, the
@@ -446,12 +446,14 @@ plan_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, int d, 
     __syncwarp();
     const float rq = qr[qt];
     // the reach of each 32-row block and of the whole tile
-    if (lane < 4) reach[lane] = ball_reach(rsub[sb0 + lane], f);  // rsub is >= 0 or +inf
+    if (lane < 4)                                          // rsub is >= 0 or +inf
+      reach[lane] = ball_reach(rsub[w.pad0 * rsub_stride + sb0 + lane], f);
     __syncwarp();
     const double reach_q = fmax(fmax(reach[0], reach[1]), fmax(reach[2], reach[3]));
     const int nkt = (w.nkeys + bn - 1) / bn;
     const int diag = (w.qrow0 - w.key0) / bn;
-    const int lo = max(0, diag - 2), hi = min(nkt - 1, diag + 2);
+    // near tiles, which the scan visits anyway (near < 0: none, the queries are not among the keys)
+    const int lo = max(0, diag - near), hi = min(nkt - 1, diag + near);
     uint32_t* out = mask + it * int64_t(words);
     const int wend = min(words, (wblk + 1) * task_words);
     for (int base = wblk * task_words * 32; base < wend * 32; base += 32) {
@@ -969,6 +971,243 @@ int prune_mask_words(int64_t max_seg, int bn) {
   return int(ceil_div(ceil_div(max_seg, bn), 32));
 }
 
+namespace {
+int plan_grid(int64_t n_items, int words, int& task_words) {
+  const int64_t want = int64_t(num_sms()) * 6 * PLAN_WARPS * PLAN_TASKS;
+  task_words = PLAN_WORDS_MAX;
+  while (task_words > 1 && n_items * ceil_div(words, task_words) < want) task_words >>= 1;
+  const int64_t ntasks = n_items * ceil_div(words, task_words);
+  return int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ntasks, PLAN_WARPS),
+                                                    int64_t(num_sms()) * 32)));
+}
+
+// ---- batch-balanced scans: queries in a region of their own behind the keys ----
+
+// squared distance of every row to the mean of its 128-row tile (rows of no dense region are far)
+__global__ void __launch_bounds__(PR_T)
+tile_spread_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ perm,
+                   int64_t ngroups, double* __restrict__ out) {
+  constexpr int W = PR_T / 32, R = QTILE / W;
+  __shared__ double part[W][MSC_MAX_D];
+  __shared__ float c[MSC_MAX_D];
+  __shared__ int cnts[W];
+  const int lane = lane_id(), wib = warp_id();
+  for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t p0 = g * QTILE + wib * R;
+    const int32_t my_i = lane < R ? perm[p0 + lane] : -1;
+    double s[4] = {0, 0, 0, 0};
+#pragma unroll 4
+    for (int r = 0; r < R; ++r) {
+      const int32_t i = __shfl_sync(FULL, my_i, r);
+      if (i < 0) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (lane + 32 * j < d) s[j] += X[int64_t(i) * d + lane + 32 * j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (lane + 32 * j < d) part[wib][lane + 32 * j] = s[j];
+    const unsigned have = __ballot_sync(FULL, my_i >= 0);
+    if (lane == 0) cnts[wib] = __popc(have);
+    __syncthreads();
+    int cnt = 0;
+    for (int w = 0; w < W; ++w) cnt += cnts[w];
+    for (int t = threadIdx.x; t < d; t += PR_T) {
+      double a = 0.0;
+      for (int w = 0; w < W; ++w) a += part[w][t];
+      c[t] = cnt ? float(a / cnt) : 0.f;
+    }
+    __syncthreads();
+    for (int r = 0; r < R; r += 4) {
+      const int rr = r + (lane >> 3);
+      const int32_t i = __shfl_sync(FULL, my_i, rr);
+      const double a = row_d2_8(X + int64_t(i < 0 ? 0 : i) * d, c, d, lane & 7);
+      if ((lane & 7) == 0)
+        out[p0 + rr] = i >= 0 ? a : __longlong_as_double(0x7ff8000000000000ll);
+    }
+  }
+}
+
+// stable partition of one sample: flagged rows first, then the others (leaf OUTLIER_LEAF)
+__global__ void flag_partition_kernel(const int32_t* __restrict__ perm,
+                                      const int32_t* __restrict__ leaf, int64_t n, int64_t npacked,
+                                      const int32_t* __restrict__ reg,
+                                      const int64_t* __restrict__ S, int32_t* __restrict__ perm2,
+                                      int32_t* __restrict__ leaf2) {
+  for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < npacked;
+       p += int64_t(gridDim.x) * blockDim.x) {
+    const bool row = p < n;
+    const int64_t pos = !row ? p : (reg[p] ? S[p] : S[n] + p - S[p]);
+    perm2[pos] = perm[p];
+    leaf2[pos] = row && !reg[p] ? OUTLIER_LEAF : leaf[p];
+  }
+}
+
+// one bit per (query tile, batch) item: the batch's key tile whose ball centre is nearest
+__global__ void nearest_tile_kernel(const WorkItem* __restrict__ items, int64_t n_items, int n4,
+                                    const float* __restrict__ qc, const float* __restrict__ kc,
+                                    const float* __restrict__ kr, int words,
+                                    uint32_t* __restrict__ mask) {
+  const int lane = lane_id();
+  const float4* kc4 = reinterpret_cast<const float4*>(kc);
+  const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t it = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; it < n_items;
+       it += warps) {
+    const WorkItem w = items[it];
+    const float4* q = reinterpret_cast<const float4*>(qc) + (w.qrow0 / QTILE) * int64_t(n4);
+    const int nkt = (w.nkeys + 255) / 256;
+    float best = F_INF;
+    int at = 0;
+    for (int kt = lane; kt < nkt; kt += 32) {
+      const int64_t g = w.key0 / 256 + kt;
+      if (kr[g] < 0.f) continue;
+      const float d2 = ball_d2<1, INTER>(q, kc4 + inter_at(g, n4), n4);
+      if (d2 < best) { best = d2; at = kt; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float od = __shfl_xor_sync(FULL, best, o);
+      const int ok = __shfl_xor_sync(FULL, at, o);
+      if (od < best || (od == best && ok < at)) { best = od; at = ok; }
+    }
+    for (int wi = lane; wi < words; wi += 32)
+      mask[it * words + wi] = wi == (at >> 5) ? 1u << (at & 31) : 0u;
+  }
+}
+
+// after the near pass: every (query, batch)'s radius R as in row_radius_kernel, its seed as in
+// partition_kernel, and the largest R of each 32-row block of queries
+__global__ void __launch_bounds__(PR_T)
+query_radius_kernel(const int32_t* __restrict__ perm, int64_t p1, int64_t n, int nb,
+                    const float* __restrict__ cand_thr, const QStat* __restrict__ qs,
+                    const KeyMax* __restrict__ km, int prec, int kmma, int d, int64_t nqblk,
+                    float* __restrict__ seed, double* __restrict__ rsub) {
+  const int lane = lane_id();
+  const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t x = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; x < nqblk * nb;
+       x += warps) {
+    const int64_t b = x / nqblk, blk = x - b * nqblk, j = blk * 32 + lane;
+    double r = 0.0;
+    if (j < n) {
+      const double thr = cand_thr[b * n + perm[p1 + j]];
+      const QStat q = qs[p1 + j];
+      const double eps = cert_eps(q, *km, prec, kmma, d);
+      r = thr + q.sq + 3.0 * eps;
+      if (!(r < 1e300)) r = __longlong_as_double(0x7ff0000000000000ll);
+      const double t = thr + 2.0 * eps;
+      seed[b * n + j] = t < 1e300 ? nextafterf(__double2float_ru(t), F_INF) : F_INF;
+    }
+    r = warp_max_d(r);
+    if (lane == 0) rsub[b * nqblk + blk] = r;
+  }
+}
+}  // namespace
+
+int launch_order_outliers(const float* X, int d, const SegDesc* seg, int64_t n, int64_t npacked,
+                          int32_t* perm, int32_t* leaf, const PruneWs& w, cudaStream_t st) {
+  const int64_t ng = npacked / QTILE;
+  const int grid = grid_for(npacked);
+  tile_spread_kernel<<<int(std::min<int64_t>(ng, int64_t(num_sms()) * 32)), PR_T, 0, st>>>(
+      X, d, perm, ng, w.rpos);
+  MSC_LAUNCH_CHECK();
+  sample_mean_partial_kernel<<<dim3(MEAN_CHUNKS, 1), PR_T, 0, st>>>(seg, 1, w.rpos, w.mean_part);
+  MSC_LAUNCH_CHECK();
+  sample_mean_final_kernel<<<1, 128, 0, st>>>(w.mean_part, 1, w.mean);
+  MSC_LAUNCH_CHECK();
+  regular_flag_kernel<<<grid, PR_T, 0, st>>>(perm, npacked, seg, 1, w.rpos, w.mean,
+                                             OUTLIER_FACTOR, w.reg);
+  MSC_LAUNCH_CHECK();
+  MSC_TRY(scan_excl_i32(w.reg, n, w.S, w.scan_scratch, st));
+  flag_partition_kernel<<<grid, PR_T, 0, st>>>(perm, leaf, n, npacked, w.reg, w.S, w.perm2,
+                                               w.leaf2);
+  MSC_LAUNCH_CHECK();
+  MSC_CUDA_TRY(cudaMemcpyAsync(perm, w.perm2, sizeof(int32_t) * npacked, cudaMemcpyDeviceToDevice,
+                               st));
+  MSC_CUDA_TRY(cudaMemcpyAsync(leaf, w.leaf2, sizeof(int32_t) * npacked, cudaMemcpyDeviceToDevice,
+                               st));
+  return MSC_OK;
+}
+
+int launch_query_balls(const float* X, int d, int64_t npk, int64_t p1, int64_t nq,
+                       const int32_t* perm, const int32_t* leaf, const double* zeros,
+                       const PruneWs& w, cudaStream_t st) {
+  const int dp = int(round_up(d, 4));
+  const int64_t most = int64_t(num_sms()) * 32, nk = p1 / 256, ns = npk / SUB;
+  group_ball_kernel<QTILE, false><<<int(std::min(nq, most)), PR_T, 0, st>>>(
+      X, d, dp, perm + p1, nq, w.qc + (p1 / QTILE) * dp, w.qr + p1 / QTILE);
+  MSC_LAUNCH_CHECK();
+  group_ball_kernel<256, true><<<int(std::min(nk, most)), PR_T, 0, st>>>(X, d, dp, perm, nk, w.kc,
+                                                                         w.kr);
+  MSC_LAUNCH_CHECK();
+  const int sgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ns, 8), num_sms() * 16)));
+  sub_ball_kernel<<<sgrid, PR_T, 0, st>>>(X, d, dp, perm, leaf, zeros, ns, w.sc, w.sr, w.rsub);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+int launch_nearest_tiles(const WorkItem* items, int64_t n_items, int d, const PruneWs& w,
+                         int words, cudaStream_t st) {
+  const int dp = int(round_up(d, 4));
+  const int grid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(n_items, 8),
+                                                             int64_t(num_sms()) * 16)));
+  nearest_tile_kernel<<<grid, PR_T, 0, st>>>(items, n_items, dp / 4, w.qc, w.kc, w.kr, words,
+                                             w.mask);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+int launch_query_plan(int d, const int32_t* perm, int64_t p1, int64_t n, int nb,
+                      const WorkItem* items, int64_t n_items, const float* cand_thr,
+                      const QStat* qs, const KeyMax* km, const Ctl* ctl, int prec, int kmma,
+                      const PruneWs& w, int words, cudaStream_t st) {
+  const int64_t nqblk = ceil_div(n, QTILE) * (QTILE / SUB);
+  const int qgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(nqblk * nb, 8),
+                                                              int64_t(num_sms()) * 16)));
+  query_radius_kernel<<<qgrid, PR_T, 0, st>>>(perm, p1, n, nb, cand_thr, qs, km, prec, kmma, d,
+                                              nqblk, w.seed, w.rsub);
+  MSC_LAUNCH_CHECK();
+  const int dp = int(round_up(d, 4));
+  const size_t smem = size_t(PLAN_WARPS) * 9 * dp * sizeof(float);
+  int task_words;
+  const int pgrid = plan_grid(n_items, words, task_words);
+  // the plan indexes R by packed 32-row block: the queries' first block is p1 / 32
+  plan_kernel<<<pgrid, PLAN_WARPS * 32, smem, st>>>(
+      items, n_items, 256, d, dp, ctl, prec, w.qc, w.qr, w.kc, w.kr, w.sc, w.sr,
+      w.rsub - p1 / SUB, words, w.mask, 0, PLAN_MAX_PAIRS, task_words, -1, nqblk);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+PruneWs carve_query_prune(Carver& c, int64_t n, int64_t npk, int64_t p1, int d, int nb,
+                          int64_t n_items, int words) {
+  PruneWs w{};
+  const int64_t npg = round_up(n, 256);
+  w.leaf = c.take<int32_t>(npg);
+  w.leaf2 = c.take<int32_t>(npk);
+  w.perm2 = c.take<int32_t>(npg);
+  w.reg = c.take<int32_t>(npg);
+  w.S = c.take<int64_t>(npg + 1);
+  w.scan_scratch = c.take<int64_t>(scan_i32_scratch_elems(npg));
+  w.rpos = c.take<double>(std::max(npg, npk));
+  w.mean = c.take<double>(1);
+  w.mean_part = c.take<double2>(MEAN_CHUNKS);
+  const int dp = int(round_up(d, 4));
+  w.qc = c.take<float>(size_t(npk / QTILE + 1) * dp);
+  w.qr = c.take<float>(npk / QTILE + 1);
+  w.kc = c.take<float>(size_t(round_up(p1 / 256, 32)) * dp);
+  w.kr = c.take<float>(p1 / 256);
+  w.sc = c.take<float>(size_t(round_up(2 * npk / SUB, 32)) * dp);
+  w.sr = c.take<float>(2 * npk / SUB);
+  const int64_t nqblk = ceil_div(n, QTILE) * (QTILE / SUB);
+  w.rsub = c.take<double>(std::max(npk / SUB, nqblk * nb));
+  w.seed = c.take<float>(size_t(n) * nb);
+  w.mask = c.take<uint32_t>(size_t(n_items) * words);
+  w.vcnt = c.take<int32_t>(n_items);
+  w.claim = c.take<int32_t>(n_items);
+  w.chist = c.take<int32_t>(COST_BUCKETS);
+  return w;
+}
+
 PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items, int words,
                     int64_t n, int kprime) {
   PruneWs w{};
@@ -1082,16 +1321,12 @@ int launch_prune_plan(const float* X, int d, int64_t npacked, const int32_t* per
   const size_t smem = size_t(PLAN_WARPS) * 9 * dp * sizeof(float);
   int max_pairs = PLAN_MAX_PAIRS;
   if (const char* env = std::getenv("MSC_B200_PLAN_PAIRS")) max_pairs = std::max(0, std::atoi(env));
-  const int64_t want = int64_t(num_sms()) * 6 * PLAN_WARPS * PLAN_TASKS;
-  int task_words = PLAN_WORDS_MAX;
-  while (task_words > 1 && n_items * ceil_div(words, task_words) < want) task_words >>= 1;
-  const int64_t ntasks = n_items * ceil_div(words, task_words);
-  const int pgrid = int(std::max<int64_t>(1, std::min<int64_t>(ceil_div(ntasks, PLAN_WARPS),
-                                                              int64_t(num_sms()) * 32)));
+  int task_words;
+  const int pgrid = plan_grid(n_items, words, task_words);
   plan_kernel<<<pgrid, PLAN_WARPS * 32, smem, st>>>(items, n_items, bn, d, dp, ctl, prec, w.qc,
                                                     w.qr, w.kc, w.kr, w.sc, w.sr, w.rsub, words,
                                                     w.mask, profiling_enabled() ? 1 : 0,
-                                                    max_pairs, task_words);
+                                                    max_pairs, task_words, 2, 0);
   MSC_LAUNCH_CHECK();
   // point test of the kept pairs, opt-in (MSC_B200_POINT_TEST=1).  Measured at 1.3M × 50: far
   // tiles kept 2.63 M → 1.63 M and main scan 33.4 → 28.0 ms, but the test itself costs ~15 ms
