@@ -29,11 +29,30 @@ namespace {
 
 constexpr int RR_WARPS = 8;
 
-__device__ __forceinline__ double d2_f64(const float* xs, const float* __restrict__ y, int d) {
+// FP64 squared distance, summed in dimension order.  The lines that the loads touch in L1 bound the
+// re-rank (70 % of its wavefronts), and here a load touches a line per lane, so pairs (d even, rows
+// 8-byte aligned) halve them: graphs of 200,000 x 50 9.03 -> 8.88 ms, of 64 samples 14.0 -> 13.8.
+// Staging the rows in shared memory touches fewer lines but costs L1 its space: 9.15 ms; half a
+// warp a row in the FP32 pass: 8.88 and 13.7, but 63.4 ms for 1.3 M cells instead of 63.2.
+__device__ __forceinline__ double d2_f64(const float* xs, const float* __restrict__ y, int d,
+                                         bool pairs) {
   double acc = 0.0;
-  for (int t = 0; t < d; ++t) {
-    double df = double(xs[t]) - double(y[t]);
-    acc += df * df;
+  if (pairs) {
+    const float2* y2 = reinterpret_cast<const float2*>(y);
+    const float2* x2 = reinterpret_cast<const float2*>(xs);
+#pragma unroll 5
+    for (int t = 0; t < d >> 1; ++t) {
+      const float2 u = y2[t], p = x2[t];
+      const double e0 = double(p.x) - double(u.x);
+      acc += e0 * e0;
+      const double e1 = double(p.y) - double(u.y);
+      acc += e1 * e1;
+    }
+  } else {
+    for (int t = 0; t < d; ++t) {
+      double df = double(xs[t]) - double(y[t]);
+      acc += df * df;
+    }
   }
   return acc;
 }
@@ -102,6 +121,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
   const int lane = lane_id(), wib = warp_id();
   float* xs = xs_all[wib];
   const int kk = k - 1;
+  const bool pairs = (d & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 7) == 0;
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   // key-side maxima and the scale
   const KeyMax kmv = *km;
@@ -172,7 +192,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
         if (w1) wsc[__popc(b0) + __popc(b1 & lt)] = c1;
         __syncwarp();
         int cw = lane < m ? wsc[lane] : INT32_MAX;
-        double gw = lane < m ? d2_f64(xs, X + int64_t(cw) * d, d) : INF;
+        double gw = lane < m ? d2_f64(xs, X + int64_t(cw) * d, d, pairs) : INF;
         __syncwarp();                                    // wsc is read before the next row
         warp_sort32_d(gw, cw);
         g0 = gw; h0 = cw;
@@ -190,8 +210,8 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
       const double lim = double(B) * (1.0 + 3.0 * delta) + 1e-300;
       const bool w0 = i0 != INT32_MAX && double(se0) <= lim;
       const bool w1 = i1 != INT32_MAX && double(se1) <= lim;
-      g0 = w0 ? d2_f64(xs, X + int64_t(i0) * d, d) : INF;
-      g1 = w1 ? d2_f64(xs, X + int64_t(i1) * d, d) : INF;
+      g0 = w0 ? d2_f64(xs, X + int64_t(i0) * d, d, pairs) : INF;
+      g1 = w1 ? d2_f64(xs, X + int64_t(i1) * d, d, pairs) : INF;
       m = __popc(__ballot_sync(FULL, w0)) + __popc(__ballot_sync(FULL, w1));
       h0 = i0; h1 = i1;
       warp_sort64_d(g0, h0, g1, h1);
