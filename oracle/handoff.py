@@ -28,8 +28,7 @@ def umap_edges(conn: sp.csr_matrix, n_epochs: int) -> dict:
     thr = np.float32(wmax / np.float32(max(n_epochs, 1)))
     keep = data >= thr
     rows = np.repeat(np.arange(n, dtype=np.int32), np.diff(C.indptr))[keep]
-    kept_per_row = np.add.reduceat(keep.astype(np.int64), C.indptr[:-1]) if n else np.zeros(0)
-    kept_per_row = np.where(np.diff(C.indptr) > 0, kept_per_row, 0)
+    kept_per_row = np.bincount(rows, minlength=n)     # (reduceat refuses empty rows at the end)
     indptr = np.concatenate([[0], np.cumsum(kept_per_row)]).astype(np.int64)
     w = data[keep]
     w64 = w.astype(np.float64)
