@@ -17,8 +17,8 @@
 // chains of loads of a warp that takes one row of some twenty entries at a time.  Here a block
 // takes EB_ROWS rows' entries as one flat range, so all lanes load and every load is coalesced; an
 // entry finds its row by a search of the block's row pointers in shared memory.  200,000 rows of
-// 22 entries, a warp per row / this: counting and scanning 33 / 17 us, compacting 63 / 41 (now bound by
-// instructions: the two FP64 divisions and the search take half of them).
+// 22 entries, a warp per row / this: counting and scanning 33 / 17 us, compacting 63 / 41.  The
+// compaction is now bound by its instructions, above all the two FP64 divisions and the search.
 #include "kernels.cuh"
 
 namespace msc {
