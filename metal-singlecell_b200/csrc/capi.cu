@@ -590,12 +590,24 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
       }
       stage_mark(st, 3);
       const VisitOrder order{w.pr.vlist, w.pr.voff, w.pr.roff, &w.ctl->ordered_ok};
+      // with a claim order: the long items in parts
+      const bool parts = claim && !ordered && n_items < LONG_FLAG / LONG_SPLIT;
+      const LongSplit lg{w.pr.claim, w.pr.part, w.pr.part_thr, std::min(P.kprime, 32)};
+      if (parts) {
+        MSC_TRY(launch_long_plan(n_items, words, cfg.ctas * num_sms(), w.pr, w.ctl, st));
+        claim = w.pr.claim2;
+      }
       MSC_TRY(launch_knn_tc(P.prec, cfg, w.Aop, w.Bop, P.npacked, P.npacked, P.L.kp, P.L.kmma,
-                            w.items, n_items, w.perm, nullptr, nullptr, &w.ctl->tc_counter[0],
+                            w.items, n_items, w.perm, nullptr,
+                            parts ? &w.ctl->n_items_main : nullptr, &w.ctl->tc_counter[0],
                             w.ctl, kscan, w.cand_idx, w.cand_thr, P.kprime, st, mask, words,
                             false, prune && P.nseg == 1, prune ? w.pr.seed : nullptr,
                             prune ? &init : nullptr, nullptr,
-                            ordered ? &order : nullptr, claim, split, P.n));
+                            ordered ? &order : nullptr, claim, split, P.n,
+                            parts ? &lg : nullptr));
+      if (parts)
+        MSC_TRY(launch_long_merge(w.items, w.ctl, w.perm, w.pr, P.kprime, lg.kper, w.cand_idx,
+                                  w.cand_thr, st));
     }
   }
   stage_mark(st, 4);

@@ -164,6 +164,7 @@ struct PruneWs {
   unsigned long long* vlist;
   int64_t vcap;       // entries vlist holds
   int32_t* claim;      // main-scan claim order of the work items (costliest first)
+  int32_t* claim2;     // the same with the long items in parts (LongSplit)
   int32_t* chist;      // its bucket counts / offsets
 };
 int prune_mask_words(int64_t max_seg, int bn);
@@ -201,6 +202,22 @@ int launch_refine_merge(const WorkItem* items3, const int32_t* n_items3, const C
                         const PruneWs& w, int kprime, int32_t* cand_idx, float* cand_thr,
                         cudaStream_t st);
 constexpr int REFINE_SPLIT = 8;
+// The main scan's longest work items, scanned in parts (prune.cu): a claim entry LONG_FLAG | (r·
+// LONG_SPLIT + s) is part s of item order[r], every LONG_SPLIT-th tile that the item visits from
+// the s-th on, its rows' kper best below their seeds written to part / part_thr at that number.
+constexpr int LONG_SPLIT = REFINE_SPLIT;      // they share the refine pass's buffers
+constexpr int LONG_FLAG = 1 << 30;
+struct LongSplit {
+  const int32_t* order;
+  int2* part;
+  float* part_thr;
+  int kper;
+};
+int launch_long_plan(int64_t n_items, int words, int n_ctas, const PruneWs& w, Ctl* ctl,
+                     cudaStream_t st);
+int launch_long_merge(const WorkItem* items, const Ctl* ctl, const int32_t* perm,
+                      const PruneWs& w, int kprime, int kper, int32_t* cand_idx,
+                      float* cand_thr, cudaStream_t st);
 // Batch-balanced scans (bbknn.cu): the queries are a region of their own behind the keys, at packed
 // rows p1 .. p1 + n, items carry their batch in pad0 and queries as packed rows, and seeds, radii
 // and thresholds are per (batch, query).
@@ -304,7 +321,8 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
                   bool reverse = false, const float* seed = nullptr,
                   const NearInit* init = nullptr, const RefineSplit* split = nullptr,
                   const VisitOrder* order = nullptr, const int32_t* claim = nullptr,
-                  int split_host = 1, int64_t thr_stride = 0);
+                  int split_host = 1, int64_t thr_stride = 0,
+                  const LongSplit* lg = nullptr);
 
 // ---- rerank.cu ----
 int launch_rerank(const float* X, int d, const int32_t* perm, const SegDesc* seg, int nseg,

@@ -365,6 +365,9 @@ struct TcParams {
   // candidates at column r·k' of the row and its threshold to cand_thr[r·thr_stride + row]
   int split_host;
   int64_t thr_stride;
+  // the main scan's long items in parts (LongSplit), long_kper 0: none
+  const int32_t* long_order;
+  int long_kper;
   float* cand_val;              // near pass: also write the values of the kept candidates
   // main pass after a near pass: load every row's list from the near pass's candidates (values,
   // original rows -> packed positions through iperm) and never offer its keys again (excl)
@@ -416,6 +419,7 @@ struct KeyTileWalk {
   bool near_only;
   int khi = 1 << 30;     // range walks stop before this tile
   bool range = false;
+  int skip = 0, step = 1;    // every step-th tile, after the first skip
   __device__ __forceinline__ void init(const WorkItem& item, int qref, int bn,
                                        const uint32_t* m, int words, bool near) {
     nkt = (item.nkeys + bn - 1) / bn;
@@ -433,8 +437,8 @@ struct KeyTileWalk {
     cur = m ? m[0] : 0u;
     nxt = (m && words > 1) ? m[1] : 0u;     // one word ahead: its load overlaps the near tiles
   }
-  // A range walk (the refine pass): no near phase, only the tiles [lo, hi), in plain order or
-  // as the mask's bits.
+  // A range walk (the refine pass, the full scan's key ranges): no near phase, only the tiles
+  // [lo, hi), in plain order or as the mask's bits.
   __device__ __forceinline__ void set_range(int lo, int hi) {
     range = true;
     np = 0;
@@ -446,8 +450,19 @@ struct KeyTileWalk {
       nxt = w + 1 < nw ? mask[w + 1] : 0u;
     }
   }
+  // one part of the walk: its s-th tile and every S-th from there
+  __device__ __forceinline__ void set_every(int s, int S) {
+    skip = s;
+    step = S;
+  }
   // the next key tile, or -1
   __device__ __forceinline__ int next() {
+    for (; skip > 0; --skip)
+      if (next_tile() < 0) return -1;
+    skip = step - 1;
+    return next_tile();
+  }
+  __device__ __forceinline__ int next_tile() {
     if (j < np) return key_tile_at(j++, diag, nkt);
     if (near_only) return -1;
     if (!mask) {
@@ -637,7 +652,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   };
   // Items split over key ranges: work item it = (query tile it / S, range it % S).
   const int S = P.split_dev ? max(1, *P.split_dev) : P.split_host;
-  auto item_of = [&](int it) { return S > 1 ? it / S : it; };
+  auto item_of = [&](int it) {
+    if (P.long_kper && (it & LONG_FLAG)) return P.long_order[(it ^ LONG_FLAG) / LONG_SPLIT];
+    return S > 1 ? it / S : it;
+  };
   auto walk_init = [&](KeyTileWalk& walk, const WorkItem& w, int it) {
     const int r = item_of(it);
     walk.init(w, P.qmap ? P.qmap[w.qrow0] : w.qrow0, P.bn,
@@ -647,6 +665,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int sidx = S > 1 ? it % S : 0;
       const int chunk = (walk.nkt + S - 1) / S;
       walk.set_range(sidx * chunk, min(walk.nkt, (sidx + 1) * chunk));
+    } else if (P.long_kper && (it & LONG_FLAG)) {
+      walk.set_every((it ^ LONG_FLAG) % LONG_SPLIT, LONG_SPLIT);
     }
   };
   // consumers: the next published item, by one thread or by a whole warp (warp_wide)
@@ -939,12 +959,18 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int nq = min(BM, w.nq - int(rank) * BM);   // this CTA's valid query rows (may be <= 0)
       const int qrow = w.qrow0 + int(rank) * BM;
       const int self = P.qmap ? (row < nq ? P.qmap[qrow + row] : -1) : qrow + row;
+      const bool lpart = P.long_kper && (it & LONG_FLAG);     // a part of a long item
+      const int kp = lpart ? P.long_kper : P.kprime;
+      if (kp != sel.kp) {
+        sel.kp = kp;
+        sel.reset();
+      }
       // pad0: the item's batch (batch-balanced scans), which has its own seeds and candidate slots
       sel.set_seed((P.seed && row < nq) ? P.seed[w.pad0 * P.thr_stride + qrow + row] : F_INF);
       if (P.init_val) {
         // both column halves start from the near pass's lists (merge_from skips the copies)
         const int nv = min(32, nq - q * 32);
-        if (nv > 0)
+        if (nv > 0 && !lpart)
           sel.load_warp(P.init_val, P.init_idx, P.iperm, P.perm, int64_t(qrow) + q * 32, nv,
                         P.cand_stride);
         if (row < nq) {
@@ -1103,7 +1129,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int nvalid = min(32, nq - wrow0);
       auto write_out = [&]() {
         const int sidx = (S > 1 ? it % S : 0) + w.pad0;
-        if (S > 1 && P.part)
+        if (lpart)
+          sel.finish_partial(P.part, P.part_thr, int64_t(it ^ LONG_FLAG) * BM + wrow0, P.perm,
+                             nvalid, P.kprime);
+        else if (S > 1 && P.part)
           sel.finish_partial(P.part, P.part_thr, int64_t(it) * BM + wrow0, P.perm, nvalid,
                              P.kprime);
         else
@@ -1398,7 +1427,7 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
                   const uint32_t* mask, int mask_words, bool near_only, bool reverse,
                   const float* seed, const NearInit* init, const RefineSplit* split,
                   const VisitOrder* order, const int32_t* claim, int split_host,
-                  int64_t thr_stride) {
+                  int64_t thr_stride, const LongSplit* lg) {
   const int prof_slot = near_only ? 0 : (qmap ? 2 : 1);
   if (!tc_config_ok(cfg, kp, kprime)) {
     set_error("tensor-core tile config (bn=%d stages=%d kpl=%d cb=%d epi=%d pair=%d) does not fit",
@@ -1436,8 +1465,10 @@ int launch_knn_tc(int prec, const TcConfig& cfg, const void* Aop, const void* Bo
   P.seed = seed;
   P.prof_slot = prof_slot;
   P.split_dev = split ? split->split_dev : nullptr;
-  P.part = split ? split->part : nullptr;
-  P.part_thr = split ? split->part_thr : nullptr;
+  P.part = split ? split->part : lg ? lg->part : nullptr;
+  P.part_thr = split ? split->part_thr : lg ? lg->part_thr : nullptr;
+  P.long_order = lg ? lg->order : nullptr;
+  P.long_kper = lg ? lg->kper : 0;
   P.cand_val = init && near_only ? init->val : nullptr;
   const bool load = init && !near_only;
   P.init_val = load ? init->val : nullptr;

@@ -122,7 +122,8 @@ struct Ctl {
   int32_t refine_split;     // work items per refine item (key ranges), 1 = not split
   int32_t n_items_refine_eff;   // n_items_refine × refine_split
   int32_t ordered_ok;           // 1: every work item's sorted visit list fits (prune.cu)
-  int32_t pad2[2];
+  int32_t n_long;               // work items of the main scan that are scanned in parts
+  int32_t n_items_main;         // claims of the main scan: a long item counts LONG_SPLIT times
 };
 
 // ------------------------------------------------------------------------------------------------

@@ -839,6 +839,115 @@ __global__ void cost_scatter_kernel(const int32_t* __restrict__ cnt, int64_t n_i
   }
 }
 
+// The long items (a tile of outliers visits most key tiles and inserts into every row at other
+// times than its neighbours) would each keep one CTA busy after the others have run out of items.
+// Those whose cost is above LONG_SHARE of a CTA's share of all are scanned in LONG_SPLIT parts by
+// different CTAs, and their lists merged.  100,000 cells: twenty tiles took 2.0 to 2.6 ms each
+// where the CTAs' mean was 0.94; graph 6.0 -> 4.9 ms, of 200,000 cells 8.9 -> 8.2.  Parts insert
+// more than the whole item, so only what would outlast a mean CTA is split: at shares of 0.5 and
+// 0.25 100,000 cells take 5.2 and 5.6 ms, 1.3 M 63 and 73 (1.0: 63).  The parts' lists hold 32 of
+// k' = 48: with 24 the 200,000 cells take 8.5 ms (more rows left to the refine pass), with 48 the
+// 100,000 take 0.2 ms more.
+constexpr double LONG_SHARE = 1.0;
+constexpr int LONG_NEAR = 5;          // near tiles an item scans besides
+constexpr int LONG_T = 1024;
+__global__ void __launch_bounds__(LONG_T)
+long_plan_kernel(const int32_t* __restrict__ cnt, int64_t n_items, int shift, int n_ctas,
+                 int max_long, const int32_t* __restrict__ order, int32_t* __restrict__ claim,
+                 Ctl* __restrict__ ctl) {
+  __shared__ unsigned long long total;
+  __shared__ int n_long;
+  if (threadIdx.x == 0) { total = 0; n_long = 0; }
+  __syncthreads();
+  unsigned long long t = 0;
+  for (int64_t i = threadIdx.x; i < n_items; i += LONG_T) t += cnt[i] + LONG_NEAR;
+  atomicAdd(&total, t);
+  __syncthreads();
+  // whole buckets of the claim order, so that the long items are its first ones
+  const double cut = double(total) / n_ctas * LONG_SHARE;
+  const int bucket = int(fmin(cut, 1e9)) >> shift;
+  int m = 0;
+  for (int64_t i = threadIdx.x; i < n_items; i += LONG_T)
+    m += min(COST_BUCKETS - 1, cnt[i] >> shift) > bucket ? 1 : 0;
+  atomicAdd(&n_long, m);
+  __syncthreads();
+  const int64_t n = min(n_long, max_long), parts = n * LONG_SPLIT;
+  for (int64_t j = threadIdx.x; j < n_items - n + parts; j += LONG_T)
+    claim[j] = j < parts ? LONG_FLAG | int32_t(j) : order[j - parts + n];
+  if (threadIdx.x == 0) {
+    ctl->n_long = int32_t(n);
+    ctl->n_items_main = int32_t(n_items - n + parts);
+  }
+}
+
+// Merge of the long items' parts: warp per row; the near pass's list (its keys are not offered
+// again) and the parts' kper entries each, the k' smallest kept.  A key that none of them holds
+// was at or above its part's threshold or, in the near pass, the near list's k'-th value, which
+// the merged k'-th value does not exceed.
+__global__ void long_merge_kernel(const WorkItem* __restrict__ items, const Ctl* __restrict__ ctl,
+                                  const int32_t* __restrict__ order,
+                                  const int32_t* __restrict__ perm,
+                                  const int2* __restrict__ part,
+                                  const float* __restrict__ part_thr,
+                                  const float* __restrict__ near_val, int kprime, int kper,
+                                  int32_t* __restrict__ cand_idx, float* __restrict__ cand_thr) {
+  const int lane = lane_id();
+  const int64_t rows = int64_t(ctl->n_long) * QTILE;
+  const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  const int total = kprime + LONG_SPLIT * kper;        // <= 9 * 64
+  for (int64_t x = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; x < rows; x += warps) {
+    const int64_t r = x / QTILE;
+    const int j = int(x % QTILE);
+    const WorkItem w = items[order[r]];
+    if (j >= w.nq) continue;                           // warp-uniform
+    const int64_t orow = perm[w.qrow0 + j];
+    float v[18];
+    int id[18];
+#pragma unroll
+    for (int t = 0; t < 18; ++t) {
+      v[t] = F_INF;
+      id[t] = -1;
+      const int e = lane + 32 * t;
+      if (e < kprime) {
+        const int c = cand_idx[orow * kprime + e];
+        if (c >= 0) { v[t] = near_val[orow * kprime + e]; id[t] = c; }
+      } else if (e < total) {
+        const int s = (e - kprime) / kper, slot = (e - kprime) % kper;
+        const int2 pe = part[((r * LONG_SPLIT + s) * QTILE + j) * kprime + slot];
+        if (pe.y >= 0) { v[t] = __int_as_float(pe.x); id[t] = pe.y; }
+      }
+    }
+    float thr = lane < LONG_SPLIT ? part_thr[(r * LONG_SPLIT + lane) * QTILE + j] : F_INF;
+    for (int o = 16; o > 0; o >>= 1) thr = fminf(thr, __shfl_xor_sync(FULL, thr, o));
+    __syncwarp();                                      // the list is read before it is written
+    float kth = F_INF;
+    for (int o = 0; o < kprime; ++o) {
+      float bv = F_INF;
+      int bt = 18;
+#pragma unroll
+      for (int t = 0; t < 18; ++t)
+        if (v[t] < bv) { bv = v[t]; bt = t; }
+      float mv = bv;                                   // warp argmin of (value, lane)
+      int ml = lane;
+      for (int off = 16; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(FULL, mv, off);
+        const int ol = __shfl_xor_sync(FULL, ml, off);
+        if (ov < mv || (ov == mv && ol < ml)) { mv = ov; ml = ol; }
+      }
+      int out = -1;
+      if (lane == ml && bt < 18) {
+#pragma unroll
+        for (int t = 0; t < 18; ++t)
+          if (t == bt) { out = id[t]; v[t] = F_INF; }
+      }
+      out = __shfl_sync(FULL, out, ml);
+      if (lane == 0) cand_idx[orow * kprime + o] = mv < F_INF ? out : -1;
+      kth = mv;
+    }
+    if (lane == 0) cand_thr[orow] = fminf(kth, thr);
+  }
+}
+
 constexpr int VO_T = 256;            // threads per block of the order kernel
 constexpr int VO_SORT_MAX = 8192;    // longest list sorted (longer ones keep tile order)
 
@@ -1240,6 +1349,7 @@ PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items
   w.roff = c.take<double>(npacked);
   w.vcnt = c.take<int32_t>(n_items);
   w.claim = c.take<int32_t>(n_items);
+  w.claim2 = c.take<int32_t>(n_items + int64_t(w.max_split_items) * (LONG_SPLIT - 1));
   w.chist = c.take<int32_t>(COST_BUCKETS);
   w.voff = c.take<int64_t>(n_items + 1);
   w.vscan = c.take<int64_t>(scan_i32_scratch_elems(n_items));
@@ -1361,6 +1471,27 @@ int launch_claim_order(int64_t n_items, int words, const PruneWs& w, cudaStream_
   cost_offsets_kernel<<<1, COST_BUCKETS, 0, st>>>(w.chist);
   MSC_LAUNCH_CHECK();
   cost_scatter_kernel<<<hgrid, PR_T, 0, st>>>(w.vcnt, n_items, shift, w.chist, w.claim);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+int launch_long_plan(int64_t n_items, int words, int n_ctas, const PruneWs& w, Ctl* ctl,
+                     cudaStream_t st) {
+  int shift = 0;
+  while ((int64_t(words) * 32 >> shift) >= COST_BUCKETS) ++shift;
+  long_plan_kernel<<<1, LONG_T, 0, st>>>(w.vcnt, n_items, shift, n_ctas, w.max_split_items,
+                                         w.claim, w.claim2, ctl);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
+int launch_long_merge(const WorkItem* items, const Ctl* ctl, const int32_t* perm,
+                      const PruneWs& w, int kprime, int kper, int32_t* cand_idx,
+                      float* cand_thr, cudaStream_t st) {
+  const int grid = int(std::max<int64_t>(
+      1, std::min<int64_t>(int64_t(w.max_split_items) * QTILE / 8, int64_t(num_sms()) * 8)));
+  long_merge_kernel<<<grid, PR_T, 0, st>>>(items, ctl, w.claim, perm, w.part, w.part_thr,
+                                           w.cand_val, kprime, kper, cand_idx, cand_thr);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
