@@ -259,16 +259,30 @@ void plan_dense(Problem& P, int prec, int d, int64_t n, int k, int kprime) {
   const int nkt = int(ceil_div(n, 256));
   P.split = 1;
   P.kper = std::max(base, k - 1);
+  auto list = [&](int S) {
+    const double m = double(k - 1 + 8) / S;
+    const int kper = int(std::ceil(m + 4.0 * std::sqrt(m * (1.0 - 1.0 / S)))) + 1;
+    return std::max(kper, int(ceil_div(std::max(kprime, k - 1), S)));
+  };
   for (int S = 2; S <= std::min(DENSE_MAX_SPLIT, nkt); S *= 2) {
     const TcConfig c = tc_default_config(prec, d, P.kper);
     if (c.pair || P.ntiles * P.split >= int64_t(DENSE_ITEMS_PER_CTA) * c.ctas * num_sms()) break;
-    const double m = double(k - 1 + 8) / S;
-    int kper = int(std::ceil(m + 4.0 * std::sqrt(m * (1.0 - 1.0 / S)))) + 1;
-    kper = std::max(kper, int(ceil_div(std::max(kprime, k - 1), S)));
+    const int kper = list(S);
     if (kper * S > DENSE_SLOTS) break;
     P.split = S;
     P.kper = kper;
   }
+  // Fewer ranges where the last round of items would leave most CTAs idle: 10,000 cells in 4
+  // ranges are 316 items for 296 CTAs, 0.45 ms, in 3 ranges 237 items, 0.41; 25,000 cells 1.135
+  // and 1.038 ms.
+  const int64_t ctas = int64_t(tc_default_config(prec, d, P.kper).ctas) * num_sms();
+  auto rounds = [&](int S) { return double(ceil_div(P.ntiles * S, ctas)) / S; };
+  for (int S = P.split - 1, S0 = P.split; S > 1; --S)
+    if (list(S) * S <= DENSE_SLOTS && rounds(S) < 0.9 * rounds(S0) &&
+        rounds(S) < rounds(P.split)) {
+      P.split = S;
+      P.kper = list(S);
+    }
   P.kprime = P.split * P.kper;
   // a stride near n / golden ratio, coprime to n, spreads cells stored by cluster over the ranges
   P.stride = 1;

@@ -653,7 +653,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   // Items split over key ranges: work item it = (query tile it / S, range it % S).
   const int S = P.split_dev ? max(1, *P.split_dev) : P.split_host;
   auto item_of = [&](int it) {
-    if (P.long_kper && (it & LONG_FLAG)) return P.long_order[(it ^ LONG_FLAG) / LONG_SPLIT];
+    if (it & LONG_FLAG) return P.long_order[(it ^ LONG_FLAG) / LONG_SPLIT];
     return S > 1 ? it / S : it;
   };
   auto walk_init = [&](KeyTileWalk& walk, const WorkItem& w, int it) {
@@ -665,7 +665,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int sidx = S > 1 ? it % S : 0;
       const int chunk = (walk.nkt + S - 1) / S;
       walk.set_range(sidx * chunk, min(walk.nkt, (sidx + 1) * chunk));
-    } else if (P.long_kper && (it & LONG_FLAG)) {
+    } else if ((it & LONG_FLAG) != 0) {
       walk.set_every((it ^ LONG_FLAG) % LONG_SPLIT, LONG_SPLIT);
     }
   };
@@ -959,12 +959,9 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int nq = min(BM, w.nq - int(rank) * BM);   // this CTA's valid query rows (may be <= 0)
       const int qrow = w.qrow0 + int(rank) * BM;
       const int self = P.qmap ? (row < nq ? P.qmap[qrow + row] : -1) : qrow + row;
-      const bool lpart = P.long_kper && (it & LONG_FLAG);     // a part of a long item
-      const int kp = lpart ? P.long_kper : P.kprime;
-      if (kp != sel.kp) {
-        sel.kp = kp;
-        sel.reset();
-      }
+      const bool lpart = (it & LONG_FLAG) != 0;     // a part of a long item
+      // a part's shorter list: the slots beyond are never the largest
+      if (lpart) sel.shorten(P.long_kper);
       // pad0: the item's batch (batch-balanced scans), which has its own seeds and candidate slots
       sel.set_seed((P.seed && row < nq) ? P.seed[w.pad0 * P.thr_stride + qrow + row] : F_INF);
       if (P.init_val) {
@@ -1129,12 +1126,9 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       const int nvalid = min(32, nq - wrow0);
       auto write_out = [&]() {
         const int sidx = (S > 1 ? it % S : 0) + w.pad0;
-        if (lpart)
-          sel.finish_partial(P.part, P.part_thr, int64_t(it ^ LONG_FLAG) * BM + wrow0, P.perm,
+        if (lpart || (S > 1 && P.part))
+          sel.finish_partial(P.part, P.part_thr, int64_t(it & ~LONG_FLAG) * BM + wrow0, P.perm,
                              nvalid, P.kprime);
-        else if (S > 1 && P.part)
-          sel.finish_partial(P.part, P.part_thr, int64_t(it) * BM + wrow0, P.perm, nvalid,
-                             P.kprime);
         else
           sel.finish(cand_idx + sidx * P.kprime, cand_thr + sidx * P.thr_stride, P.cand_stride, P.perm, P.qmap, int64_t(qrow) + wrow0,
                      nvalid, P.kprime, P.cand_val);

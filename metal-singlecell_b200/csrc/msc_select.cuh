@@ -335,6 +335,14 @@ struct RowTopK {
     seed = F_INF;
   }
 
+  // an empty list of k < k' entries, until the next reset()
+  __device__ __forceinline__ void shorten(int k) {
+    for (int s = k; s < kp; ++s) hv[s * ROWS + row] = -F_INF;
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      if (g * GS >= k) gmax[g] = -F_INF;
+  }
+
   __device__ __forceinline__ void set_seed(float s) {
     seed = s;
     thr_f = fminf(thr_f, s);
