@@ -656,6 +656,12 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
                                  P.prec, P.L.kmma, P.L3.kmma, P.d, w.pr, st));
       mask3 = w.pr.mask3;
     }
+    const float* seed3 = nullptr;
+    if (prune && P.kref <= P.kprime) {
+      MSC_TRY(launch_refine_seed(w.qmap, &w.ctl->n_refine, P.n, w.perm, w.cand_thr, w.qs, w.km,
+                                 w.qs3, w.km3, w.ctl, P.prec, P.L.kmma, P.L3.kmma, P.d, w.pr, st));
+      seed3 = w.pr.seed3;
+    }
     const RefineSplit rs{&w.ctl->refine_split, parts ? w.pr.part : nullptr,
                          parts ? w.pr.part_thr : nullptr};
     const int64_t max_work = parts ? std::max<int64_t>(P.ntiles,
@@ -664,7 +670,7 @@ int run_knn(const Problem& P, const KnnWs& w, const float* X, int32_t* knn_idx, 
     MSC_TRY(launch_knn_tc(PREC_BF16X3, cfg3, w.A3, w.B3, P.n, P.npacked, P.L3.kp, P.L3.kmma,
                           w.items3, max_work, w.perm, w.qmap, &w.ctl->n_items_refine_eff,
                           &w.ctl->tc_counter[1], w.ctl, P.kref, w.cand_idx, w.cand_thr,
-                          P.kref, st, mask3, words3, false, false, nullptr, nullptr,
+                          P.kref, st, mask3, words3, false, false, seed3, nullptr,
                           parts ? &rs : nullptr));
     if (parts)
       MSC_TRY(launch_refine_merge(w.items3, &w.ctl->n_items_refine, w.ctl, w.qmap, w.perm, P.n,

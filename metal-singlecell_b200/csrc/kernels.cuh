@@ -164,6 +164,7 @@ struct PruneWs {
   unsigned long long* vlist;
   int64_t vcap;       // entries vlist holds
   int32_t* claim;      // main-scan claim order of the work items (costliest first)
+  float* seed3;        // per refine row: a bound on its k'-th three-term value
   int32_t* claim2;     // the same with the long items in parts (LongSplit)
   int32_t* chist;      // its bucket counts / offsets
 };
@@ -215,6 +216,11 @@ struct LongSplit {
 };
 int launch_long_plan(int64_t n_items, int words, int n_ctas, const PruneWs& w, Ctl* ctl,
                      cudaStream_t st);
+// after the main scan: seeds of the refine rows (PruneWs::seed3)
+int launch_refine_seed(const int32_t* qmap, const int32_t* n_rows, int64_t max_rows,
+                       const int32_t* perm, const float* cand_thr, const QStat* qs,
+                       const KeyMax* km, const QStat* qs3, const KeyMax* km3, const Ctl* ctl,
+                       int prec, int kmma, int kmma3, int d, const PruneWs& w, cudaStream_t st);
 int launch_long_merge(const WorkItem* items, const Ctl* ctl, const int32_t* perm,
                       const PruneWs& w, int kprime, int kper, int32_t* cand_idx,
                       float* cand_thr, cudaStream_t st);

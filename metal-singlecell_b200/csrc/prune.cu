@@ -708,10 +708,40 @@ __global__ void refine_mask_kernel(const WorkItem* __restrict__ items3,
   }
 }
 
+// Seeds of the refine pass: the main scan kept k' keys with one-term values at or below thr, so
+// their true values are at most (thr + eps1)/f² and their three-term values at most eps3 more: the
+// row's k'-th three-term value does not exceed that, and the pass need not keep anything above.
+// Without it each of a row's eight parts fills a list anew (18 insertions per cell of the sample,
+// now one): graphs of 200,000 cells 8.2 -> 7.55 ms, of 1.3 M 63.1 -> 61.5.
+// (A row of a long item has its merged k'-th value in seed and excl.x = -1: its threshold can be
+// a part's, which fewer than k' keys may reach.)
+__global__ void refine_seed_kernel(const int32_t* __restrict__ qmap,
+                                   const int32_t* __restrict__ n_rows,
+                                   const int32_t* __restrict__ perm,
+                                   const float* __restrict__ cand_thr,
+                                   const float* __restrict__ seed, const int4* __restrict__ excl,
+                                   const QStat* __restrict__ qs, const KeyMax* __restrict__ km,
+                                   const QStat* __restrict__ qs3, const KeyMax* __restrict__ km3,
+                                   const Ctl* __restrict__ ctl, int prec, int kmma, int kmma3,
+                                   int d, float* __restrict__ seed3) {
+  const int64_t n = *n_rows;
+  const double f = op_scale(prec, ctl), f3 = op_scale(PREC_BF16X3, ctl);
+  const KeyMax K1 = *km, K3 = *km3;
+  for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < n;
+       q += int64_t(gridDim.x) * blockDim.x) {
+    const int32_t p = qmap[q];
+    const double t = excl[p].x == -1 ? seed[p] : cand_thr[perm[p]];
+    const double e1 = cert_eps(qs[p], K1, prec, kmma, d);
+    const double e3 = cert_eps(qs3[p], K3, PREC_BF16X3, kmma3, d);
+    const double s = (t + e1) * (f3 / f) * (f3 / f) + e3;
+    seed3[q] = s < 1e30 ? nextafterf(__double2float_ru(s), F_INF) : F_INF;   // NaN: no seed
+  }
+}
+
 // Merge of a split refine pass: warp per refine row; the S·k' entries of its S work items, the k'
-// smallest kept (ties: lower lane, then lower slot).  The threshold is the k'-th smallest: each
-// work item's list holds k' values at or below its own k'-th value, so the merged k'-th value is
-// at most every work item's, and every key a work item dropped is at least that item's.
+// smallest kept (ties: lower lane, then lower slot).  The threshold is the k'-th smallest or, if
+// that is less, the work items' smallest (their seed, with which a list may stay short): every key
+// that a work item dropped is at least its threshold.
 __global__ void refine_merge_kernel(const WorkItem* __restrict__ items3,
                                     const int32_t* __restrict__ n_items3,
                                     const Ctl* __restrict__ ctl, const int32_t* __restrict__ qmap,
@@ -744,6 +774,8 @@ __global__ void refine_merge_kernel(const WorkItem* __restrict__ items3,
       }
     }
     const int64_t orow = perm[qmap[w.qrow0 + j]];
+    float thr = lane < S ? part_thr[(int64_t(r) * S + lane) * QTILE + j] : F_INF;   // S <= 32
+    for (int o = 16; o > 0; o >>= 1) thr = fminf(thr, __shfl_xor_sync(FULL, thr, o));
     float kth = F_INF;
     for (int o = 0; o < kprime; ++o) {
       float bv = F_INF;
@@ -769,7 +801,7 @@ __global__ void refine_merge_kernel(const WorkItem* __restrict__ items3,
       if (lane == 0) cand_idx[orow * kprime + o] = mv < F_INF ? out : -1;
       kth = mv;
     }
-    if (lane == 0) cand_thr[orow] = kth;
+    if (lane == 0) cand_thr[orow] = fminf(kth, thr);
   }
 }
 
@@ -890,7 +922,8 @@ __global__ void long_merge_kernel(const WorkItem* __restrict__ items, const Ctl*
                                   const int2* __restrict__ part,
                                   const float* __restrict__ part_thr,
                                   const float* __restrict__ near_val, int kprime, int kper,
-                                  int32_t* __restrict__ cand_idx, float* __restrict__ cand_thr) {
+                                  int32_t* __restrict__ cand_idx, float* __restrict__ cand_thr,
+                                  float* __restrict__ seed, int4* __restrict__ excl) {
   const int lane = lane_id();
   const int64_t rows = int64_t(ctl->n_long) * QTILE;
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -944,7 +977,11 @@ __global__ void long_merge_kernel(const WorkItem* __restrict__ items, const Ctl*
       if (lane == 0) cand_idx[orow * kprime + o] = mv < F_INF ? out : -1;
       kth = mv;
     }
-    if (lane == 0) cand_thr[orow] = fminf(kth, thr);
+    if (lane == 0) {
+      cand_thr[orow] = fminf(kth, thr);
+      seed[w.qrow0 + j] = fminf(kth, seed[w.qrow0 + j]);   // for the refine pass (refine_seed)
+      excl[w.qrow0 + j].x = -1;
+    }
   }
 }
 
@@ -1347,6 +1384,7 @@ PruneWs carve_prune(Carver& c, int64_t npacked, int nseg, int d, int64_t n_items
   carve_refine_parts(c, w, int(std::min<int64_t>(256, n_items)), kprime);
   w.seed = c.take<float>(npacked);
   w.roff = c.take<double>(npacked);
+  w.seed3 = c.take<float>(n);
   w.vcnt = c.take<int32_t>(n_items);
   w.claim = c.take<int32_t>(n_items);
   w.claim2 = c.take<int32_t>(n_items + int64_t(w.max_split_items) * (LONG_SPLIT - 1));
@@ -1475,6 +1513,17 @@ int launch_claim_order(int64_t n_items, int words, const PruneWs& w, cudaStream_
   return MSC_OK;
 }
 
+int launch_refine_seed(const int32_t* qmap, const int32_t* n_rows, int64_t max_rows,
+                       const int32_t* perm, const float* cand_thr, const QStat* qs,
+                       const KeyMax* km, const QStat* qs3, const KeyMax* km3, const Ctl* ctl,
+                       int prec, int kmma, int kmma3, int d, const PruneWs& w, cudaStream_t st) {
+  refine_seed_kernel<<<grid_for(max_rows), PR_T, 0, st>>>(qmap, n_rows, perm, cand_thr, w.seed,
+                                                          w.excl, qs, km, qs3, km3, ctl, prec,
+                                                          kmma, kmma3, d, w.seed3);
+  MSC_LAUNCH_CHECK();
+  return MSC_OK;
+}
+
 int launch_long_plan(int64_t n_items, int words, int n_ctas, const PruneWs& w, Ctl* ctl,
                      cudaStream_t st) {
   int shift = 0;
@@ -1491,7 +1540,8 @@ int launch_long_merge(const WorkItem* items, const Ctl* ctl, const int32_t* perm
   const int grid = int(std::max<int64_t>(
       1, std::min<int64_t>(int64_t(w.max_split_items) * QTILE / 8, int64_t(num_sms()) * 8)));
   long_merge_kernel<<<grid, PR_T, 0, st>>>(items, ctl, w.claim, perm, w.part, w.part_thr,
-                                           w.cand_val, kprime, kper, cand_idx, cand_thr);
+                                           w.cand_val, kprime, kper, cand_idx, cand_thr, w.seed,
+                                           w.excl);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }
