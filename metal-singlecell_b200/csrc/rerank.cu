@@ -57,18 +57,6 @@ __device__ __forceinline__ double d2_f64(const float* xs, const float* __restric
   return acc;
 }
 
-// the same for the full scans: eight loads in flight (a scanned row waits for little else; an
-// uncertified row of 25,000 keys took 5 ms by itself)
-__device__ __forceinline__ double d2_f64_scan(const float* xs, const float* __restrict__ y, int d) {
-  double acc = 0.0;
-#pragma unroll 8
-  for (int t = 0; t < d; ++t) {
-    double df = double(xs[t]) - double(y[t]);
-    acc += df * df;
-  }
-  return acc;
-}
-
 // One lane's share of the FP32 squared distance of a shared-memory row xs and row y when the 4
 // lanes of a group split the row (part = lane & 3 takes every 4th 8-byte pair, or every 4th
 // element of a row that is not 8-byte aligned); the group then sums the four shares.  The warp
@@ -304,7 +292,7 @@ fp64_scan_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__
       double v = INF;
       int vi = INT32_MAX;
       if (jj < ns && off + jj != i) {
-        v = d2_f64_scan(xs, X + (off + jj) * d, d);
+        v = d2_f64(xs, X + (off + jj) * d, d, false);
         vi = int(off + jj);
       }
       top.offer(v, vi, kk);
