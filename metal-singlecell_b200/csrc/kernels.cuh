@@ -84,6 +84,11 @@ __device__ __forceinline__ double cert_eps(const QStat& q, const KeyMax& km, int
   return 2.0 * dot_err + Kn + acc_err + 0x1p-40 * (q.sq + Ks);
 }
 
+// An FP32 sum v of d squares has the relative error bound (d+4)·2^-24 while its terms are normal
+// numbers.  Below that range each of its d roundings may be off by 2^-150, which no relative bound
+// covers: |v - s| <= (d+4)·2^-24·s + f32_sq_floor(d).  (Embeddings of a spread near 1e-21 get there.)
+__device__ __forceinline__ double f32_sq_floor(int d) { return double(d) * 0x1p-149; }
+
 // ---- prep.cu ----
 int launch_normalize(const float* X, float* Xn, int64_t n, int d, int64_t* nonfinite,
                      cudaStream_t st);
