@@ -76,11 +76,12 @@ __device__ __forceinline__ double cert_eps(const QStat& q, const KeyMax& km, int
   const double Ks = __uint_as_float(km.sq);
   const double qh = q.hi, ql = q.lo, qr = q.res;
   const double dot_err = ql * Kl + (qh + ql) * Kr + qr * (Kh + Kl) + qr * Kr;
+  // the last terms: what sums below FP32's normal range lose (a tensor core may flush them to zero)
   double acc_err;
   if (prec == PREC_FP32)
-    acc_err = 0x1p-23 * ((2.0 * d + 4.0) * qh * Kh + 2.0 * Ks);
+    acc_err = 0x1p-23 * ((2.0 * d + 4.0) * qh * Kh + 2.0 * Ks) + (2.0 * d + 8.0) * 0x1p-149;
   else
-    acc_err = double(kmma) * 0x1p-22 * (2.0 * (qh + ql) * (Kh + Kl) + Ks);
+    acc_err = double(kmma) * (0x1p-22 * (2.0 * (qh + ql) * (Kh + Kl) + Ks) + 0x1p-126);
   return 2.0 * dot_err + Kn + acc_err + 0x1p-40 * (q.sq + Ks);
 }
 

@@ -32,3 +32,38 @@ def assert_lists(X, k, **kw):
 @pytest.mark.parametrize("k", [83, 200])
 def test_wide_lists(k, scale):
     assert_lists(cells(scale), k)
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("precision", ["fp16", "bf16x3", "bf16", "fp32"])
+def test_candidate_lists(precision, scale):
+    assert_lists(cells(scale), 15, precision=precision)
+
+
+@pytest.mark.parametrize("scale", [1e-20, 1e-21, 1e-22])
+def test_pruned_scan(scale):
+    import torch
+    X = synth.gaussian_mixture(60_000, 50, 40, seed=11, sizes="lognormal", noise_frac=0.01)
+    X = (X.astype(np.float64) * scale).astype(np.float32)
+    idx, dist, _ = nbm.knn_device(torch.from_numpy(X).cuda(), 15)
+    rows = np.sort(np.random.default_rng(5).choice(X.shape[0], 1_000, replace=False))
+    ri, _, rd = oracle.knn_exact(X, 15, rows=rows)
+    np.testing.assert_array_equal(idx.cpu().numpy()[rows], ri.astype(np.int32))
+    np.testing.assert_array_equal(dist.cpu().numpy()[rows], rd)
+
+
+@pytest.mark.parametrize("scale", SCALES)
+@pytest.mark.parametrize("precision", ["fp16", "bf16x3"])
+@pytest.mark.parametrize("least", ["-1", "0"])               # batch by batch, in locality order
+def test_batch_balanced_lists(least, precision, scale, monkeypatch):
+    import torch
+    from oracle import bbknn as obb
+    from msc_b200 import bbknn as bbm
+    monkeypatch.setenv("MSC_B200_BB_ORDER", least)
+    X, batch = cells(scale), np.random.default_rng(1).integers(0, 3, 1_500)
+    _, codes, counts = bbm.batch_codes(batch)
+    res = bbm.bbknn_device(torch.from_numpy(X).cuda(), torch.from_numpy(codes).cuda(), counts, 3,
+                           precision=precision)
+    _, _, _, inter = obb.bbknn(X, batch, 3, n_pcs=None)
+    np.testing.assert_array_equal(res["knn_idx"].cpu().numpy(), inter["idx"].astype(np.int32))
+    np.testing.assert_array_equal(res["knn_dist"].cpu().numpy(), inter["dist"])
