@@ -420,7 +420,8 @@ struct RowTopK {
   // Merge another selector of the same row (same layout, base `other`) into this one.  Nothing is
   // published meanwhile: the partner reads this row's published threshold as +inf until the next
   // tile.  Entries in the excluded ranges are skipped: both were loaded with the same earlier
-  // candidates, so this one holds its own copy or has dropped the key for k' better ones.
+  // candidates, so this one holds its own copy or has dropped the key for k' better ones.  Slots
+  // without a key are skipped: free ones, and those beyond a shortened list, which hold -inf.
   __device__ __forceinline__ void merge_from(const void* other) {
     const float* OV = static_cast<const float*>(other) + row;
     const int* OC = reinterpret_cast<const int*>(static_cast<const float*>(other) + KH * ROWS) + row;
@@ -430,7 +431,7 @@ struct RowTopK {
       const float v = OV[s * ROWS];
       const int c = OC[s * ROWS];
       const bool loaded = (c >= ex_r0 && c < ex_r1) || (c >= ex_o0 && c < ex_o1);
-      if (v < thr && !loaded) insert(v, c);
+      if (c >= 0 && v < thr && !loaded) insert(v, c);
     }
     pub_own = keep;
   }
