@@ -273,7 +273,7 @@ bb_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1,
   const KeyMax kmv = *km;
   const double f = op_scale(prec, ctl);
   const double f2 = f * f;
-  const double delta = double(d + 4) * 0x1p-24, slack = 2.0 * f32_sq_floor(d);
+  const double delta = double(d + 4) * 0x1p-24;
   const double INF = __longlong_as_double(0x7ff0000000000000ll);
   int64_t n_cert = 0;
   for (int64_t i = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; i < n; i += nwarps) {
@@ -287,7 +287,7 @@ bb_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1,
     warp_sort64_d(v0, i0, v1, i1);
     const double B = __shfl_sync(FULL, kk - 1 < 32 ? v0 : v1, (kk - 1) & 31);
     // FP64 for the window of FP32 values within B·(1+3δ) and the rounding of subnormal sums
-    const double lim = B * (1.0 + 3.0 * delta) + slack;
+    const double lim = B * (1.0 + 3.0 * delta) + 2.0 * F32_SQ_FLOOR;
     const bool w0 = i0 != INT32_MAX && v0 <= lim;
     const bool w1 = i1 != INT32_MAX && v1 <= lim;
     double g0 = w0 ? bb_d2_f64(xs, X + int64_t(i0) * d, d) : INF;
@@ -347,7 +347,7 @@ bb_group_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1
   const KeyMax kmv = *km;
   const double f = op_scale(prec, ctl);
   const double f2 = f * f;
-  const double delta = double(d + 4) * 0x1p-24, slack = 2.0 * f32_sq_floor(d);
+  const double delta = double(d + 4) * 0x1p-24;
   const double INF = __longlong_as_double(0x7ff0000000000000ll);
   const unsigned lt = (1u << lane) - 1u;
   int64_t n_cert = 0;
@@ -376,7 +376,7 @@ bb_group_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1
       bool ok = !__any_sync(FULL, isnan(e));
       float sv = e;
       warp_sort32_f(sv);
-      const double lim = double(__shfl_sync(FULL, sv, kk - 1)) * (1.0 + 3.0 * delta) + slack;
+      const double lim = double(__shfl_sync(FULL, sv, kk - 1)) * (1.0 + 3.0 * delta) + 2.0 * F32_SQ_FLOOR;
       const bool in = c >= 0 && double(e) <= lim;
       const unsigned m = __ballot_sync(FULL, in);
       const int nw = __popc(m);

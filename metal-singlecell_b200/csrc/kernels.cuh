@@ -87,8 +87,10 @@ __device__ __forceinline__ double cert_eps(const QStat& q, const KeyMax& km, int
 
 // An FP32 sum v of d squares has the relative error bound (d+4)·2^-24 while its terms are normal
 // numbers.  Below that range each of its d roundings may be off by 2^-150, which no relative bound
-// covers: |v - s| <= (d+4)·2^-24·s + f32_sq_floor(d).  (Embeddings of a spread near 1e-21 get there.)
-__device__ __forceinline__ double f32_sq_floor(int d) { return double(d) * 0x1p-149; }
+// covers: |v - s| <= (d+4)·2^-24·s + F32_SQ_FLOOR / 2.  (Embeddings of a spread near 1e-21 get
+// there.)  One constant for every d: as a value computed from d it held registers through the
+// re-rank and the plan, which cost graphs of 200,000 cells 0.3 %.
+constexpr double F32_SQ_FLOOR = MSC_MAX_D * 0x1p-149;
 
 // ---- prep.cu ----
 int launch_normalize(const float* X, float* Xn, int64_t n, int d, int64_t* nonfinite,

@@ -349,9 +349,11 @@ sub_ball_kernel(const float* __restrict__ X, int d, int dp,
 // taken once per ball u (ball_reach) and a test compares squares (its 1e-12 covers the FP64
 // roundings).  An empty ball is separated from everything; an unknown R (reach +inf) from nothing.
 // Centres are n4 float4 (zero padded), SA and SB float4s apart; the FP32 distance is lowered by its
-// rounding bound (d+8 units of 2^-23 relative, and f32_sq_floor) before the test.
+// rounding bound (d+8 units of 2^-23 relative) before the test; what its square loses below FP32's
+// normal range is in reach (far + a squared is at least far² + a²).
 __device__ __forceinline__ double ball_reach(double R, double f) {
-  return R < 1e300 ? sqrt(R * (1.0 + 1e-9)) / f : __longlong_as_double(0x7ff0000000000000ll);
+  return R < 1e300 ? sqrt(R * (1.0 + 1e-9)) / f + sqrt(F32_SQ_FLOOR)
+                   : __longlong_as_double(0x7ff0000000000000ll);
 }
 template <int SA, int SB>
 __device__ __forceinline__ float ball_d2(const float4* a, const float4* b, int n4) {
@@ -369,7 +371,7 @@ __device__ __forceinline__ float ball_d2(const float4* a, const float4* b, int n
 }
 __device__ __forceinline__ bool apart(float d2, float ru, float rw, double reach, int d) {
   if (ru < 0.f || rw < 0.f) return true;
-  const double lo = double(d2) * (1.0 - double(d + 8) * 0x1p-23) - f32_sq_floor(d);
+  const double lo = double(d2) * (1.0 - double(d + 8) * 0x1p-23);
   const double far = (double(ru) + double(rw) + reach) * (1.0 + 1e-12);
   return lo > far * far;
 }
@@ -576,7 +578,7 @@ point_test_kernel(const float* __restrict__ X, int d, int dp, const int32_t* __r
   constexpr int NW = POINT_T / 32;
   const double f = op_scale(prec, ctl);
   const double f2 = f * f;
-  const double shrink = 1.0 - double(d + 8) * 0x1p-23, low = f32_sq_floor(d);
+  const double shrink = 1.0 - double(d + 8) * 0x1p-23;
   long long cleared = 0;
   if (tid < 256 / 32) pad_bits[tid] = 0u;
   for (int64_t gb = blockIdx.x; gb < nkt_all * POINT_SLICES; gb += gridDim.x) {   // block-uniform
@@ -632,7 +634,7 @@ point_test_kernel(const float* __restrict__ X, int d, int dp, const int32_t* __r
               const float u = c[t] - ys[t * 256 + key];
               acc = fmaf(u, u, acc);
             }
-            const double L = sqrt(fmax(0.0, double(acc) * shrink - low)) - double(rq);
+            const double L = sqrt(fmax(0.0, double(acc) * shrink - F32_SQ_FLOOR)) - double(rq);
             sep = L > 0.0 && f2 * L * L > R * (1.0 + 1e-9);
           }
           all = __all_sync(FULL, sep);
@@ -1062,7 +1064,7 @@ visit_order_kernel(const WorkItem* __restrict__ items, int64_t n_items, int bn, 
           }
           const float sum = (s0 + s1) + (s2 + s3);
           dist = sum;
-          const double L = sqrt(fmax(0.0, double(sum) * (1.0 - e) - f32_sq_floor(d))) -
+          const double L = sqrt(fmax(0.0, double(sum) * (1.0 - e) - F32_SQ_FLOOR)) -
                            double(rq) - double(rk);
           need = L > 0.0 ? __double2float_rd(f2 * L * L * (1.0 - 1e-12)) : 0.f;
         } else {

@@ -115,7 +115,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
   const KeyMax kmv = *km;
   const double f = op_scale(prec, ctl);
   const double f2 = f * f;
-  const double delta = double(d + 4) * 0x1p-24, slack = 2.0 * f32_sq_floor(d);
+  const double delta = double(d + 4) * 0x1p-24;
   int64_t n_cert = 0, n_ties = 0;
   const int64_t count = rows ? int64_t(*nrows) : npacked;
   for (int64_t wq = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; wq < count;
@@ -168,7 +168,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
       float s0 = e0, s1 = e1;
       warp_sort64_f(s0, s1);
       const float Bf = __shfl_sync(FULL, kk - 1 < 32 ? s0 : s1, (kk - 1) & 31);
-      const double limf = double(Bf) * (1.0 + 3.0 * delta) + slack;
+      const double limf = double(Bf) * (1.0 + 3.0 * delta) + 2.0 * F32_SQ_FLOOR;
       const bool w0 = c0 >= 0 && double(e0) <= limf;
       const bool w1 = c1 >= 0 && double(e1) <= limf;
       const unsigned b0 = __ballot_sync(FULL, w0), b1 = __ballot_sync(FULL, w1);
@@ -195,7 +195,7 @@ rerank_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ pe
       warp_sort64_d(v0, i0, v1, i1);
       const float se0 = float(v0), se1 = float(v1);
       const float B = __shfl_sync(FULL, kk - 1 < 32 ? se0 : se1, (kk - 1) & 31);
-      const double lim = double(B) * (1.0 + 3.0 * delta) + slack;
+      const double lim = double(B) * (1.0 + 3.0 * delta) + 2.0 * F32_SQ_FLOOR;
       const bool w0 = i0 != INT32_MAX && double(se0) <= lim;
       const bool w1 = i1 != INT32_MAX && double(se1) <= lim;
       g0 = w0 ? d2_f64(xs, X + int64_t(i0) * d, d, pairs) : INF;

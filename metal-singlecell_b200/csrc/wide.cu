@@ -13,8 +13,7 @@
 //               row's buffer (δ = (d+4)·2^-24, the FP32 sum's relative error bound);
 //   3. select   B = the (k-1)-th smallest FP32 value of the buffer; the keys within B·(1 + 3δ) + 2φ
 //               are recomputed in FP64 (dimension order) and ordered by (FP64 value, index).
-//               φ = d·2^-149 covers the roundings of sums below FP32's normal range
-//               (f32_sq_floor).
+//               φ (F32_SQ_FLOOR) covers the roundings of sums below FP32's normal range.
 //
 // A key left out in step 2 has an FP32 value above T', hence a squared distance above (T'-φ)/(1+δ);
 // the row is exact when its (k-1)-th FP64 value is below that, else (too few or too many collected,
@@ -292,7 +291,6 @@ wide_select_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
   double* val = val_all[wib];
   float* xs = xs_all[wib];
   const float delta = float(d + 4) * 0x1p-24f;
-  const double floor_d = f32_sq_floor(d);
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   int done = 0;
   for (int64_t rr = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; rr < nrows;
@@ -315,7 +313,7 @@ wide_select_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
         if (__reduce_add_sync(FULL, n_le) < kk) lo = mid + 1;
         else hi = mid;
       }
-      const double lim = double(__uint_as_float(hi)) * (1.0 + 3.0 * double(delta)) + 2.0 * floor_d;
+      const double lim = double(__uint_as_float(hi)) * (1.0 + 3.0 * double(delta)) + 2.0 * F32_SQ_FLOOR;
       int w = 0;                                        // the window's keys
       for (int e0 = 0; e0 < c; e0 += 32) {
         const int e = e0 + lane;
@@ -351,7 +349,7 @@ wide_select_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
             if (s * 32 < w) rank[s] += dless(vf, jf, g[s], id[s]);
         }
         bool below = false;                             // the kk-th value is below the bound
-        const double bound = (double(thr[p]) - floor_d) / (1.0 + double(delta));
+        const double bound = (double(thr[p]) - F32_SQ_FLOOR) / (1.0 + double(delta));
 #pragma unroll
         for (int s = 0; s < SLOTS; ++s)
           below = below || (s * 32 + lane < w && rank[s] == kk - 1 && g[s] < bound);
