@@ -347,8 +347,13 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
     const int64_t most = env && *env ? std::atoll(env) : DENSE_MAX_CELLS;
     if (n <= most) {
       P.dense = true;
+      // Rows come to the refine pass because their k-th place is crowded, so its lists stay as long
+      // as the one-term pass's unless 32 candidates are twice the neighbours already.  (k + 8
+      // of them left 5,885 of 57,000 x 128 rows, k = 33, to the FP64 scan where 48 leave 22: graph
+      // 192 and 39 ms.  At k = 15 32 and 48 leave the same rows, and 20,000 BF16 cells take 1.47
+      // ms with 32, 1.78 with 48.)
+      P.kref = 2 * (k - 1) <= 32 ? 32 : std::max(P.kprime, default_kprime(P.prec, k));
       plan_dense(P, P.prec, d, n, k, kprime);
-      P.kref = std::min(P.kprime, std::max(k - 1, default_kprime(PREC_BF16X3, k)));
     }
   }
   if (P.candidates && k > 1 && (P.prec == PREC_FP16 || P.prec == PREC_BF16)) {
@@ -400,7 +405,7 @@ KnnWs carve_knn(Carver& c, const Problem& P) {
     w.Bop = c.take<uint16_t>(size_t(P.npacked) * P.L.kp);
   }
   w.qs = c.take<QStat>(P.npacked);
-  w.cand_idx = c.take<int32_t>(size_t(P.n) * P.kprime);
+  w.cand_idx = c.take<int32_t>(size_t(P.n) * std::max(P.kprime, P.kref));
   w.cand_thr = c.take<float>(size_t(P.n) * P.split);
   w.fail_rows = c.take<int32_t>(P.n);
   w.perm = c.take<int32_t>(P.npacked);
