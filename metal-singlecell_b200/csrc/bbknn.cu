@@ -667,12 +667,15 @@ BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int pre
   P.candidates = P.kk_max + 1 <= 64 && prec != PREC_FP32 && d <= MSC_MAX_D;
   P.kprime = 0;
   if (P.candidates) {
-    // over-fetch: the certificate compares the kk-th neighbour with the k'-th candidate, a wide
-    // margin already at k' = 24 for the usual kk = 3 (the self path's k' = 48 is sized for the
-    // 15th neighbour); wider lists for larger kk.  8 batches of 200,000 x 50: k' = 32 no cell
-    // uncertified, 14.3 ms; 24 none, 13.3 ms; 16 two to eleven of 1.6 M, each an FP64 scan
+    // over-fetch: the certificate compares the kk-th neighbour with the k'-th candidate (the self
+    // path's k' = 48 is sized for the 15th neighbour); wider lists for larger kk.  A cell it cannot
+    // certify takes an FP64 scan of the batch, milliseconds for a lone one, which is more than
+    // shorter lists save: with one-term operands k' = 24 saves 7 % where every cell passes (8
+    // batches of 200,000 x 50, FP16: 13.7 against 14.7 ms), but 123,000 x 30 with one such cell
+    // took 8.8 ms against 6.2, 60,000 x 50 in BF16 146 against 91.  The three-term split left no
+    // cell at 24.
     P.kprime = prec == PREC_BF16X3 ? std::min(64, std::max(24, P.kk_max + 9))
-                                   : std::min(64, std::max(24, P.kk_max + 16));
+                                   : std::min(64, std::max(32, P.kk_max + 16));
     P.L = op_layout(prec, d);
     P.cfg = tc_default_config(prec, d, P.kprime);
     if (P.cfg.pair || !tc_config_ok(P.cfg, P.L.kp, P.kprime)) P.candidates = false;
