@@ -180,18 +180,6 @@ __device__ __forceinline__ float bb_d2_f32(const float* xs, const float* __restr
   return acc;
 }
 
-// the same for the scans: eight loads in flight (a scanned row waits for little else)
-__device__ __forceinline__ double bb_d2_f64_scan(const float* xs, const float* __restrict__ y,
-                                                 int d) {
-  double acc = 0.0;
-#pragma unroll 8
-  for (int t = 0; t < d; ++t) {
-    const double df = double(xs[t]) - double(y[t]);
-    acc += df * df;
-  }
-  return acc;
-}
-
 // four lanes' shares of an FP32 squared distance (part = lane & 3 takes every fourth 8-byte pair, or
 // every fourth element of a row that is not 8-byte aligned); any order of the sum stays within the
 // (d+4)·2^-24 the windows assume
@@ -239,7 +227,7 @@ __device__ __forceinline__ void bb_scan_row(const float* __restrict__ X, int d, 
     if (jj < nb) {
       const int32_t c = perm[jj];
       if (c >= 0) {
-        v = bb_d2_f64_scan(xs, X + int64_t(c) * d, d);
+        v = bb_d2_f64(xs, X + int64_t(c) * d, d);
         vi = c;
       }
     }
