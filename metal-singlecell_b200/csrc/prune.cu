@@ -882,7 +882,11 @@ __global__ void cost_scatter_kernel(const int32_t* __restrict__ cnt, int64_t n_i
 // 0.25 100,000 cells take 5.2 and 5.6 ms, 1.3 M 63 and 73 (1.0: 63).  The parts' lists hold 32 of
 // k' = 48: with 24 the 200,000 cells take 8.5 ms (more rows left to the refine pass), with 48 the
 // 100,000 take 0.2 ms more.
-constexpr double LONG_SHARE = 1.0;
+// With fewer than two items per CTA a CTA's share falls below the items' mean, and items like all the
+// others would count as long: of 31,382 uniform cells (246 items, 296 CTAs) every one was, with five
+// times the insertions.  So a long item also costs LONG_TIMES the mean: cohorts of 43,947 cells in
+// seven samples 3.44 -> 2.30 ms, of 24,866 in four 2.42 -> 1.70.
+constexpr double LONG_SHARE = 1.0, LONG_TIMES = 2.0;
 constexpr int LONG_NEAR = 5;          // near tiles an item scans besides
 constexpr int LONG_T = 1024;
 __global__ void __launch_bounds__(LONG_T)
@@ -898,7 +902,7 @@ long_plan_kernel(const int32_t* __restrict__ cnt, int64_t n_items, int shift, in
   atomicAdd(&total, t);
   __syncthreads();
   // whole buckets of the claim order, so that the long items are its first ones
-  const double cut = double(total) / n_ctas * LONG_SHARE;
+  const double cut = double(total) * fmax(LONG_SHARE / n_ctas, LONG_TIMES / double(n_items));
   const int bucket = int(fmin(cut, 1e9)) >> shift;
   int m = 0;
   for (int64_t i = threadIdx.x; i < n_items; i += LONG_T)
