@@ -37,6 +37,7 @@ namespace {
 constexpr int SP_T = 128;                 // threads per block of the search kernels
 constexpr int SP_W = SP_T / 32;
 constexpr int LANE_R = 4;                 // kNN: largest box of cells one lane walks
+constexpr int FAR_RUN = 32;               // ... most points of a row of cells it reads alone
 constexpr double CELL_PER_K = 0.33;       // kNN in the plane: points per cell / k
 constexpr int SORT_TILE = 256;            // columns staged per warp by the row sort
 constexpr int SORT_E = 4;                 // entries ranked per lane per group
@@ -416,38 +417,63 @@ sp_knn_far_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ ce
     int rmax = 0;
 #pragma unroll
     for (int a = 0; a < D; ++a) rmax = max(rmax, max(c[a], g.g[a] - 1 - c[a]));
-    // f(first, last + 1) for the lane's rows of box R, cut to the cells within r
+    // f(first, step, last + 1) for the points of box R, cut to the cells within r: a lane takes a
+    // row of cells, and a row of more than FAR_RUN points goes to the whole warp (a lone lane
+    // reading the 30,000 points of one cell is a load latency for each: 11 ms).
     auto rows = [&](int R, double r, auto&& f) {
       const int y0 = max(c[1] - R, 0), y1 = min(c[1] + R, g.g[1] - 1), ny = y1 - y0 + 1;
       const int z0 = D == 3 ? max(c[2] - R, 0) : 0, z1 = D == 3 ? min(c[2] + R, g.g[2] - 1) : 0;
-      for (int64_t e = lane; e < int64_t(ny) * (z1 - z0 + 1); e += 32) {
-        const int y = y0 + int(e % ny), z = z0 + int(e / ny);
-        double rest = r * r;                       // (reach along x)², from the row's distance
-        const double ly = g.o[1] + double(y) * g.cs;
-        const double ey = fmax(0.0, fmax(ly - double(qq[1]), double(qq[1]) - (ly + g.cs)));
-        rest -= ey * ey;
-        if (D == 3) {
-          const double lz = g.o[2] + double(z) * g.cs;
-          const double ez = fmax(0.0, fmax(lz - double(qq[2]), double(qq[2]) - (lz + g.cs)));
-          rest -= ez * ez;
+      const int64_t nrow = int64_t(ny) * (z1 - z0 + 1);
+      for (int64_t e0 = 0; e0 < nrow; e0 += 32) {  // warp-uniform
+        const int64_t e = e0 + lane;
+        int64_t a = 0, b = 0;
+        if (e < nrow) {
+          const int y = y0 + int(e % ny), z = z0 + int(e / ny);
+          double rest = r * r;                     // (reach along x)², from the row's distance
+          const double ly = g.o[1] + double(y) * g.cs;
+          const double ey = fmax(0.0, fmax(ly - double(qq[1]), double(qq[1]) - (ly + g.cs)));
+          rest -= ey * ey;
+          if (D == 3) {
+            const double lz = g.o[2] + double(z) * g.cs;
+            const double ez = fmax(0.0, fmax(lz - double(qq[2]), double(qq[2]) - (lz + g.cs)));
+            rest -= ez * ez;
+          }
+          int x0 = max(c[0] - R, 0), x1 = min(c[0] + R, g.g[0] - 1);
+          if (rest < 1e300) {                      // one cell to spare on either side
+            const double h = sqrt(fmax(rest, 0.0)) / g.cs + 1.0;
+            const double at = (double(qq[0]) - g.o[0]) / g.cs;
+            x0 = max(x0, int(fmax(floor(at - h), 0.0)));
+            x1 = min(x1, int(fmin(floor(at + h), double(g.g[0] - 1))));
+          }
+          if (rest >= 0.0 && x0 <= x1) {
+            const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
+            a = cell_start[row + x0];
+            b = cell_start[row + x1 + 1];
+          }
         }
-        if (rest < 0.0) continue;
-        int x0 = max(c[0] - R, 0), x1 = min(c[0] + R, g.g[0] - 1);
-        if (rest < 1e300) {                        // one cell to spare on either side
-          const double h = sqrt(rest) / g.cs + 1.0;
-          const double at = (double(qq[0]) - g.o[0]) / g.cs;
-          x0 = max(x0, int(fmax(floor(at - h), 0.0)));
-          x1 = min(x1, int(fmin(floor(at + h), double(g.g[0] - 1))));
-        }
-        if (x0 > x1) continue;
-        const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
-        f(cell_start[row + x0], cell_start[row + x1 + 1]);
+        unsigned longs = __ballot_sync(0xffffffffu, b - a > FAR_RUN);
+        bool own = true;                           // the lanes' own rows first
+        do {
+          int64_t i = a, last = b - a > FAR_RUN ? a : b;
+          int step = 1;
+          if (!own) {
+            const int src = __ffs(longs) - 1;
+            longs &= longs - 1;
+            i = __shfl_sync(0xffffffffu, a, src) + lane;
+            last = __shfl_sync(0xffffffffu, b, src);
+            step = 32;
+          }
+          own = false;
+          if (i < last) f(i, step, last);
+          __syncwarp();
+        } while (longs);
       }
     };
     int R = LANE_R;
     for (;; R *= 2) {
       long long have = 0;
-      rows(min(R, rmax), INFINITY, [&](int64_t a, int64_t b) { have += b - a; });
+      rows(min(R, rmax), INFINITY,
+           [&](int64_t i, int step, int64_t last) { have += (last - i + step - 1) / step; });
       for (int off = 16; off > 0; off >>= 1) have += __shfl_xor_sync(0xffffffffu, have, off);
       if (have >= k || R >= rmax) break;
     }
@@ -457,10 +483,12 @@ sp_knn_far_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ ce
     for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
       for (int j = 0; j < K; ++j) { s[j] = INFINITY; id[j] = INT_MAX; }
-      rows(min(R, rmax), r, [&](int64_t a, int64_t b) {
-        evals += b - a;
-        for (; a < b; ++a) {
-          const float4 p = pts[a];
+      rows(min(R, rmax), r, [&](int64_t i, int step, int64_t last) {
+        evals += (last - i + step - 1) / step;
+        float4 ahead = pts[i];
+        for (; i < last; i += step) {
+          const float4 p = ahead;                  // the next one loads meanwhile
+          if (i + step < last) ahead = pts[i + step];
           const int pid = __float_as_int(p.w);
           const float sd = __fsqrt_rn(sq_dist<D>(p, q));
           if (pid == qi || !key_less(sd, pid, s[K - 1], id[K - 1])) continue;
