@@ -37,6 +37,8 @@ namespace {
 constexpr int SP_T = 128;                 // threads per block of the search kernels
 constexpr int SP_W = SP_T / 32;
 constexpr int LANE_R = 4;                 // kNN: largest box of cells one lane walks
+constexpr int LANE_UNROLL_K = 16;         // ... longest list whose insertion is worth copying
+constexpr int FAR_FIRST = 8;              // ... points of it in the first pass / list length
 constexpr int FAR_RUN = 32;               // ... most points of a row of cells it reads alone
 constexpr double CELL_PER_K = 0.33;       // kNN in the plane: points per cell / k
 constexpr int SORT_TILE = 256;            // columns staged per warp by the row sort
@@ -256,8 +258,39 @@ __device__ __forceinline__ void scan_run(const float4* __restrict__ pts, int64_t
   for (; a < b; ++a) f(pts[a]);
 }
 
-// blocks per SM by list length: latency-bound walks want warps (K = 8: 0.67 -> 0.55 ms at 10 blocks)
-constexpr int knn_blocks(int K) { return K <= 8 ? 10 : (K <= 16 ? 6 : (K <= 32 ? 4 : 2)); }
+// hit(d2, id) for those of `len` points whose squared distance to q passes test(d2), few of them.
+// Four points at a time: their loads and distances do not wait for one another, and one branch
+// passes over all four.
+template <int D, class T, class F>
+__device__ __forceinline__ void scan_hits(const float4* __restrict__ at, int len, const float4& q,
+                                          T&& test, F&& hit) {
+  int t = 0;
+  for (; t + 4 <= len; t += 4) {
+    float d2[4];
+    int id[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 p = at[t + u];
+      d2[u] = sq_dist<D>(p, q);
+      id[u] = __float_as_int(p.w);
+    }
+    if (test(fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])))) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (test(d2[u])) hit(d2[u], id[u]);
+    }
+  }
+  for (; t < len; ++t) {
+    const float4 p = at[t];
+    const float d2 = sq_dist<D>(p, q);
+    if (test(d2)) hit(d2, __float_as_int(p.w));
+  }
+}
+
+// blocks per SM by list length: latency-bound walks want warps (K = 8: 0.67 -> 0.55 ms at 10
+// blocks), long lists registers (K = 32: 42,319 points in space 14.5 -> 10.9 ms at 3 for 4).  0: no
+// bound, the compiler's choice (K = 64: 168 registers; uniform 100,000, k = 65, 1.5 ms, 2.0 at 2)
+constexpr int knn_blocks(int K) { return K <= 8 ? 10 : (K <= 16 ? 6 : (K <= 32 ? 3 : 0)); }
 template <int K, int D>
 __global__ void __launch_bounds__(SP_T, knn_blocks(K))
 sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_start,
@@ -286,34 +319,59 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
     float t2 = prefilter(s[K - 1]);
     const int rmax = max(max(cx, g.g[0] - 1 - cx),
                          max(max(cy, g.g[1] - 1 - cy), D == 3 ? max(cz, g.g[2] - 1 - cz) : 0));
-    auto visit = [&](const float4& p) {
-      const float d2 = sq_dist<D>(p, q);
-      const int pid = __float_as_int(p.w);
-      if (d2 <= t2 && pid != qi) {
-        const float sd = __fsqrt_rn(d2);
-        if (key_less(sd, pid, s[K - 1], id[K - 1])) {
+    auto insert = [&](float d2, int pid) {
+      const float sd = __fsqrt_rn(d2);
+      if (pid == qi || !key_less(sd, pid, s[K - 1], id[K - 1])) return;
 #pragma unroll
-          for (int j = K - 1; j > 0; --j) {
-            const bool lp = key_less(sd, pid, s[j - 1], id[j - 1]);
-            const bool lc = key_less(sd, pid, s[j], id[j]);
-            const float ns = lp ? s[j - 1] : (lc ? sd : s[j]);
-            const int ni = lp ? id[j - 1] : (lc ? pid : id[j]);
-            s[j] = ns;
-            id[j] = ni;
-          }
-          if (key_less(sd, pid, s[0], id[0])) { s[0] = sd; id[0] = pid; }
-          t2 = prefilter(s[K - 1]);
-        }
+      for (int j = K - 1; j > 0; --j) {
+        const bool lp = key_less(sd, pid, s[j - 1], id[j - 1]);
+        const bool lc = key_less(sd, pid, s[j], id[j]);
+        const float ns = lp ? s[j - 1] : (lc ? sd : s[j]);
+        const int ni = lp ? id[j - 1] : (lc ? pid : id[j]);
+        s[j] = ns;
+        id[j] = ni;
       }
+      if (key_less(sd, pid, s[0], id[0])) { s[0] = sd; id[0] = pid; }
+      t2 = prefilter(s[K - 1]);
     };
+    // The points of cells x0..x1 of a row of cells, four at a time.  The insertion is K steps of code,
+    // some 8 KB at K = 64: copied for every point and every place that scans a run it did not stay in
+    // the instruction cache.  So there is one such place, and lists beyond LANE_UNROLL_K insert a
+    // group's hits in a loop: uniform 100,000 points, k = 65, 3.6 -> 2.0 ms, in space 7.8 -> 3.3; a
+    // slide of uneven density, 274,473 spots, k = 40, 121 -> 47.  The unrolled groups serve the short
+    // lists better (1M spots, k = 7: 0.52 against 0.67 ms).
     auto run = [&](int y, int z, int x0, int x1) {
       x0 = max(x0, 0);
       x1 = min(x1, g.g[0] - 1);
-      if (x0 > x1 || y < 0 || y >= g.g[1] || z < 0 || z >= g.g[2]) return;
+      if (x0 > x1) return;
       const int64_t row = (int64_t(z) * g.g[1] + y) * g.g[0];
-      const int64_t a = cell_start[row + x0], b = cell_start[row + x1 + 1];
-      evals += b - a;
-      scan_run(pts, a, b, visit);
+      const int64_t a = cell_start[row + x0];
+      const int len = int(cell_start[row + x1 + 1] - a);
+      const float4* at = pts + a;
+      evals += len;
+      if constexpr (K <= LANE_UNROLL_K) {
+        scan_hits<D>(at, len, q, [&](float d2) { return d2 <= t2; }, insert);
+        return;
+      }
+#pragma unroll 1
+      for (int t = 0; t < len; t += 4) {
+        float d2[4];
+        int pid[4];
+        unsigned m = 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 p = at[min(t + u, len - 1)];
+          d2[u] = sq_dist<D>(p, q);
+          pid[u] = __float_as_int(p.w);
+          if (d2[u] <= t2 && t + u < len) m |= 1u << u;
+        }
+#pragma unroll 1
+        for (; m; m &= m - 1) {
+          const bool odd = (m & 0xAu & (0u - m)) != 0u, high = (m & 3u) == 0u;
+          insert(high ? (odd ? d2[3] : d2[2]) : (odd ? d2[1] : d2[0]),
+                 high ? (odd ? pid[3] : pid[2]) : (odd ? pid[1] : pid[0]));
+        }
+      }
     };
     // Boxes of cells |d| <= R around the query's cell, R = 1 first; the cells of the last box (P) are
     // left out of the next, and rows of cells beyond the list's last distance r are skipped.  r says
@@ -321,9 +379,15 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
     // the warp pass: its one lane would walk thousands of row ranges while the launch waits.
     bool defer = false;
     for (int P = -1, R = 1;;) {
-      const int zlo = D == 3 ? max(-R, -cz) : 0, zhi = D == 3 ? min(R, g.g[2] - 1 - cz) : 0;
-      for (int dz = zlo; dz <= zhi; ++dz) {
-        for (int dy = max(-R, -cy); dy <= min(R, g.g[1] - 1 - cy); ++dy) {
+      // the query's own row of cells first (its near points bound the list early: 1M spots, k = 7,
+      // 0.57 -> 0.52 ms), then outwards: 0, -1, 1, -2, ...
+      for (int tz = 0; tz <= (D == 3 ? 2 * R : 0); ++tz) {
+        const int dz = (tz & 1) ? -((tz + 1) >> 1) : tz >> 1;
+        if (D == 3 && (cz + dz < 0 || cz + dz >= g.g[2])) continue;
+#pragma unroll 1
+        for (int ty = 0; ty <= 2 * R; ++ty) {
+          const int dy = (ty & 1) ? -((ty + 1) >> 1) : ty >> 1;
+          if (cy + dy < 0 || cy + dy >= g.g[1]) continue;
           if (P >= 1) {
             const double far = double(s[K - 1]) * (1.0 + 4e-6) + g.eps_abs;
             const double ly = g.o[1] + double(cy + dy) * g.cs;           // the row's lower face
@@ -333,12 +397,12 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
               if (lz - double(q.z) > far || double(q.z) - (lz + g.cs) > far) continue;
             }
           }
-          if (abs(dy) > P || (D == 3 && abs(dz) > P)) {
-            run(cy + dy, cz + dz, cx - R, cx + R);
-          } else {
-            run(cy + dy, cz + dz, cx - R, cx - P - 1);
-            run(cy + dy, cz + dz, cx + P + 1, cx + R);
-          }
+          // all of the row, or its cells on either side of the last box
+          const bool full = abs(dy) > P || (D == 3 && abs(dz) > P);
+#pragma unroll 1
+          for (int side = full ? 1 : 0; side < 2; ++side)
+            run(cy + dy, cz + dz, full || side == 0 ? cx - R : cx + P + 1,
+                full || side == 1 ? cx + R : cx - P - 1);
         }
       }
       // distance from the query to the nearest face of the box of cells within R that has
@@ -395,7 +459,9 @@ sp_knn_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_s
 // The queries the lane pass left open, a warp each: the lanes share a box's rows of cells.  First the
 // smallest box of a doubling sequence that holds k points (from the cell starts alone), then that
 // box's (k-1)-th distance r, then the rows and cells within r: every point that can be nearer.
-// Each lane keeps a sorted list of what it sees; the warp takes the smallest head m times.
+// Each lane keeps a sorted list of what it sees; the warp takes the smallest head m times.  Any k
+// points bound the distance, so the first pass takes only a few of a long row: 46,931 points with
+// three far outliers 7.1 -> 6.4 ms.
 template <int K, int D>
 __global__ void __launch_bounds__(SP_T)
 sp_knn_far_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ cell_start,
@@ -483,15 +549,24 @@ sp_knn_far_kernel(const float4* __restrict__ pts, const int64_t* __restrict__ ce
     for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
       for (int j = 0; j < K; ++j) { s[j] = INFINITY; id[j] = INT_MAX; }
+      const float rf = __double2float_ru(r);
       rows(min(R, rmax), r, [&](int64_t i, int step, int64_t last) {
-        evals += (last - i + step - 1) / step;
-        float4 ahead = pts[i];
-        for (; i < last; i += step) {
-          const float4 p = ahead;                  // the next one loads meanwhile
-          if (i + step < last) ahead = pts[i + step];
+        // any k points bound the distance: of a long row the first pass takes its first few
+        if (pass == 0 && step == 32) last = min(last, i - lane + FAR_FIRST * K);
+        evals += max(int64_t(0), (last - i + step - 1) / step);
+        float4 p4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p4[u] = pts[min(i + u * step, last - 1)];
+        for (int u = 0; i < last; i += step) {
+          const float4 p = u == 0 ? p4[0] : (u == 1 ? p4[1] : (u == 2 ? p4[2] : p4[3]));
+          if (++u == 4) {                          // the next four, whose loads overlap
+            u = 0;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) p4[v] = pts[min(i + (v + 1) * step, last - 1)];
+          }
           const int pid = __float_as_int(p.w);
           const float sd = __fsqrt_rn(sq_dist<D>(p, q));
-          if (pid == qi || !key_less(sd, pid, s[K - 1], id[K - 1])) continue;
+          if (pid == qi || sd > rf || !key_less(sd, pid, s[K - 1], id[K - 1])) continue;
 #pragma unroll
           for (int j = K - 1; j > 0; --j) {
             const bool lp = key_less(sd, pid, s[j - 1], id[j - 1]);
