@@ -26,3 +26,19 @@ def test_clumps_and_lone_points(clump, k, dims):
     oi, od = osp.grid_knn(P, k)
     np.testing.assert_array_equal(idx.cpu().numpy(), oi)
     np.testing.assert_array_equal(dist.cpu().numpy(), od)
+
+
+@pytest.mark.parametrize("dims,width", [(2, 1.0), (3, 1.0), (3, 0.0), (2, 40.0)])
+@pytest.mark.parametrize("n,k", [(2_094, 45), (5_000, 9)])
+def test_points_along_a_line_need_one_box(n, k, dims, width):
+    import torch
+    rng = np.random.default_rng(n + dims)
+    P = rng.normal(0, 1, (n, dims)) * width
+    P[:, 0] = rng.random(n) * 10_000
+    P = P.astype(np.float32)
+    idx, dist, stats = msp.knn_grid_device(torch.from_numpy(P).cuda(), k)
+    oi, od = osp.grid_knn(P, k)
+    np.testing.assert_array_equal(idx.cpu().numpy(), oi)
+    np.testing.assert_array_equal(dist.cpu().numpy(), od)
+    # most queries end in the first box of cells (in the plane and in space about one in four goes on)
+    assert int(stats[_lib.SP_STAT_EXPANDED]) <= n // 3
