@@ -115,7 +115,7 @@ size_t sample_smem(int d, int m) {
 __global__ void __launch_bounds__(SM_T)
 wide_sample_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ perm,
                    const SegDesc* __restrict__ seg, int nseg, int64_t npacked, int m_max, int kk,
-                   float* __restrict__ thr, int32_t* __restrict__ cnt) {
+                   int cap, float* __restrict__ thr, int32_t* __restrict__ cnt) {
   extern __shared__ __align__(16) float wd_smem[];
   float* xq = wd_smem;                                  // [d][SM_Q]
   float* ys = xq + d * SM_Q;                            // two tiles [SM_KEYS][d | 1]
@@ -181,6 +181,7 @@ wide_sample_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
       lo = __reduce_min_sync(FULL, lo);
       hi = __reduce_max_sync(FULL, hi);
       const int r = wide_rank(ns, m, kk), slack = max(2, r / 8);
+      int below = m;                                    // values at or below hi
       // the smallest pattern with at least r values at or below it, or one with few more than r
       while (lo < hi) {
         const unsigned mid = lo + (hi - lo) / 2;
@@ -188,12 +189,20 @@ wide_sample_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
 #pragma unroll 4
         for (int e = lane; e < m; e += 32) c += __float_as_uint(v[e]) <= mid;
         c = __reduce_add_sync(FULL, c);
-        if (c < r) lo = mid + 1;
-        else hi = mid;
+        if (c < r) {
+          lo = mid + 1;
+        } else {
+          hi = mid;
+          below = c;
+        }
         if (c >= r && c <= r + slack) break;
       }
-      if (lane == 0)
-        thr[p0 + w] = perm[p0 + w] >= 0 ? __uint_as_float(hi) * (1.f + 8.f * delta) : -1.f;
+      // A sample with many more values at or below it than r (coincident cells) says that more
+      // keys than the buffer takes lie there: the row goes to the FP64 scan with nothing collected
+      // (9,000 equal cells, k = 83, 5.03 -> 2.94 ms).
+      const float T = __uint_as_float(hi) * (1.f + 8.f * delta);
+      const bool fits = int64_t(below) * ns <= int64_t(cap) * m;
+      if (lane == 0) thr[p0 + w] = fits && perm[p0 + w] >= 0 ? T : -1.f;
     }
   }
 }
@@ -401,8 +410,8 @@ int launch_wide_scan(const float* X, int d, const int32_t* perm, const SegDesc* 
   MSC_CUDA_TRY(raise_smem_cap(wide_sample_kernel, ssm));
   MSC_CUDA_TRY(raise_smem_cap(wide_collect_kernel, csm));
   const int sgrid = int(std::min<int64_t>(npacked / SM_Q, int64_t(sms) * 64));
-  wide_sample_kernel<<<sgrid, SM_T, ssm, st>>>(X, d, perm, seg, nseg, npacked, m, kk, ws.thr,
-                                               ws.cnt);
+  wide_sample_kernel<<<sgrid, SM_T, ssm, st>>>(X, d, perm, seg, nseg, npacked, m, kk, cap,
+                                               ws.thr, ws.cnt);
   MSC_LAUNCH_CHECK();
   const int64_t rows = wide_rows(npacked, kk);
   const int resident = sms * resident_blocks_fn(reinterpret_cast<const void*>(wide_collect_kernel),
