@@ -53,15 +53,17 @@ extern "C" {
 #define MSC_STAT_TIMEOUT        1   /* device waits that gave up                                 */
 #define MSC_STAT_CERTIFIED      2   /* rows whose candidate set was proven to hold the exact kNN */
 #define MSC_STAT_REFINED        3   /* rows re-run through the BF16x3 candidate stage            */
-#define MSC_STAT_RESCANNED      4   /* rows finished by the exact FP64 full scan                 */
+#define MSC_STAT_RESCANNED      4   /* rows finished without candidates: by the search for more than
+                                       65 neighbours or by the exact FP64 full scan              */
 #define MSC_STAT_FP64_TIES      5   /* candidates re-ranked in FP64 at the k-th boundary         */
 #define MSC_STAT_CONN_NNZ       6   /* nnz of the connectivities CSR                              */
 #define MSC_STAT_PRECISION      7   /* candidate precision actually used (FP32 when the operand
                                        row is too wide for the tensor-core tile; -1: FP64 scan) */
 #define MSC_STATS_LEN           8
 
-#define MSC_MAX_K               129 /* largest n_neighbors (above 65 every row takes the FP64 scan) */
-#define MSC_MAX_K_KNN           513 /* largest n_neighbors of msc_knn alone (FP64 scan above 65)  */
+#define MSC_MAX_K               129 /* largest n_neighbors (above 65: FP32 differences, FP64 around the
+                                       k-th place; see msc_knn)                                   */
+#define MSC_MAX_K_KNN           513 /* largest n_neighbors of msc_knn alone                      */
 #define MSC_MAX_D               128 /* largest representation width                             */
 
 int         msc_version(void);
@@ -80,10 +82,11 @@ int       msc_profile_enable(int on);
 int       msc_profile_read(float* ms_out, int max_stages);
 /* pipeline counters of the tensor-core candidate kernel summed over CTAs since the last
  * msc_profile_enable(1) (cycles waiting / busy per role, hot chunks, compactions, candidate
- * insertions, CTAs), and in slots 10 and 11 the key tiles beyond the near ones that pruning
- * kept / could have kept; with max_counters >= 64, out[16 + 16·j + i] holds counter i of the
- * near pass (j = 0), the main scan (j = 1) and the refine pass (j = 2) alone; synchronizes the
- * device. */
+ * insertions, CTAs), in slots 10 and 11 the key tiles beyond the near ones that pruning
+ * kept / could have kept, and in slot 15 the work items that the main scan took in parts; with
+ * max_counters >= 64, out[16 + 16·j + i] holds counter i of the near pass (j = 0), the main scan
+ * (j = 1) and the refine pass (j = 2) alone; with max_counters >= 65, out[64] the rows that the
+ * search for more than 65 neighbours finished without an FP64 scan; synchronizes the device. */
 int       msc_profile_counters(unsigned long long* out, int max_counters);
 
 /* Self-test of the bounded device waits that every pipeline wait uses (no counterpart in the
@@ -126,8 +129,10 @@ int msc_neighbors_ex(const float* X_dev, int64_t n, int32_t d, int32_t k, int32_
  * distance (neighbors.py:117-118), the register top-k kernel `topk_rows` (neighbors.py:25-79),
  * the fp32 recompute (neighbors.py:122-123) and the host sort (neighbors.py:129-131), as one fused
  * candidate kernel + exact re-rank.  Self first; ties by index.  n_neighbors up to MSC_MAX_K_KNN
- * (scrublet's k_adj + 1 over observed and simulated cells reaches several hundred); above 65
- * every row takes the exact FP64 scan.
+ * (scrublet's k_adj + 1 over observed and simulated cells reaches several hundred).  Above 65
+ * neighbours FP32 differences decide all but the keys around the k-th place, which are compared in
+ * FP64; rows left open, and every row of a sample so large that 4,096 sampled cells hold fewer
+ * than six of a row's neighbours (45,000 cells at 66, 69,000 at 100), take the exact FP64 scan.
  * ------------------------------------------------------------------------------------------- */
 size_t msc_knn_workspace_bytes(int64_t n, int32_t d, int32_t k, int32_t metric, int32_t precision,
                                int32_t kprime);

@@ -760,6 +760,7 @@ int msc_profile_enable(int on) {
   timer().last = -1;
   if (on) {
     MSC_TRY(tc_counters_clear());
+    MSC_TRY(wide_counter_clear());
     return prune_counters_clear();
   }
   return MSC_OK;
@@ -769,10 +770,11 @@ int msc_profile_counters(unsigned long long* out, int max_counters) {
   if (!out || max_counters < 1) { set_error("out/max_counters invalid"); return MSC_ERR_INVALID_ARG; }
   MSC_CUDA_TRY(cudaDeviceSynchronize());
   MSC_TRY(tc_counters(out, max_counters));
-  unsigned long long pt[5];
+  unsigned long long pt[6];
   MSC_TRY(prune_counters(pt));
   for (int i = 0; i < 2 && 10 + i < max_counters; ++i) out[10 + i] = pt[i];
-  for (int i = 2; i < 5 && 10 + i < max_counters; ++i) out[10 + i] = pt[i];
+  for (int i = 2; i < 6 && 10 + i < max_counters; ++i) out[10 + i] = pt[i];
+  if (max_counters > 64) MSC_TRY(wide_counter(&out[64]));
   return MSC_OK;
 }
 

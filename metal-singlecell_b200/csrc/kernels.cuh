@@ -374,6 +374,9 @@ struct WideWs {
   int2* buf;          // (value, key) of the rows in flight
 };
 WideWs carve_wide(Carver& c, int64_t npacked, int k);
+// rows it finished since the last clear, while profiling
+int wide_counter(unsigned long long* out);
+int wide_counter_clear();
 int launch_wide_scan(const float* X, int d, const int32_t* perm, const SegDesc* seg, int nseg,
                      int64_t npacked, int64_t max_seg, int k, int cosine, const WideWs& ws,
                      int32_t* knn_idx, float* knn_dist, int32_t* fail_rows, Ctl* ctl,

@@ -39,7 +39,7 @@ constexpr int PR_T = 256;
 
 // summed over plans while profiling: key tiles visited beyond the near tiles, all such tiles,
 // tiles that failed level 1, tiles that reached the pair tests, pair tests
-__device__ unsigned long long g_prune_tiles[5];
+__device__ unsigned long long g_prune_tiles[6];
 constexpr int SUB = 32;          // rows per sub-block (two balls each)
 constexpr float NO_BALL = -1.f;  // radius of a ball without rows
 constexpr double OUTLIER_FACTOR = 4.0;   // default; MSC_B200_OUTLIER_FACTOR overrides (tuning)
@@ -892,7 +892,7 @@ constexpr int LONG_T = 1024;
 __global__ void __launch_bounds__(LONG_T)
 long_plan_kernel(const int32_t* __restrict__ cnt, int64_t n_items, int shift, int n_ctas,
                  int max_long, const int32_t* __restrict__ order, int32_t* __restrict__ claim,
-                 Ctl* __restrict__ ctl) {
+                 Ctl* __restrict__ ctl, int prof) {
   __shared__ unsigned long long total;
   __shared__ int n_long;
   if (threadIdx.x == 0) { total = 0; n_long = 0; }
@@ -915,6 +915,7 @@ long_plan_kernel(const int32_t* __restrict__ cnt, int64_t n_items, int shift, in
   if (threadIdx.x == 0) {
     ctl->n_long = int32_t(n);
     ctl->n_items_main = int32_t(n_items - n + parts);
+    if (prof) atomicAdd(&g_prune_tiles[5], (unsigned long long)n);
   }
 }
 
@@ -1445,11 +1446,11 @@ int launch_prune_partition(const float* X, int d, const SegDesc* seg, int nseg, 
 }
 
 int prune_counters(unsigned long long* out) {
-  MSC_CUDA_TRY(cudaMemcpyFromSymbol(out, g_prune_tiles, sizeof(unsigned long long) * 5));
+  MSC_CUDA_TRY(cudaMemcpyFromSymbol(out, g_prune_tiles, sizeof(unsigned long long) * 6));
   return MSC_OK;
 }
 int prune_counters_clear() {
-  const unsigned long long z[5] = {0, 0, 0, 0, 0};
+  const unsigned long long z[6] = {};
   MSC_CUDA_TRY(cudaMemcpyToSymbol(g_prune_tiles, z, sizeof(z)));
   return MSC_OK;
 }
@@ -1536,7 +1537,7 @@ int launch_long_plan(int64_t n_items, int words, int n_ctas, const PruneWs& w, C
   int shift = 0;
   while ((int64_t(words) * 32 >> shift) >= COST_BUCKETS) ++shift;
   long_plan_kernel<<<1, LONG_T, 0, st>>>(w.vcnt, n_items, shift, n_ctas, w.max_split_items,
-                                         w.claim, w.claim2, ctl);
+                                         w.claim, w.claim2, ctl, profiling_enabled() ? 1 : 0);
   MSC_LAUNCH_CHECK();
   return MSC_OK;
 }

@@ -34,6 +34,8 @@ namespace msc {
 
 namespace {
 
+__device__ unsigned long long g_wide_rows;      // rows finished, while profiling
+
 constexpr int WD_CAP_PER_SLOT = 8;        // buffer entries per list entry
 constexpr int WD_SAMPLE_MIN = 512, WD_SAMPLE_MAX = 4096;
 constexpr size_t WD_SMEM_MAX = size_t(227) * 1024 - 1024;
@@ -291,7 +293,7 @@ wide_select_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
                    int64_t row0, int64_t nrows, const float* __restrict__ thr,
                    const int32_t* __restrict__ cnt, const int2* __restrict__ buf, int cap, int k,
                    int cosine, int32_t* __restrict__ knn_idx, float* __restrict__ knn_dist,
-                   int32_t* __restrict__ fail_rows, Ctl* __restrict__ ctl) {
+                   int32_t* __restrict__ fail_rows, Ctl* __restrict__ ctl, int prof) {
   __shared__ int win_all[SE_WARPS][32 * SLOTS];
   __shared__ double val_all[SE_WARPS][32 * SLOTS];
   __shared__ __align__(16) float xs_all[SE_WARPS][MSC_MAX_D];
@@ -382,6 +384,7 @@ wide_select_kernel(const float* __restrict__ X, int d, const int32_t* __restrict
   if (lane == 0 && done)
     atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->stats[MSC_STAT_RESCANNED]),
               (unsigned long long)done);
+  if (prof && lane == 0 && done) atomicAdd(&g_wide_rows, (unsigned long long)done);
 }
 
 }  // namespace
@@ -390,6 +393,16 @@ bool wide_scan_ok(int64_t max_seg, int d, int k) {
   const int kk = k - 1, m = wide_sample(max_seg, kk);
   if (kk < 1 || kk > 512 || (m < max_seg && double(kk) * m < 5.9 * double(max_seg))) return false;
   return sample_smem(d, m) <= WD_SMEM_MAX && collect_smem(d) <= WD_SMEM_MAX;
+}
+
+int wide_counter(unsigned long long* out) {
+  MSC_CUDA_TRY(cudaMemcpyFromSymbol(out, g_wide_rows, sizeof(*out)));
+  return MSC_OK;
+}
+int wide_counter_clear() {
+  const unsigned long long z = 0;
+  MSC_CUDA_TRY(cudaMemcpyToSymbol(g_wide_rows, &z, sizeof(z)));
+  return MSC_OK;
 }
 
 WideWs carve_wide(Carver& c, int64_t npacked, int k) {
@@ -414,6 +427,7 @@ int launch_wide_scan(const float* X, int d, const int32_t* perm, const SegDesc* 
                                                ws.thr, ws.cnt);
   MSC_LAUNCH_CHECK();
   const int64_t rows = wide_rows(npacked, kk);
+  const int prof = profiling_enabled() ? 1 : 0;
   const int resident = sms * resident_blocks_fn(reinterpret_cast<const void*>(wide_collect_kernel),
                                                 CO_T, csm);
   for (int64_t r0 = 0; r0 < npacked; r0 += rows) {
@@ -430,15 +444,15 @@ int launch_wide_scan(const float* X, int d, const int32_t* perm, const SegDesc* 
     if (kk <= 128)
       wide_select_kernel<4><<<g, SE_WARPS * 32, 0, st>>>(X, d, perm, r0, nr, ws.thr, ws.cnt,
                                                          ws.buf, cap, k, cosine, knn_idx,
-                                                         knn_dist, fail_rows, ctl);
+                                                         knn_dist, fail_rows, ctl, prof);
     else if (kk <= 256)
       wide_select_kernel<8><<<g, SE_WARPS * 32, 0, st>>>(X, d, perm, r0, nr, ws.thr, ws.cnt,
                                                          ws.buf, cap, k, cosine, knn_idx,
-                                                         knn_dist, fail_rows, ctl);
+                                                         knn_dist, fail_rows, ctl, prof);
     else
       wide_select_kernel<16><<<g, SE_WARPS * 32, 0, st>>>(X, d, perm, r0, nr, ws.thr, ws.cnt,
                                                           ws.buf, cap, k, cosine, knn_idx,
-                                                          knn_dist, fail_rows, ctl);
+                                                          knn_dist, fail_rows, ctl, prof);
     MSC_LAUNCH_CHECK();
   }
   return MSC_OK;
