@@ -239,10 +239,15 @@ int check_common(int64_t n, int d, int k, int metric, int prec, int kprime,
 
 // Small samples are scanned in full, in no particular order: the order's ~14 launches per level,
 // the near pass and the plan cost a fixed time that the scan they save does not repay.
-// Graph times of the ordered and pruned path against the full scan (k = 15 at 50
-// dimensions / k = 10 at 100, cosine): 2.30 / 2.59 against 0.76 / 0.75 ms at 10,000 cells, 3.16 /
-// 4.08 against 1.66 / 1.81 at 31,007, 4.34 / 5.56 against 3.21 / 3.27 at 57,000, 4.82 / 6.44
-// against 4.89 / 5.12 at 80,000: the line lies where the full scan still wins at every width.
+// Graph times in ms of the ordered and pruned path / the full scan (k = 15 at 50 dimensions; k = 10
+// at 100, cosine):
+//              clustered, 1 % noise              uniform
+//   10,000     1.79 / 0.42    2.21 / 0.60
+//   40,000     2.51 / 1.98    3.14 / 2.06        3.40 / 1.72    4.05 / 1.85
+//   57,000     2.86 / 2.94    3.63 / 2.96        4.38 / 2.65    5.21 / 2.73
+//   80,000     3.54 / 4.61    4.40 / 4.78        6.33 / 4.24    7.27 / 4.39
+// What can be pruned is not known before the order is made.  At the line clustered samples are about
+// even (20 dimensions 2.62 / 2.83) and the others well ahead.
 constexpr int64_t DENSE_MAX_CELLS = 224 * 256;
 // work items of the full scan aimed at per resident CTA, ranges at most, list slots at most
 constexpr int DENSE_ITEMS_PER_CTA = 3, DENSE_MAX_SPLIT = 8, DENSE_SLOTS = 64;
