@@ -233,22 +233,20 @@ __device__ __forceinline__ float bb_part_d2_f32(const float* xs, const float* __
   return a0 + a1;
 }
 
-// a warp's FP64 scan of one batch (keys perm[0..nb)) for cell i: the kk <= 128 nearest by
-// (d², index) to oi / od
-__device__ __forceinline__ void bb_scan_row(const float* __restrict__ X, int d, int64_t i,
-                                            const int32_t* __restrict__ perm, int64_t nb, int kk,
-                                            float* xs, int32_t* oi, float* od) {
+// a warp's FP64 scan of keys perm[lo..hi) for cell i (xs: its row): the kk <= 128 nearest by
+// (d², index) in top
+__device__ __forceinline__ void bb_scan_keys(const float* __restrict__ X, int d, int64_t i,
+                                             const int32_t* __restrict__ perm, int64_t lo,
+                                             int64_t hi, int kk, float* xs, WarpTop128& top) {
   const int lane = lane_id();
-  const double INF = __longlong_as_double(0x7ff0000000000000ll);
   for (int t = lane; t < d; t += 32) xs[t] = X[i * d + t];
   __syncwarp();
-  WarpTop128 top;
   top.init();
-  for (int64_t base = 0; base < nb; base += 32) {
+  for (int64_t base = lo; base < hi; base += 32) {
     const int64_t jj = base + lane;
-    double v = INF;
+    double v = __longlong_as_double(0x7ff0000000000000ll);
     int vi = INT32_MAX;
-    if (jj < nb) {
+    if (jj < hi) {
       const int32_t c = perm[jj];
       if (c >= 0) {
         v = bb_d2_f64(xs, X + int64_t(c) * d, d);
@@ -257,15 +255,44 @@ __device__ __forceinline__ void bb_scan_row(const float* __restrict__ X, int d, 
     }
     top.offer(v, vi, kk);
   }
+}
+// a cell's kk neighbours in a batch to oi / od (warp-collective)
+__device__ __forceinline__ void bb_write_row(const WarpTop128& top, int64_t i, int kk, int32_t* oi,
+                                             float* od) {
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
-    const int r = s * 32 + lane;
+    const int r = s * 32 + lane_id();
     if (r < kk) {
       oi[r] = top.ai[s] == INT32_MAX ? int32_t(i) : top.ai[s];
       od[r] = __double2float_rn(sqrt(top.a[s]));
     }
   }
   __syncwarp();
+}
+
+// A block's FP64 scan of a batch for one cell: its warps take an eighth of the keys each and are
+// merged (kk <= 32).  While there are no more cells to scan than blocks this is what the scans do: a
+// lone cell is otherwise one warp's chain of FP64 sums over the whole batch.  56,723 x 50 with 23
+// such cells 6.9 -> 4.3 ms, 54,089 x 7 with 41 3.8 -> 2.6.  The warps' lists take the place of their
+// rows (xs): shared memory of their own would cost the scans of many cells L1, 2 to 4 %.
+__device__ __forceinline__ void bb_scan_block(const float* __restrict__ X, int d, int64_t i,
+                                              const int32_t* __restrict__ perm, int64_t nb, int kk,
+                                              float (*xs)[MSC_MAX_D], int32_t* oi, float* od) {
+  static_assert(sizeof(xs[0]) >= 32 * (sizeof(double) + sizeof(int)), "a list fits a row");
+  const int lane = lane_id(), wib = warp_id();
+  const int64_t per = (nb + BB_WARPS * 32 - 1) / (BB_WARPS * 32) * 32;
+  WarpTop128 top;
+  bb_scan_keys(X, d, i, perm, wib * per, min64(nb, (wib + 1) * per), kk, xs[wib], top);
+  __syncwarp();                                          // the row is read
+  reinterpret_cast<double*>(xs[wib])[lane] = top.a[0];
+  reinterpret_cast<int*>(xs[wib])[64 + lane] = top.ai[0];
+  __syncthreads();
+  if (wib == 0) {
+    for (int q = 1; q < BB_WARPS; ++q)
+      top.offer(reinterpret_cast<const double*>(xs[q])[lane],
+                reinterpret_cast<const int*>(xs[q])[64 + lane], kk);
+    bb_write_row(top, i, kk, oi, od);
+  }
 }
 
 // One warp per cell i: its k' candidates in batch b (original rows, -1 = none) → the kk nearest
@@ -430,7 +457,7 @@ bb_group_rerank_kernel(const float* __restrict__ X, int d, int64_t n, int64_t p1
     atomicAdd(reinterpret_cast<unsigned long long*>(n_cert_out), (unsigned long long)n_cert);
 }
 
-// FP64 scan of the listed (cell, batch) pairs of a group
+// FP64 scan of the listed (cell, batch) pairs of a group: a warp each, or a block (bb_scan_block)
 __global__ void __launch_bounds__(BB_T)
 bb_group_scan_kernel(const float* __restrict__ X, int d, const int32_t* __restrict__ list,
                      const BbBatches B, const int32_t* __restrict__ rows,
@@ -440,14 +467,24 @@ bb_group_scan_kernel(const float* __restrict__ X, int d, const int32_t* __restri
   __shared__ __align__(16) float xs_all[BB_WARPS][MSC_MAX_D];
   const int lane = lane_id(), wib = warp_id();
   const int64_t count = *nrows;
+  if (count <= gridDim.x) {
+    if (blockIdx.x >= count) return;
+    const int b = bats[blockIdx.x];
+    const int64_t i = rows[blockIdx.x];
+    bb_scan_block(X, d, i, list + B.start[b], B.nb[b], B.kk[b], xs_all,
+                  knn_idx + i * K + B.col0[b], knn_dist + i * K + B.col0[b]);
+    if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(n_scanned), 1ull);
+    return;
+  }
+  WarpTop128 top;
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   int64_t done = 0;
   for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w < count;
        w += nwarps) {
-    const int b = bats[w];
-    bb_scan_row(X, d, rows[w], list + B.start[b], B.nb[b], B.kk[b], xs_all[wib],
-                knn_idx + int64_t(rows[w]) * K + B.col0[b],
-                knn_dist + int64_t(rows[w]) * K + B.col0[b]);
+    const int b = bats[w], kk = B.kk[b];
+    const int64_t i = rows[w];
+    bb_scan_keys(X, d, i, list + B.start[b], 0, B.nb[b], kk, xs_all[wib], top);
+    bb_write_row(top, i, kk, knn_idx + i * K + B.col0[b], knn_dist + i * K + B.col0[b]);
     ++done;
   }
   if (lane == 0 && done)
@@ -465,13 +502,22 @@ bb_scan_kernel(const float* __restrict__ X, int d, int64_t n, const int32_t* __r
   __shared__ __align__(16) float xs_all[BB_WARPS][MSC_MAX_D];
   const int lane = lane_id(), wib = warp_id();
   const int64_t count = rows ? int64_t(*nrows) : n;
+  if (rows && count <= gridDim.x && kk <= 32) {
+    if (blockIdx.x >= count) return;
+    const int64_t i = rows[blockIdx.x];
+    bb_scan_block(X, d, i, perm + poff, nb, kk, xs_all, knn_idx + i * K + col0,
+                  knn_dist + i * K + col0);
+    if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(n_scanned), 1ull);
+    return;
+  }
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   int64_t done = 0;
   for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w < count;
        w += nwarps) {
     const int64_t i = rows ? int64_t(rows[w]) : w;
-    bb_scan_row(X, d, i, perm + poff, nb, kk, xs_all[wib], knn_idx + i * K + col0,
-                knn_dist + i * K + col0);
+    WarpTop128 top;
+    bb_scan_keys(X, d, i, perm + poff, 0, nb, kk, xs_all[wib], top);
+    bb_write_row(top, i, kk, knn_idx + i * K + col0, knn_dist + i * K + col0);
     ++done;
   }
   if (lane == 0 && done)
@@ -680,14 +726,15 @@ BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int pre
   P.kprime = 0;
   if (P.candidates) {
     // over-fetch: the certificate compares the kk-th neighbour with the k'-th candidate (the self
-    // path's k' = 48 is sized for the 15th neighbour); wider lists for larger kk.  A cell it cannot
-    // certify takes an FP64 scan of the batch, milliseconds for a lone one, which is more than
-    // shorter lists save: with one-term operands k' = 24 saves 7 % where every cell passes (8
-    // batches of 200,000 x 50, FP16: 13.7 against 14.7 ms), but 123,000 x 30 with one such cell
-    // took 8.8 ms against 6.2, 60,000 x 50 in BF16 146 against 91.  The three-term split left no
-    // cell at 24.
+    // path's k' = 48 is sized for the 15th neighbour), and a cell that it cannot certify takes an
+    // FP64 scan of the batch.  24 candidates save 6 to 10 % against 32 where no cell fails (8 batches
+    // of 200,000 x 50, FP16: 13.7 and 14.7 ms).  For up to four neighbours they leave none to some
+    // tens of cells that 32 would not; for more, or with BF16 operands, they left thousands
+    // (60,000 x 50 BF16 146 ms against 91; 132,000 x 50 FP16 with 13 neighbours 19.0 against 15.1).
+    // The three-term split left none at 24.
+    const bool few = prec == PREC_FP16 && P.kk_max <= 4;
     P.kprime = prec == PREC_BF16X3 ? std::min(64, std::max(24, P.kk_max + 9))
-                                   : std::min(64, std::max(32, P.kk_max + 16));
+                                   : std::min(64, std::max(few ? 24 : 32, P.kk_max + 16));
     P.L = op_layout(prec, d);
     P.cfg = tc_default_config(prec, d, P.kprime);
     if (P.cfg.pair || !tc_config_ok(P.cfg, P.L.kp, P.kprime)) P.candidates = false;
