@@ -741,10 +741,16 @@ BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int pre
   }
   P.ntiles = ceil_div(n, QTILE);
   // the ordered scan: lists the group re-rank takes, 256-key tiles, and enough cells that the order
-  // and the plan cost less than the tiles they save: 16,384 cells in 8 batches 2.17 ms plain, 2.21
-  // ordered; 30,000 in 4 batches 2.20 / 2.29; 60,000 in 8 8.0 / 4.9.  MSC_B200_BB_ORDER=<cells>
-  // moves the line (tests; 0: always, negative: never).
-  int64_t least = BB_ORDER_MIN;
+  // and the plan cost less than the tiles they save.  Batch by batch the scan is a launch per stage
+  // and batch, so the line lies lower the more batches there are.  ms batch by batch / ordered:
+  //            clustered data                  Gaussian data (nothing to prune)
+  //   cells    2 batches    8                  2            8
+  //   33,000   1.62 / 2.71  3.42 / 3.23        1.62 / 2.68  3.48 / 3.91
+  //   45,000   2.65 / 2.91  5.43 / 3.88        2.65 / 3.32  5.45 / 5.17
+  //   60,000   3.73 / 3.25  7.43 / 4.70        3.73 / 4.34  7.46 / 6.88
+  // The line is where clustered data, the usual, is even (4 batches: about 38,000).
+  // MSC_B200_BB_ORDER=<cells> moves it (tests; 0: always, negative: never).
+  int64_t least = std::max<int64_t>(BB_ORDER_MIN, BB_ORDER_MIN * 3 / 4 * (nb + 2) / nb);
   if (const char* e = std::getenv("MSC_B200_BB_ORDER")) {
     least = std::atoll(e);
     if (least < 0) least = INT64_MAX;
