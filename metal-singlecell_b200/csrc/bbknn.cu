@@ -23,7 +23,7 @@
 // keys alike; a near pass scans every query tile's nearest key tile of each batch, and its radii give
 // masks of the key tiles that can still matter (prune.cu), so that a query tile visits a few tiles
 // of a batch instead of all.  All batches run in one launch per stage.  200,000 x 50, 8 batches, 3
-// neighbours in each: the graph 38.0 ms batch by batch, 13.3 ordered.
+// neighbours in each: the graph 35.3 ms batch by batch, 14.0 ordered.
 //
 // The distances graph drops the diagonal and every zero distance (neighbors.py:554-557); the
 // trimming keeps an entry (i, j) of value v when v != 0, v >= θ_i and v >= θ_j, θ_i being the
@@ -728,11 +728,11 @@ BbPlan bb_plan(int64_t n, int d, const int64_t* counts, int nb, int kwb, int pre
     // over-fetch: the certificate compares the kk-th neighbour with the k'-th candidate (the self
     // path's k' = 48 is sized for the 15th neighbour), and a cell that it cannot certify takes an
     // FP64 scan of the batch.  24 candidates save 6 to 10 % against 32 where no cell fails (8 batches
-    // of 200,000 x 50, FP16: 13.7 and 14.7 ms).  For up to four neighbours they leave none to some
+    // of 200,000 x 50, FP16: 13.7 and 14.7 ms).  For up to six neighbours they leave none to some
     // tens of cells that 32 would not; for more, or with BF16 operands, they left thousands
     // (60,000 x 50 BF16 146 ms against 91; 132,000 x 50 FP16 with 13 neighbours 19.0 against 15.1).
     // The three-term split left none at 24.
-    const bool few = prec == PREC_FP16 && P.kk_max <= 4;
+    const bool few = prec == PREC_FP16 && P.kk_max <= 6;
     P.kprime = prec == PREC_BF16X3 ? std::min(64, std::max(24, P.kk_max + 9))
                                    : std::min(64, std::max(few ? 24 : 32, P.kk_max + 16));
     P.L = op_layout(prec, d);
