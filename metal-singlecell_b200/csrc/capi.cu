@@ -353,11 +353,12 @@ int make_problem(Problem& P, int64_t n, int d, int k, int metric, int prec, int 
     if (n <= most) {
       P.dense = true;
       // Rows come to the refine pass because their k-th place is crowded, so its lists stay as long
-      // as the one-term pass's unless 32 candidates are twice the neighbours already.  (k + 8
-      // of them left 5,885 of 57,000 x 128 rows, k = 33, to the FP64 scan where 48 leave 22: graph
-      // 192 and 39 ms.  At k = 15 32 and 48 leave the same rows, and 20,000 BF16 cells take 1.47
-      // ms with 32, 1.78 with 48.)
-      P.kref = 2 * (k - 1) <= 32 ? 32 : std::max(P.kprime, default_kprime(P.prec, k));
+      // as the one-term pass's unless 32 candidates have room, the less the wider the rows.  With
+      // lists of max(32, k + 8) 57,000 x 128 cells, k = 33, left 5,885 rows to the FP64 scan where 48
+      // leave 22: graph 192 and 39 ms.  With 32, 57,000 mixture cells in BF16, nearly every row
+      // refined: 31 and 50 dimensions none to k = 22, 128 none at k = 17, some from 18 on.  Where both
+      // leave none 32 are 1 to 20 % faster (15,220 x 31, k = 18, 0.618 and 0.649 ms).
+      P.kref = k <= (d <= 50 ? 22 : 17) ? 32 : std::max(P.kprime, default_kprime(P.prec, k));
       plan_dense(P, P.prec, d, n, k, kprime);
     }
   }
